@@ -24,6 +24,7 @@ extern "C" void dem_count_replayed_launches(unsigned long long k) { dem_count_la
 
 namespace dem {
 int sym_sorted_prepare(dem_ctx *ctx);
+int direct_fp64_prepare(dem_ctx *ctx);
 int direct_plan(const dem_ctx *ctx, int n, int periodic, int *schedule, int *i_per_thread, int *threads,
                 long long *ctas, int *j_splits);
 }
@@ -212,6 +213,7 @@ int dem_ctx_create(int device, int capacity, dem_ctx **out) {
         if (!rc) ctx->scan_tmp_bytes = need;
     }
     if (!rc) rc = dem::sym_sorted_prepare(ctx);
+    if (!rc) rc = dem::direct_fp64_prepare(ctx);
     if (rc) {
         fprintf(stderr, "dem_ctx_create: %s\n", ctx->last_error.c_str());
         dem_ctx_destroy(ctx);

@@ -1,160 +1,363 @@
 // direct_fp64.cu -- plain-FP64 direct O(N^2) passes (the reference drop-in).
 //
-// One thread owns one droplet i and sums its pair terms over j = 0..n-1 in
-// ascending order, exactly like the reference's serial inner loop, with every
-// expression evaluated in the reference's order.  This file is compiled with
-// -fmad=false so no multiply-add is contracted: each operation rounds once,
-// and the results are bit-identical to the CPU restatement of
+// Every droplet's pair terms are summed over j = 0..n-1 in ascending order,
+// exactly like the reference's serial inner loop, with every expression
+// evaluated in the reference's order.  This file is compiled with -fmad=false
+// so no multiply-add is contracted: each operation rounds once, and the
+// results are bit-identical to the CPU restatement of
 //   dem/force_calculator/direct_droplet_force_calculator.py:183-253 (forces)
 //   dem/force_calculator/direct_droplet_force_calculator.py:354-411 (convection).
 //
-// j-tiles (x, y, z, r, r^3) are staged in shared memory and read as
-// broadcasts; the pair work is FP64-pipe bound (IEEE sqrt / division).
+// Only the additions are serial, not the terms.  A CTA takes R droplets (rows):
+// 256 producer threads evaluate the terms of a tile of j's, side by side, into
+// shared memory while one adder thread per (row, component) adds the previous
+// tile's terms to its running sum in j order (an FP64 addition has 8 cycles of
+// latency, so a chain takes ~10 cycles per j) and stages the next tile's j's.
+// One thread per droplet, which this replaces, kept a term's whole latency in
+// the chain (~430 ns per j and pass) and left most of the chip idle below
+// n ~ 60,000.  The terms use square root, reciprocals and quotients without
+// branches (ieee64.cuh), so that a thread has several terms in flight, and the
+// six quotients of an Oseen term share one reciprocal.
+//
+// Bound: the FP64 pipe (59 / 86 operations per pair) at large n, the adders'
+// chains and the terms' latency at small n.  Force / convection pass, periodic,
+// us, before -> now: n = 500 137 / 310 -> 13 / 13; 2,000 527 / 1,220 -> 34 / 43;
+// 8,000 2,090 / 4,860 -> 328 / 446; 20,011 5,650 / 12,800 -> 1,800 / 2,520 (FP64
+// pipe 68 / 74 % of peak; more resident warps, larger tiles or 512 producers
+// change that by a few per cent either way).
 //
 // With the periodic-image correction loaded, the convection kernel adds each
 // pair's correction term right after its Stokeslet term and the self term
-// after the loop (:413-464), bit-identical to the CPU restatement.
+// after the loop (:413-464), bit-identical to the CPU restatement.  It is
+// bound by the correction table's gathers: n = 2,000 7,520 -> 550 us, 8,192
+// 30,800 -> 7,600.
 #include "common.cuh"
 #include "corr.cuh"
+#include "ieee64.cuh"
+#include <type_traits>
 
 namespace dem {
 
-constexpr int F64_THREADS = 128;
-constexpr int F64_TILE = 128;
+#ifndef ORD_UNROLL
+#define ORD_UNROLL 4
+#endif
+enum : int { FORCE64 = 0, OSEEN64 = 1, OSEEN64_CORR = 2 };
 
-template <bool PERIODIC>
-__global__ void __launch_bounds__(F64_THREADS) direct_force_fp64_kernel(int n, const double *__restrict__ x,
-                                                                        const double *__restrict__ y,
-                                                                        const double *__restrict__ z,
-                                                                        const double *__restrict__ r, double m_const,
-                                                                        double L, double halfL, double *__restrict__ fx,
-                                                                        double *__restrict__ fy, double *__restrict__ fz) {
-    __shared__ double sx[F64_TILE], sy[F64_TILE], sz[F64_TILE], sr[F64_TILE], sr3[F64_TILE];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    double xi = 0, yi = 0, zi = 0, ri = 0, mri3 = 0;
-    if (active) {
-        xi = x[i];
-        yi = y[i];
-        zi = z[i];
-        ri = r[i];
-        mri3 = m_const * ipow3(ri);  // (m_const * r_i**3) is the first product of :189
-    }
-    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
-    for (int t0 = 0; t0 < n; t0 += F64_TILE) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < F64_TILE; k += blockDim.x) {
-            const int j = t0 + k;
-            if (j < n) {
-                sx[k] = x[j];
-                sy[k] = y[j];
-                sz[k] = z[j];
-                const double rj = r[j];
-                sr[k] = rj;
-                sr3[k] = ipow3(rj);
-            }
-        }
-        __syncthreads();
-        const int cnt = min(F64_TILE, n - t0);
-        if (!active) continue;
-        for (int k = 0; k < cnt; ++k) {
-            if (t0 + k == i) continue;
-            double dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;
-            if (PERIODIC) {
-                dx = mic64(dx, L, halfL);
-                dy = mic64(dy, L, halfL);
-                dz = mic64(dz, L, halfL);
-            }
-            const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
-            const double r_mag = sqrt(dx2 + dy2 + dz2);
-            if (r_mag > ri + sr[k]) {
-                const double M = mri3 * sr3[k] / ipow7(r_mag);
-                const double fxy = M * (4 * dz2 - dx2 - dy2);
-                Fx += fxy * dx;
-                Fy += fxy * dy;
-                Fz += M * (2 * dz2 - 3 * dx2 - 3 * dy2) * dz;
-            }
-        }
-    }
-    if (active) {
-        fx[i] = Fx;
-        fy[i] = Fy;
-        fz[i] = Fz;
+constexpr int ORD_P = 256;  // producer threads
+constexpr int NV = 6;       // doubles staged per j: x, y, z, r^3, r, - (force) or x, y, z, Fx, Fy, Fz
+
+template <int R, int KIND>
+struct OrdShape {
+    static constexpr int SUBS = ORD_P / R;                       // j's evaluated side by side per row
+    static constexpr int U = SUBS > 32 || KIND == OSEEN64_CORR ? 2 : 4;  // terms per producer thread and tile
+    static constexpr int TJ = SUBS * U;                          // j's per tile
+    static constexpr int ADD_T = (3 * R + 31) / 32 * 32;         // adder threads: one per (row, component)
+    static constexpr int THREADS = ORD_P + ADD_T;
+    static constexpr int CTAS = KIND == OSEEN64_CORR ? 2 : 3;    // per SM: 64 - 72 registers (the correction: 112)
+    static constexpr int PLANES = KIND == OSEEN64_CORR ? 6 : 3;  // terms per pair
+    static constexpr int CS = TJ * R + (R < 16 ? R : 0);         // plane stride (narrow rows: offset banks)
+    static constexpr int LOADS = (TJ + ADD_T - 1) / ADD_T;       // staged j's per adder thread
+    static constexpr size_t SMEM = sizeof(double) * (2 * PLANES * CS + 2 * NV * TJ);
+    static_assert(TJ <= ORD_P, "tile 0 is staged by the first TJ threads");
+};
+
+struct Ord64Args {
+    int n;
+    const double *x, *y, *z, *r;
+    const double *fx, *fy, *fz;
+    double coeff;  // m_const / eta
+    double L, halfL;
+    CorrDev corr;
+    double *ox, *oy, *oz;
+};
+
+struct D3 {
+    double x, y, z;
+};
+
+// a coordinate: zero or 2^-300 <= |v| < 2^90, so that differences of two are zero or >= 2^-352
+__device__ __forceinline__ bool coord_ok(double v) { return v == 0.0 || hi_in(fabs(v), hi_of_pow2(-300), hi_of_pow2(90)); }
+__device__ __forceinline__ bool factor_ok(double v) { return hi_in(v, hi_of_pow2(-125), hi_of_pow2(125)); }
+
+// ---- pair terms -------------------------------------------------------------
+// Minimum image, as mic64 (:234-240): the subtraction predicated, not selected.
+__device__ __forceinline__ void image1(double &d, double L, double halfL) {
+    asm("{\n\t.reg .pred p;\n\tsetp.gt.f64 p, %1, %2;\n\t@p sub.rn.f64 %0, %0, %3;\n\t}"
+        : "+d"(d)
+        : "d"(fabs(d)), "d"(halfL), "d"(copysign(L, d)));
+}
+
+template <bool PER>
+__device__ __forceinline__ void image3(double &x, double &y, double &z, double L, double halfL) {
+    if (PER) {
+        image1(x, L, halfL);
+        image1(y, L, halfL);
+        image1(z, L, halfL);
     }
 }
 
-template <bool PERIODIC, bool CORR>
-__global__ void __launch_bounds__(F64_THREADS) direct_convection_fp64_kernel(
-    int n, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-    const double *__restrict__ fx, const double *__restrict__ fy, const double *__restrict__ fz, double eta,
-    double L, double halfL, CorrDev corr, double *__restrict__ vx, double *__restrict__ vy,
-    double *__restrict__ vz) {
-    __shared__ double sx[F64_TILE], sy[F64_TILE], sz[F64_TILE], sfx[F64_TILE], sfy[F64_TILE], sfz[F64_TILE];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    double xi = 0, yi = 0, zi = 0;
-    if (active) {
-        xi = x[i];
-        yi = y[i];
-        zi = z[i];
+// The force term of a separation, :183-200 (0 inside the contact cut, :246).  PLAIN: every operand;
+// else returns false where the branch-free operations do not apply.
+template <bool PLAIN>
+__device__ __forceinline__ bool force_term64(double dx, double dy, double dz, double mri3, double rj3, double reach,
+                                             D3 &t) {
+    const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
+    const double r2 = dx2 + dy2 + dz2;
+    double M, r_mag;
+    bool ok = true;
+    if (PLAIN) {
+        r_mag = sqrt(r2);
+        M = mri3 * rj3 / ipow7(r_mag);
+    } else {
+        double h;
+        r_mag = sqrt_rn(r2, h);
+        const double r7 = ipow7(r_mag);
+        M = quotient_rn(mri3 * rj3, r7, rcp_rn(r7));
+        ok = hi_in(r2, hi_of_pow2(-200), hi_of_pow2(200)) && !low_word_ones(r7);
     }
-    double Cx = 0.0, Cy = 0.0, Cz = 0.0;
-    for (int t0 = 0; t0 < n; t0 += F64_TILE) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < F64_TILE; k += blockDim.x) {
-            const int j = t0 + k;
-            if (j < n) {
-                sx[k] = x[j];
-                sy[k] = y[j];
-                sz[k] = z[j];
-                sfx[k] = fx[j];
-                sfy[k] = fy[j];
-                sfz[k] = fz[j];
-            }
+    const bool keep = r_mag > reach;
+    if (!PLAIN) M = keep ? M : 0.0;  // finite operands: the terms become zeros
+    // 4 dz^2 and 2 dz^2 are exact: one rounding each with the difference that follows
+    const double fxy = M * (__fma_rn(4.0, dz2, -dx2) - dy2);
+    t.x = fxy * dx;
+    t.y = fxy * dy;
+    t.z = M * (__fma_rn(2.0, dz2, -(3 * dx2)) - 3 * dy2) * dz;
+    if (PLAIN && !keep) t = D3{0.0, 0.0, 0.0};
+    return ok;
+}
+
+// The Oseen term of a separation, :382-411.
+template <bool PLAIN>
+__device__ __forceinline__ bool oseen_term64(double X, double Y, double Z, double Fx, double Fy, double Fz,
+                                             double eta, D3 &t) {
+    const double XX = X * X, YY = Y * Y, ZZ = Z * Z;
+    const double r2 = XX + YY + ZZ;
+    double inv_r, xx, yy, zz, xy, xz, yz;
+    bool ok = true;
+    if (PLAIN) {
+        const double rr = sqrt(r2);
+        const double r3 = ipow3(rr);
+        inv_r = 1 / rr;
+        xx = XX / r3;
+        yy = YY / r3;
+        zz = ZZ / r3;
+        xy = (X * Y) / r3;
+        xz = (X * Z) / r3;
+        yz = (Y * Z) / r3;
+    } else {
+        double h;
+        const double rr = sqrt_rn(r2, h);
+        const double r3 = ipow3(rr);
+        inv_r = rcp_last(rr, rcp_last(rr, times_pow2(h, 1)));
+        const double y3 = rcp_rn(r3);
+        xx = quotient_rn(XX, r3, y3);
+        yy = quotient_rn(YY, r3, y3);
+        zz = quotient_rn(ZZ, r3, y3);
+        xy = quotient_rn(X * Y, r3, y3);
+        xz = quotient_rn(X * Z, r3, y3);
+        yz = quotient_rn(Y * Z, r3, y3);
+        ok = hi_in(r2, hi_of_pow2(-200), hi_of_pow2(200)) && !low_word_ones(rr) && !low_word_ones(r3);
+    }
+    t.x = eta * ((inv_r + xx) * Fx + xy * Fy + xz * Fz);
+    t.y = eta * (xy * Fx + (inv_r + yy) * Fy + yz * Fz);
+    t.z = eta * (xz * Fx + yz * Fy + (inv_r + zz) * Fz);
+    return ok;
+}
+
+template <int R, bool PER, int KIND>
+__global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>::CTAS) ordered_pass_kernel(const Ord64Args a) {
+    using S = OrdShape<R, KIND>;
+    extern __shared__ __align__(16) double ord_smem[];
+    double *const stage = ord_smem;                 // [2][TJ][NV]
+    double *const terms = ord_smem + 2 * NV * S::TJ;  // [2][PLANES][CS]: the term of (j, row) at j * R + row
+    const int tid = threadIdx.x;
+    const int n = a.n;
+    const int row0 = blockIdx.x * R;
+    const int ntiles = (n + S::TJ - 1) / S::TJ;
+
+    const double *const src[NV] = {a.x, a.y, a.z, KIND == FORCE64 ? a.r : a.fx, a.fy, a.fz};
+    constexpr int NSRC = KIND == FORCE64 ? 4 : 6;
+    // Writes droplet j's values to its stage slot (NaN past the end: no fast term); whether it is fit for
+    // the branch-free operations.
+    auto put = [&](double *slot, double (&v)[NSRC], bool in) {
+        if (!in) v[0] = __longlong_as_double(0x7ff8000000000000ll);
+        double w3 = v[3], w4 = KIND == FORCE64 ? v[3] : v[NSRC - 2];
+        if (KIND == FORCE64) w3 = ipow3(w4);
+        slot[0] = v[0], slot[1] = v[1], slot[2] = v[2];
+        slot[3] = w3, slot[4] = w4;
+        if (KIND != FORCE64) slot[5] = v[NSRC - 1];
+        return coord_ok(v[0]) && coord_ok(v[1]) && coord_ok(v[2]) && (KIND != FORCE64 || factor_ok(w3));
+    };
+    int odd = 0;
+    if (tid < S::TJ) {
+        double v[NSRC];
+#pragma unroll
+        for (int w = 0; w < NSRC; ++w) v[w] = tid < n ? src[w][tid] : 0.0;
+        odd = !put(stage + NV * tid, v, tid < n) && tid < n;
+    }
+    odd = __syncthreads_or(odd);
+
+    if (tid < ORD_P) {
+        const int row = tid % R, sub = tid / R;
+        const int i = row0 + row;
+        const int ii = min(i, n - 1);
+        const double xi = a.x[ii], yi = a.y[ii], zi = a.z[ii];
+        double ri = 0.0, mri3 = 0.0;
+        if (KIND == FORCE64) {
+            ri = a.r[ii];
+            mri3 = a.coeff * ipow3(ri);  // (m_const * r_i**3) is the first product of :189
         }
-        __syncthreads();
-        const int cnt = min(F64_TILE, n - t0);
-        if (!active) continue;
-        for (int k = 0; k < cnt; ++k) {
-            if (t0 + k == i) continue;
-            double X = xi - sx[k], Y = yi - sy[k], Z = zi - sz[k];
-            if (PERIODIC) {
-                X = mic64(X, L, halfL);
-                Y = mic64(Y, L, halfL);
-                Z = mic64(Z, L, halfL);
+        const bool row_ok = coord_ok(xi) && coord_ok(yi) && coord_ok(zi) && (KIND != FORCE64 || factor_ok(mri3)) &&
+                            (!PER || hi_in(a.L, hi_of_pow2(-300), hi_of_pow2(90)));
+        for (int t = 0; t <= ntiles; ++t) {
+            if (t < ntiles) {
+                const double *const s = stage + (t & 1) * NV * S::TJ + NV * sub;
+                double *const o = terms + (t & 1) * S::PLANES * S::CS + sub * R + row;
+                // The term of the thread's u-th j, written to its slots; false: the operands need the
+                // operators (PLAIN).
+                auto term = [&](int u, auto plain) {
+                    const double2 *const q = reinterpret_cast<const double2 *>(s + u * S::SUBS * NV);
+                    const double2 p0 = q[0], p1 = q[1], p2 = q[2];  // (x, y), (z, r^3 | Fx), (r | Fy, Fz)
+                    double *const w = o + u * S::SUBS * R;
+                    D3 v;
+                    bool ok;
+                    double X, Y, Z;
+                    if (KIND == FORCE64) {
+                        X = p0.x - xi, Y = p0.y - yi, Z = p1.x - zi;
+                        image3<PER>(X, Y, Z, a.L, a.halfL);
+                        ok = force_term64<decltype(plain)::value>(X, Y, Z, mri3, p1.y, ri + p2.x, v);
+                    } else {
+                        X = xi - p0.x, Y = yi - p0.y, Z = zi - p1.x;
+                        image3<PER>(X, Y, Z, a.L, a.halfL);
+                        ok = oseen_term64<decltype(plain)::value>(X, Y, Z, p1.y, p2.x, p2.y, a.coeff, v);
+                    }
+                    w[0] = v.x;
+                    w[S::CS] = v.y;
+                    w[2 * S::CS] = v.z;
+                    if (KIND == OSEEN64_CORR) {
+                        D3 c{0.0, 0.0, 0.0};
+                        corr_pair64(a.corr, X, Y, Z, p1.y, p2.x, p2.y, c.x, c.y, c.z);
+                        w[3 * S::CS] = c.x;
+                        w[4 * S::CS] = c.y;
+                        w[5 * S::CS] = c.z;
+                    }
+                    return ok;
+                };
+                unsigned redo = row_ok && !odd ? 0u : (1u << S::U) - 1u;
+#pragma unroll
+                for (int u = 0; u < S::U; ++u) redo |= term(u, std::false_type{}) ? 0u : 1u << u;
+                while (redo) {
+                    const int u = __ffs(redo) - 1;
+                    redo &= redo - 1;
+                    const int j = t * S::TJ + sub + u * S::SUBS;
+                    if (j < n && j != i) {
+                        term(u, std::true_type{});
+                    } else {  // no term: adding +0 leaves a running sum as it is
+#pragma unroll
+                        for (int p = 0; p < S::PLANES; ++p) o[u * S::SUBS * R + p * S::CS] = 0.0;
+                    }
+                }
             }
-            const double rr = sqrt(X * X + Y * Y + Z * Z);
-            const double r3 = ipow3(rr);
-            const double Fx = sfx[k], Fy = sfy[k], Fz = sfz[k];
-            const double inv_r = 1 / rr;
-            const double xy = (X * Y) / r3, xz = (X * Z) / r3, yz = (Y * Z) / r3;
-            Cx += eta * ((inv_r + (X * X) / r3) * Fx + xy * Fy + xz * Fz);
-            Cy += eta * (xy * Fx + (inv_r + (Y * Y) / r3) * Fy + yz * Fz);
-            Cz += eta * (xz * Fx + yz * Fy + (inv_r + (Z * Z) / r3) * Fz);
-            if (CORR) corr_pair64(corr, X, Y, Z, Fx, Fy, Fz, Cx, Cy, Cz);
+            odd = __syncthreads_or(0);
+        }
+    } else {
+        const int q = tid - ORD_P;
+        const int comp = q / R, row = q % R;
+        const bool chain = comp < 3;
+        double acc = 0.0;
+        for (int t = 0; t <= ntiles; ++t) {
+            // tile t + 1: the loads are issued before the sums of tile t - 1, used after them
+            const int j0 = (t + 1) * S::TJ;
+            double v[S::LOADS][NSRC];
+            if (t + 1 < ntiles) {
+#pragma unroll
+                for (int l = 0; l < S::LOADS; ++l) {
+                    const int k = q + l * S::ADD_T, j = j0 + k;
+#pragma unroll
+                    for (int w = 0; w < NSRC; ++w) v[l][w] = k < S::TJ && j < n ? src[w][j] : 0.0;
+                }
+            }
+            if (t > 0 && chain) {
+                const double *p = terms + ((t - 1) & 1) * S::PLANES * S::CS + comp * S::CS + row;
+#pragma unroll 16
+                for (int k = 0; k < S::TJ; ++k) {
+                    acc += p[k * R];
+                    if (KIND == OSEEN64_CORR) acc += p[3 * S::CS + k * R];
+                }
+            }
+            odd = 0;
+            if (t + 1 < ntiles) {
+                double *const s = stage + ((t + 1) & 1) * NV * S::TJ;
+#pragma unroll
+                for (int l = 0; l < S::LOADS; ++l) {
+                    const int k = q + l * S::ADD_T;
+                    if (k < S::TJ) odd |= !put(s + NV * k, v[l], j0 + k < n) && j0 + k < n;
+                }
+            }
+            __syncthreads_or(odd);
+        }
+        const int i = row0 + row;
+        if (chain && i < n) {
+            if (KIND == OSEEN64_CORR) acc += a.corr.g_self * (comp == 0 ? a.fx : comp == 1 ? a.fy : a.fz)[i];
+            (comp == 0 ? a.ox : comp == 1 ? a.oy : a.oz)[i] = acc;
         }
     }
-    if (CORR && active) {
-        Cx += corr.g_self * fx[i];
-        Cy += corr.g_self * fy[i];
-        Cz += corr.g_self * fz[i];
-    }
-    if (active) {
-        vx[i] = Cx;
-        vy[i] = Cy;
-        vz[i] = Cz;
-    }
+}
+
+template <int R, bool PER, int KIND>
+static void launch_ordered(const Ord64Args &a, cudaStream_t s) {
+    using S = OrdShape<R, KIND>;
+    ordered_pass_kernel<R, PER, KIND><<<ceil_div(a.n, R), S::THREADS, S::SMEM, counted(s)>>>(a);
+}
+
+template <int R, int KIND>
+static cudaError_t allow_smem() {
+    cudaError_t e = cudaFuncSetAttribute(ordered_pass_kernel<R, true, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)OrdShape<R, KIND>::SMEM);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(ordered_pass_kernel<R, false, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)OrdShape<R, KIND>::SMEM);
+}
+
+template <int KIND>
+static cudaError_t allow_smem_all() {
+    cudaError_t e = allow_smem<4, KIND>();
+    if (e == cudaSuccess) e = allow_smem<8, KIND>();
+    if (e == cudaSuccess) e = allow_smem<16, KIND>();
+    return e;
+}
+
+// Shared-memory limits of the ordered passes, set at context creation (a pass may run under capture).
+int direct_fp64_prepare(dem_ctx *ctx) {
+    cudaError_t e = allow_smem_all<FORCE64>();
+    if (e == cudaSuccess) e = allow_smem_all<OSEEN64>();
+    if (e == cudaSuccess) e = allow_smem_all<OSEEN64_CORR>();
+    return dem_check_cuda(ctx, e, "direct_fp64 attributes");
+}
+
+// Rows per CTA.  Few rows per CTA spread a small box over the SMs (one wave: 3 CTAs of 4 rows per SM hold
+// 12 n_SM = 1,776 rows); more rows per CTA use the adders' lanes fully.  Force + convection, periodic, us,
+// with 4 / 8 / 16 rows: n = 500: 26 / 31 / 36; 1,776: 66 / 69 / 77; 2,500: 140 / 126 / 149; 10,000: 1,516 /
+// 1,215 / 1,240; 13,000: 2,526 / 1,891 / 1,921; 16,000: 3,871 / 2,910 / 2,716; 30,000: 12,998 / 9,951 / 9,246
+// (32 rows are slower throughout).  With the correction, bound by its gathers, 4 and 8 rows are as fast
+// as 16 or faster from n = 4,097 to 16,384.
+template <int KIND>
+static void run_ordered(const dem_ctx *ctx, const Ord64Args &a, int periodic, cudaStream_t s) {
+    const int sm = ctx->sm_count;
+    if (a.n <= 12 * sm)
+        periodic ? launch_ordered<4, true, KIND>(a, s) : launch_ordered<4, false, KIND>(a, s);
+    else if (KIND == OSEEN64_CORR || a.n <= 95 * sm)
+        periodic ? launch_ordered<8, true, KIND>(a, s) : launch_ordered<8, false, KIND>(a, s);
+    else
+        periodic ? launch_ordered<16, true, KIND>(a, s) : launch_ordered<16, false, KIND>(a, s);
 }
 
 int launch_direct_forces_fp64(dem_ctx *ctx, int n, const double *x, const double *y, const double *z,
                               const double *r, double m_const, double L, int periodic, double *fx, double *fy,
                               double *fz, cudaStream_t s) {
-    const int grid = ceil_div(n, F64_THREADS);
+    const Ord64Args a{n, x, y, z, r, nullptr, nullptr, nullptr, m_const, L, L * 0.5, CorrDev{}, fx, fy, fz};
     dem_prof_begin(ctx, "fp64_force_pass", s);
-    if (periodic)
-        direct_force_fp64_kernel<true><<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, r, m_const, L, L * 0.5, fx, fy, fz);
-    else
-        direct_force_fp64_kernel<false><<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, r, m_const, L, L * 0.5, fx, fy, fz);
+    run_ordered<FORCE64>(ctx, a, periodic, s);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "direct_force_fp64");
 }
@@ -162,15 +365,9 @@ int launch_direct_forces_fp64(dem_ctx *ctx, int n, const double *x, const double
 int launch_direct_convection_fp64(dem_ctx *ctx, int n, const double *x, const double *y, const double *z,
                                   const double *fx, const double *fy, const double *fz, double eta, double L,
                                   int periodic, double *vx, double *vy, double *vz, cudaStream_t s) {
-    const int grid = ceil_div(n, F64_THREADS);
+    const Ord64Args a{n, x, y, z, nullptr, fx, fy, fz, eta, L, L * 0.5, CorrDev{}, vx, vy, vz};
     dem_prof_begin(ctx, "fp64_convection_pass", s);
-    const CorrDev none{};
-    if (periodic)
-        direct_convection_fp64_kernel<true, false>
-            <<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, fx, fy, fz, eta, L, L * 0.5, none, vx, vy, vz);
-    else
-        direct_convection_fp64_kernel<false, false>
-            <<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, fx, fy, fz, eta, L, L * 0.5, none, vx, vy, vz);
+    run_ordered<OSEEN64>(ctx, a, periodic, s);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "direct_convection_fp64");
 }
@@ -179,15 +376,9 @@ int launch_direct_convection_fp64_corr(dem_ctx *ctx, const dem_corr *c, int n, c
                                        const double *z, const double *fx, const double *fy, const double *fz,
                                        double eta, double L, int periodic, double *vx, double *vy, double *vz,
                                        cudaStream_t s) {
-    const int grid = ceil_div(n, F64_THREADS);
-    const CorrDev cv = corr_view(c);
+    const Ord64Args a{n, x, y, z, nullptr, fx, fy, fz, eta, L, L * 0.5, corr_view(c), vx, vy, vz};
     dem_prof_begin(ctx, "fp64_convection_corr_pass", s);
-    if (periodic)
-        direct_convection_fp64_kernel<true, true>
-            <<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, fx, fy, fz, eta, L, L * 0.5, cv, vx, vy, vz);
-    else
-        direct_convection_fp64_kernel<false, true>
-            <<<grid, F64_THREADS, 0, counted(s)>>>(n, x, y, z, fx, fy, fz, eta, L, L * 0.5, cv, vx, vy, vz);
+    run_ordered<OSEEN64_CORR>(ctx, a, periodic, s);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "direct_convection_fp64_corr");
 }
