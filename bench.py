@@ -768,9 +768,9 @@ def run_adjoint(args, device):
 
 
 # FP64 operations of vjp_pair_kernel per ordered pair (adds and multiplies 1, FMA 2), counted
-# from its source: separation and |d|^-1 (Newton) 20, force-term Hessian and radius terms 76,
-# the two Oseen K terms 90
-FLOPS_VJP_PAIR = 186
+# from its source per unordered pair (each evaluated once): separation and |d|^-1 24, force-term
+# Hessian and radius terms 46, the two Oseen K terms 65, their sum into both sides 15
+FLOPS_VJP_PAIR = 150 / 2
 FP64_PEAK_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12  # SMs x FP64 lanes x 2 flop x max SM clock
 
 
@@ -806,7 +806,7 @@ def report_adjoint(args, res):
                                "steps; loss = mean squared z displacement + pair softplus((2.5 (r_i+r_j) - |r_ij|) "
                                "/ 1 um); gradients w.r.t. initial positions, radii and |E|",
                    **res},
-        "roofline": {"kernel": "vjp_pass (vjp_pair_kernel + its fixed-order finish)", "bound": "fp64_pipe",
+        "roofline": {"kernel": "vjp_pass (vjp_pair_kernel + its fixed-order sums)", "bound": "fp64_pipe",
                      "achieved": achieved, "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s",
                      "frac": achieved / FP64_PEAK_TFLOPS,
                      "peak_source": "148 SMs x 64 FP64 lanes x 2 flop x 1965 MHz (max SM clock); "

@@ -23,108 +23,146 @@
 //   * d(sum_k lambda_k.V_k)/dx_i = eta sum_{j != i} [K(e_ij; lambda_i, F_j) + K(e_ij; lambda_j, F_i)],
 //       K(e; a, b) = grad_e(a^T G(e) b) = [(e.b) a + (e.a) b - (a.b) e] / |e|^3 - 3 (a.e)(e.b) e / |e|^5;
 //   * d(lambda_i.F_i / (gamma r_i))/dr_i = -lambda_i.F_i / (gamma r_i^2).
-// Everything is FP64.  Both O(N^2) passes (mu and the pair terms) cut the j range
-// into chunks, one CTA per (128 droplets i, chunk): at N = 16,384 one thread per i
-// alone would fill 128 CTAs on 148 SMs.  The chunks' partial sums are added in
-// chunk order (deterministic).  1 / |d| comes from an FP32 estimate refined by
-// two Newton steps in FP64 (rsqrt_nr), not from an IEEE square root and division.
+// Everything is FP64.  Both O(N^2) passes evaluate every unordered pair once: G is
+// even, and a pair's gradient
+//   g = (m/3) r_i^3 r_j^3 H(d) (mu_j - mu_i) - eta [K(d; lambda_i, F_j) + K(d; lambda_j, F_i)]
+// enters x_i with + and x_j with -, its S = (mu_j - mu_i).f(d) enters r_i as r_j^3 S
+// and r_j as r_i^3 S.  With q = dz^2 / r^2, n = mu_j - mu_i, p = d.n / r^2:
+//   H n   = r^-5 [(15 q - 3) n + ((15 - 105 q) p + 30 dz nz / r^2) d + (30 dz p - 6 nz) z],
+//   n.f   = r^-5 [(5 q - 1) d.n - 2 dz nz].
 #include "common.cuh"
+#include "ieee64.cuh"
 
 namespace dem {
 
-constexpr int VJP_THREADS = 128;
-constexpr int VJP_TILE = 128;
-
-// 1 / sqrt(x) for x > 0 by Newton's method on f(y) = y^-2 - x: y <- y (3 - x y^2) / 2,
-// which converges quadratically, from the FP32 estimate rsqrtf (relative error
-// ~2^-23): two steps reach FP64 rounding.  Outside FP32's range: sqrt and a division.
-__device__ __forceinline__ double rsqrt_nr(double x) {
-    if (!(x > 1e-30 && x < 1e30)) return 1.0 / sqrt(x);
-    double y = (double)rsqrtf((float)x);
-    const double hx = 0.5 * x;
-    y = y * fma(-hx, y * y, 1.5);
-    y = y * fma(-hx, y * y, 1.5);
-    return y;
-}
-
-// The j range [j0, j1) of split blockIdx.y.
-struct VjpSplit {
-    int chunk;  // j per split (a multiple of VJP_TILE)
-    int splits;
+// ---------------------------------------------------------------------------
+// Block pairs.  A CTA of W warps takes a pair of blocks (I <= J) of B = 32 W IPT
+// droplets.  A lane keeps IPT droplets of I in registers; a warp goes through
+// block J 32 droplets at a time, lane l meeting droplet (l + s) mod 32 in step
+// s, and the j-side sums travel with their droplet (one shuffle per step), so
+// both sides of a pair are added without atomics.  The warps' j-side sums meet
+// in shared memory in warp order; every block pair leaves one record per side,
+// and the finish kernels add a droplet's records in block order
+// (deterministic).  A diagonal pair (I == J) meets every ordered pair and keeps
+// its i side.
+//
+// Bound: the FP64 pipe, ~106 operations per unordered pair, ~39 in the mu pass
+// (before: one thread per droplet and j chunk, every ordered pair).  Mu / pair
+// pass with their sums, periodic, us, before -> now: n = 2,000 40 / 85 -> 30 / 44;
+// 16,384 970 / 3,050 -> 480 / 1,080 (72 % of the pipe's issue rate by that count).
+// ---------------------------------------------------------------------------
+struct VjpBlocks {
+    int nb;           // blocks
+    int row0;         // first block row of this launch
+    long long item0;  // block pairs before it
 };
 
-// Oseen pass applied to lambda, partial sums of split s: part[(3 s + c) n + i] = sum_j G(e_ij) lambda_j
-// over the split's j != i (e = mic(x_i - x_j), G(e) = I / |e| + e e^T / |e|^3).
-template <bool PER>
-__global__ void __launch_bounds__(VJP_THREADS) vjp_oseen_kernel(int n, const double *__restrict__ x,
-                                                                const double *__restrict__ y,
-                                                                const double *__restrict__ z,
-                                                                const double *__restrict__ lx,
-                                                                const double *__restrict__ ly,
-                                                                const double *__restrict__ lz, double L, double halfL,
-                                                                VjpSplit sp, double *__restrict__ part) {
-    __shared__ double sx[VJP_TILE], sy[VJP_TILE], sz[VJP_TILE], slx[VJP_TILE], sly[VJP_TILE], slz[VJP_TILE];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    const double xi = active ? x[i] : 0.0, yi = active ? y[i] : 0.0, zi = active ? z[i] : 0.0;
-    const int j0 = blockIdx.y * sp.chunk, j1 = min(n, j0 + sp.chunk);
-    double ux = 0.0, uy = 0.0, uz = 0.0;
-    for (int t0 = j0; t0 < j1; t0 += VJP_TILE) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < VJP_TILE; k += blockDim.x) {
-            const int j = t0 + k;
-            if (j < j1) {
-                sx[k] = x[j];
-                sy[k] = y[j];
-                sz[k] = z[j];
-                slx[k] = lx[j];
-                sly[k] = ly[j];
-                slz[k] = lz[j];
-            }
-        }
-        __syncthreads();
-        const int cnt = min(VJP_TILE, j1 - t0);
-        if (!active) continue;
-        for (int k = 0; k < cnt; ++k) {
-            if (t0 + k == i) continue;
-            double ex = xi - sx[k], ey = yi - sy[k], ez = zi - sz[k];
-            if (PER) {
-                ex = mic64(ex, L, halfL);
-                ey = mic64(ey, L, halfL);
-                ez = mic64(ez, L, halfL);
-            }
-            const double r2 = ex * ex + ey * ey + ez * ez;
-            const double ir = rsqrt_nr(r2), ir2 = ir * ir;
-            const double el = (ex * slx[k] + ey * sly[k] + ez * slz[k]) * ir2;
-            ux += (slx[k] + ex * el) * ir;
-            uy += (sly[k] + ey * el) * ir;
-            uz += (slz[k] + ez * el) * ir;
-        }
-    }
-    if (!active) return;
-    double *o = part + (size_t)blockIdx.y * 3 * n;
-    o[i] = ux;
-    o[n + i] = uy;
-    o[2 * (size_t)n + i] = uz;
+__host__ __device__ __forceinline__ long long pairs_before(int nb, int row) {
+    return (long long)row * nb - (long long)row * (row - 1) / 2;
 }
 
-// mu_i = eta sum_s part_s + lambda_i / (gamma r_i)  (splits in order)
-__global__ void vjp_mu_kernel(int n, int splits, const double *__restrict__ part, const double *__restrict__ r,
-                              const double *__restrict__ lx, const double *__restrict__ ly,
-                              const double *__restrict__ lz, double eta, double stokes, double *__restrict__ mx,
-                              double *__restrict__ my, double *__restrict__ mz) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double ux = 0.0, uy = 0.0, uz = 0.0;
-        for (int s = 0; s < splits; ++s) {
-            const double *o = part + (size_t)s * 3 * n;
-            ux += o[i];
-            uy += o[n + i];
-            uz += o[2 * (size_t)n + i];
+__device__ __forceinline__ void block_pair(const VjpBlocks &b, int &I, int &J) {
+    const long long t = b.item0 + blockIdx.x;
+    const double h = b.nb + 0.5;
+    int i = (int)(h - sqrt(fmax(h * h - 2.0 * (double)t, 0.0)));
+    i = max(b.row0, min(i, b.nb - 1));
+    while (i > b.row0 && pairs_before(b.nb, i) > t) --i;
+    while (i + 1 < b.nb && pairs_before(b.nb, i + 1) <= t) ++i;
+    I = i;
+    J = i + (int)(t - pairs_before(b.nb, i));
+}
+
+template <bool PER>
+__device__ __forceinline__ double image64(double d, double L, double halfL) {
+    return PER ? mic64(d, L, halfL) : d;
+}
+
+// 1 / sqrt(x) to ~1 ulp: seed y (2^-20), e = 1 - x y^2 and y (1 + e / 2 + 3/8 e^2).
+__device__ __forceinline__ double rsqrt64(double x) {
+    const double y = rsqrt_seed(x);
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y, fma(0.375, e, 0.5) * e, y);
+}
+
+__device__ __forceinline__ double from_next_lane(double v, int lane) {
+    return __shfl_sync(0xffffffffu, v, (lane + 1) & 31);
+}
+
+// mu pass: u_i = sum_j G(d_ij) lambda_j.  Records: [item][side][3][B].
+template <int W, int IPT, bool PER>
+__global__ void __launch_bounds__(32 * W) vjp_oseen_kernel(int n, const double *__restrict__ x,
+                                                           const double *__restrict__ y, const double *__restrict__ z,
+                                                           const double *__restrict__ lx,
+                                                           const double *__restrict__ ly,
+                                                           const double *__restrict__ lz, double L, double halfL,
+                                                           VjpBlocks blocks, double *__restrict__ records) {
+    constexpr int B = 32 * W * IPT;
+    __shared__ double sj[W][6][32];
+    __shared__ double plane[W][3][B];
+    int I, J;
+    block_pair(blocks, I, J);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double *const src[6] = {x, y, z, lx, ly, lz};
+    double xi[IPT], yi[IPT], zi[IPT], ax[IPT], ay[IPT], az[IPT], ux[IPT], uy[IPT], uz[IPT];
+    int ii[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int i = I * B + (warp * IPT + k) * 32 + lane;
+        ii[k] = i < n ? i : -1;
+        xi[k] = i < n ? x[i] : 0.0, yi[k] = i < n ? y[i] : 0.0, zi[k] = i < n ? z[i] : 0.0;
+        ax[k] = i < n ? lx[i] : 0.0, ay[k] = i < n ? ly[i] : 0.0, az[k] = i < n ? lz[i] : 0.0;
+        ux[k] = uy[k] = uz[k] = 0.0;
+    }
+    for (int t = 0; t < B / 32; ++t) {
+        const int jb = J * B + 32 * t;
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sj[warp][c][lane] = jb + lane < n ? src[c][jb + lane] : 0.0;
+        __syncwarp();
+        double vx = 0.0, vy = 0.0, vz = 0.0;
+        for (int s = 0; s < 32; ++s) {
+            const int jl = (lane + s) & 31, j = jb + jl;
+            const double *const q = &sj[warp][0][jl];
+            const double xj = q[0], yj = q[32], zj = q[64], bx = q[96], by = q[128], bz = q[160];
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) {
+                const double dx = image64<PER>(xj - xi[k], L, halfL), dy = image64<PER>(yj - yi[k], L, halfL),
+                             dz = image64<PER>(zj - zi[k], L, halfL);
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const double ir = j < n && ii[k] >= 0 && ii[k] != j ? rsqrt64(r2) : 0.0, ir3 = ir * ir * ir;
+                const double cj = (dx * bx + dy * by + dz * bz) * ir3;
+                const double ci = (dx * ax[k] + dy * ay[k] + dz * az[k]) * ir3;
+                ux[k] = fma(bx, ir, fma(dx, cj, ux[k]));
+                uy[k] = fma(by, ir, fma(dy, cj, uy[k]));
+                uz[k] = fma(bz, ir, fma(dz, cj, uz[k]));
+                vx = fma(ax[k], ir, fma(dx, ci, vx));
+                vy = fma(ay[k], ir, fma(dy, ci, vy));
+                vz = fma(az[k], ir, fma(dz, ci, vz));
+            }
+            vx = from_next_lane(vx, lane);
+            vy = from_next_lane(vy, lane);
+            vz = from_next_lane(vz, lane);
         }
-        const double a = 1.0 / (stokes * r[i]);
-        mx[i] = eta * ux + a * lx[i];
-        my[i] = eta * uy + a * ly[i];
-        mz[i] = eta * uz + a * lz[i];
+        plane[warp][0][32 * t + lane] = vx;
+        plane[warp][1][32 * t + lane] = vy;
+        plane[warp][2][32 * t + lane] = vz;
+    }
+    double *const o = records + (size_t)blockIdx.x * 6 * B;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int p = (warp * IPT + k) * 32 + lane;
+        o[p] = ux[k];
+        o[B + p] = uy[k];
+        o[2 * B + p] = uz[k];
+    }
+    if (I == J) return;
+    __syncthreads();
+    for (int p = threadIdx.x; p < 3 * B; p += 32 * W) {
+        const int c = p / B, k = p % B;
+        double v = plane[0][c][k];
+#pragma unroll
+        for (int w = 1; w < W; ++w) v += plane[w][c][k];
+        o[3 * B + p] = v;
     }
 }
 
@@ -136,156 +174,225 @@ struct VjpArgs {
     const double *mx, *my, *mz;  // mu: cotangent on F
     double m_const, eta, stokes, L, halfL;
     double *gx, *gy, *gz, *gr;
-    VjpSplit sp;
-    double *part;  // [splits][7][n] partial sums (vjp_pair_kernel)
 };
 
-// Partial sums of split s over its j != i:
-//   part[(7 s + 0..2) n + i] = sum_j r_j^3 H(d_ij) (mu_j - mu_i)   (force terms, cut |d| > r_i + r_j)
-//   part[(7 s + 3) n + i]    = sum_j r_j^3 (mu_j - mu_i).f(d_ij)
-//   part[(7 s + 4..6) n + i] = sum_j K(e_ij; lambda_i, F_j) + K(e_ij; lambda_j, F_i)
-template <bool PER>
-__global__ void __launch_bounds__(VJP_THREADS) vjp_pair_kernel(const VjpArgs a) {
-    __shared__ double sx[VJP_TILE], sy[VJP_TILE], sz[VJP_TILE], sr[VJP_TILE];
-    __shared__ double smx[VJP_TILE], smy[VJP_TILE], smz[VJP_TILE];
-    __shared__ double slx[VJP_TILE], sly[VJP_TILE], slz[VJP_TILE];
-    __shared__ double sfx[VJP_TILE], sfy[VJP_TILE], sfz[VJP_TILE];
+// Pair terms.  Records: [item][side][4][B]: the gradient's three components (i side +, j side - g) and
+// sum of r_other^3 S.
+template <int W, int IPT, bool PER>
+__global__ void __launch_bounds__(32 * W) vjp_pair_kernel(const VjpArgs a, VjpBlocks blocks,
+                                                          double *__restrict__ records) {
+    constexpr int B = 32 * W * IPT;
+    __shared__ double sj[W][14][32];
+    __shared__ double plane[W][4][B];
+    int I, J;
+    block_pair(blocks, I, J);
     const int n = a.n;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < n;
-    double xi = 0, yi = 0, zi = 0, ri = 0, mix = 0, miy = 0, miz = 0, lix = 0, liy = 0, liz = 0, fix = 0, fiy = 0,
-           fiz = 0;
-    if (active) {
-        xi = a.x[i];
-        yi = a.y[i];
-        zi = a.z[i];
-        ri = a.r[i];
-        mix = a.mx[i];
-        miy = a.my[i];
-        miz = a.mz[i];
-        lix = a.lx[i];
-        liy = a.ly[i];
-        liz = a.lz[i];
-        fix = a.fx[i];
-        fiy = a.fy[i];
-        fiz = a.fz[i];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double *const src[13] = {a.x, a.y, a.z, a.r, a.mx, a.my, a.mz, a.lx, a.ly, a.lz, a.fx, a.fy, a.fz};
+    double v[IPT][13], wi[IPT];
+    double gx[IPT], gy[IPT], gz[IPT], gs[IPT];
+    int ii[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int i = I * B + (warp * IPT + k) * 32 + lane;
+        ii[k] = i < n ? i : -1;
+#pragma unroll
+        for (int c = 0; c < 13; ++c) v[k][c] = i < n ? src[c][i] : 0.0;
+        wi[k] = ipow3(v[k][3]);
+        gx[k] = gy[k] = gz[k] = gs[k] = 0.0;
     }
-    double hx = 0, hy = 0, hz = 0;  // sum_j r_j^3 H (mu_j - mu_i)
-    double gR = 0;                  // sum_j r_j^3 (mu_j - mu_i).f
-    double kx = 0, ky = 0, kz = 0;  // sum_j K(e; lambda_i, F_j) + K(e; lambda_j, F_i)
-    const int j0 = blockIdx.y * a.sp.chunk, j1 = min(n, j0 + a.sp.chunk);
-    for (int t0 = j0; t0 < j1; t0 += VJP_TILE) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < VJP_TILE; k += blockDim.x) {
-            const int j = t0 + k;
-            if (j < j1) {
-                sx[k] = a.x[j];
-                sy[k] = a.y[j];
-                sz[k] = a.z[j];
-                sr[k] = a.r[j];
-                smx[k] = a.mx[j];
-                smy[k] = a.my[j];
-                smz[k] = a.mz[j];
-                slx[k] = a.lx[j];
-                sly[k] = a.ly[j];
-                slz[k] = a.lz[j];
-                sfx[k] = a.fx[j];
-                sfy[k] = a.fy[j];
-                sfz[k] = a.fz[j];
-            }
-        }
-        __syncthreads();
-        const int cnt = min(VJP_TILE, j1 - t0);
-        if (!active) continue;
-        for (int k = 0; k < cnt; ++k) {
-            if (t0 + k == i) continue;
-            double dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;  // d = x_j - x_i
-            if (PER) {
-                dx = mic64(dx, a.L, a.halfL);
-                dy = mic64(dy, a.L, a.halfL);
-                dz = mic64(dz, a.L, a.halfL);
-            }
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            const double ir = rsqrt_nr(r2), ir2 = ir * ir, ir3 = ir2 * ir, ir5 = ir3 * ir2;
-            if (r2 * ir > ri + sr[k]) {  // force terms (contact cut of the forward pass, |d| = r2 / |d|)
-                const double ir7 = ir5 * ir2, ir9 = ir7 * ir2;
-                const double w = ipow3(sr[k]);
-                const double nx = smx[k] - mix, ny = smy[k] - miy, nz = smz[k] - miz;
+    const double m3 = a.m_const / 3.0;
+    for (int t = 0; t < B / 32; ++t) {
+        const int jb = J * B + 32 * t;
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 13; ++c) sj[warp][c][lane] = jb + lane < n ? src[c][jb + lane] : 0.0;
+        sj[warp][13][lane] = jb + lane < n ? ipow3(a.r[jb + lane]) : 0.0;
+        __syncwarp();
+        double hx = 0.0, hy = 0.0, hz = 0.0, hs = 0.0;  // droplet j's side: - sum g, sum r_i^3 S
+        for (int s = 0; s < 32; ++s) {
+            const int jl = (lane + s) & 31, j = jb + jl;
+            const double *const q = &sj[warp][0][jl];
+            const double wj = q[13 * 32];
+            const double ljx = q[7 * 32], ljy = q[8 * 32], ljz = q[9 * 32];
+            const double fjx = q[10 * 32], fjy = q[11 * 32], fjz = q[12 * 32];
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) {
+                const double lix = v[k][7], liy = v[k][8], liz = v[k][9], fix = v[k][10], fiy = v[k][11], fiz = v[k][12];
+                const double dx = image64<PER>(q[0] - v[k][0], a.L, a.halfL),
+                             dy = image64<PER>(q[32] - v[k][1], a.L, a.halfL),
+                             dz = image64<PER>(q[64] - v[k][2], a.L, a.halfL);
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const double ir = j < n && ii[k] >= 0 && ii[k] != j ? rsqrt64(r2) : 0.0;
+                const double ir2 = ir * ir, ir3 = ir2 * ir, ir5 = ir3 * ir2;
+                // force terms, inside the contact cut of the forward pass (|d| = r2 / |d|) none
+                const double c5 = r2 * ir > v[k][3] + q[3 * 32] ? ir5 : 0.0;
+                const double nx = q[4 * 32] - v[k][4], ny = q[5 * 32] - v[k][5], nz = q[6 * 32] - v[k][6];
                 const double dn = dx * nx + dy * ny + dz * nz;
-                const double z2 = dz * dz;
-                const double c1 = -3.0 * ir5 + 15.0 * z2 * ir7;
-                const double c2 = (15.0 * ir7 - 105.0 * z2 * ir9) * dn;
-                const double c3 = 30.0 * dz * ir7 * nz;
-                hx += w * (c1 * nx + c2 * dx + c3 * dx);
-                hy += w * (c1 * ny + c2 * dy + c3 * dy);
-                hz += w * (c1 * nz + c2 * dz - 6.0 * ir5 * nz + 30.0 * dz * ir7 * dn + c3 * dz);
-                const double axy = (4.0 * z2 - dx * dx - dy * dy) * ir7;
-                const double az = (2.0 * z2 - 3.0 * dx * dx - 3.0 * dy * dy) * ir7;
-                gR += w * (nx * dx * axy + ny * dy * axy + nz * dz * az);
+                const double u = dz * ir2, qz = dz * u, p = dn * ir2;
+                const double a0 = fma(15.0, qz, -3.0);
+                const double a1 = fma(30.0 * u, nz, fma(-105.0, qz, 15.0) * p);
+                const double a2 = fma(30.0 * dz, p, -6.0 * nz);
+                const double S = c5 * fma(fma(5.0, qz, -1.0), dn, -2.0 * dz * nz);
+                const double wf = (m3 * wi[k]) * wj * c5;
+                // Oseen terms
+                const double dl = dx * lix + dy * liy + dz * liz, ef = dx * fjx + dy * fjy + dz * fjz;
+                const double el = dx * ljx + dy * ljy + dz * ljz, df = dx * fix + dy * fiy + dz * fiz;
+                const double ab = lix * fjx + liy * fjy + liz * fjz + ljx * fix + ljy * fiy + ljz * fiz;
+                const double cd = fma(-3.0 * ir2, fma(dl, ef, el * df), -ab);
+                const double kf = -a.eta * ir3;
+                const double kx = fma(ef, lix, fma(dl, fjx, fma(df, ljx, fma(el, fix, cd * dx))));
+                const double ky = fma(ef, liy, fma(dl, fjy, fma(df, ljy, fma(el, fiy, cd * dy))));
+                const double kz = fma(ef, liz, fma(dl, fjz, fma(df, ljz, fma(el, fiz, cd * dz))));
+                const double tx = fma(wf, fma(a0, nx, a1 * dx), kf * kx);
+                const double ty = fma(wf, fma(a0, ny, a1 * dy), kf * ky);
+                const double tz = fma(wf, fma(a0, nz, fma(a1, dz, a2)), kf * kz);
+                gx[k] += tx;
+                gy[k] += ty;
+                gz[k] += tz;
+                gs[k] = fma(wj, S, gs[k]);
+                hx -= tx;
+                hy -= ty;
+                hz -= tz;
+                hs = fma(wi[k], S, hs);
             }
-            // Oseen terms with e = x_i - x_j = -d (no cut)
-            const double ex = -dx, ey = -dy, ez = -dz;
-            {  // K(e; lambda_i, F_j)
-                const double ax_ = lix, ay_ = liy, az_ = liz, bx = sfx[k], by = sfy[k], bz = sfz[k];
-                const double eb = ex * bx + ey * by + ez * bz, ea = ex * ax_ + ey * ay_ + ez * az_;
-                const double ab = ax_ * bx + ay_ * by + az_ * bz;
-                const double q = 3.0 * ea * eb * ir5;
-                kx += (eb * ax_ + ea * bx - ab * ex) * ir3 - q * ex;
-                ky += (eb * ay_ + ea * by - ab * ey) * ir3 - q * ey;
-                kz += (eb * az_ + ea * bz - ab * ez) * ir3 - q * ez;
-            }
-            {  // K(e; lambda_j, F_i)
-                const double ax_ = slx[k], ay_ = sly[k], az_ = slz[k], bx = fix, by = fiy, bz = fiz;
-                const double eb = ex * bx + ey * by + ez * bz, ea = ex * ax_ + ey * ay_ + ez * az_;
-                const double ab = ax_ * bx + ay_ * by + az_ * bz;
-                const double q = 3.0 * ea * eb * ir5;
-                kx += (eb * ax_ + ea * bx - ab * ex) * ir3 - q * ex;
-                ky += (eb * ay_ + ea * by - ab * ey) * ir3 - q * ey;
-                kz += (eb * az_ + ea * bz - ab * ez) * ir3 - q * ez;
-            }
+            hx = from_next_lane(hx, lane);
+            hy = from_next_lane(hy, lane);
+            hz = from_next_lane(hz, lane);
+            hs = from_next_lane(hs, lane);
         }
+        plane[warp][0][32 * t + lane] = hx;
+        plane[warp][1][32 * t + lane] = hy;
+        plane[warp][2][32 * t + lane] = hz;
+        plane[warp][3][32 * t + lane] = hs;
     }
-    if (!active) return;
-    double *o = a.part + (size_t)blockIdx.y * 7 * n;
-    o[i] = hx;
-    o[n + i] = hy;
-    o[2 * (size_t)n + i] = hz;
-    o[3 * (size_t)n + i] = gR;
-    o[4 * (size_t)n + i] = kx;
-    o[5 * (size_t)n + i] = ky;
-    o[6 * (size_t)n + i] = kz;
+    double *const o = records + (size_t)blockIdx.x * 8 * B;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int p = (warp * IPT + k) * 32 + lane;
+        o[p] = gx[k];
+        o[B + p] = gy[k];
+        o[2 * B + p] = gz[k];
+        o[3 * B + p] = gs[k];
+    }
+    if (I == J) return;
+    __syncthreads();
+    for (int p = threadIdx.x; p < 4 * B; p += 32 * W) {
+        const int c = p / B, k = p % B;
+        double w = plane[0][c][k];
+#pragma unroll
+        for (int ww = 1; ww < W; ++ww) w += plane[ww][c][k];
+        o[4 * B + p] = w;
+    }
 }
 
-// The gradients from the splits' partial sums (in split order).
-__global__ void vjp_finish_kernel(const VjpArgs a) {
+// sums[c][i] (+)= droplet i's records of block rows [row0, row1), in block order.
+template <int NC>
+__global__ void vjp_sum_kernel(int n, int B, int nb, int row0, int row1, const double *__restrict__ records,
+                               double *__restrict__ sums) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)NC * n) return;
+    const int c = (int)(t / n), i = (int)(t % n), b = i / B, k = i % B;
+    const long long base = pairs_before(nb, row0);
+    double v = row0 ? sums[t] : 0.0;
+    for (int I = row0; I < min(b, row1); ++I)  // j side of (I, b)
+        v += records[((size_t)(pairs_before(nb, I) + (b - I) - base) * 2 * NC + NC + c) * B + k];
+    if (b >= row0 && b < row1)  // i side of (b, J)
+        for (int J = b; J < nb; ++J)
+            v += records[((size_t)(pairs_before(nb, b) + (J - b) - base) * 2 * NC + c) * B + k];
+    sums[t] = v;
+}
+
+// mu_i = eta sum_i + lambda_i / (gamma r_i)
+__global__ void vjp_mu_kernel(int n, const double *__restrict__ sums, const double *__restrict__ r,
+                              const double *__restrict__ lx, const double *__restrict__ ly,
+                              const double *__restrict__ lz, double eta, double stokes, double *__restrict__ mx,
+                              double *__restrict__ my, double *__restrict__ mz) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double a = 1.0 / (stokes * r[i]);
+        mx[i] = eta * sums[i] + a * lx[i];
+        my[i] = eta * sums[n + i] + a * ly[i];
+        mz[i] = eta * sums[2 * (size_t)n + i] + a * lz[i];
+    }
+}
+
+// The gradients from the sums.
+__global__ void vjp_finish_kernel(const VjpArgs a, const double *__restrict__ sums) {
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double v[7] = {0, 0, 0, 0, 0, 0, 0};
-        for (int s = 0; s < a.sp.splits; ++s) {
-            const double *o = a.part + (size_t)s * 7 * n;
-#pragma unroll
-            for (int c = 0; c < 7; ++c) v[c] += o[(size_t)c * n + i];
-        }
         const double ri = a.r[i];
-        const double cf = a.m_const / 3.0 * ipow3(ri);
-        a.gx[i] = cf * v[0] + a.eta * v[4];
-        a.gy[i] = cf * v[1] + a.eta * v[5];
-        a.gz[i] = cf * v[2] + a.eta * v[6];
+        a.gx[i] = sums[i];
+        a.gy[i] = sums[n + i];
+        a.gz[i] = sums[2 * (size_t)n + i];
         const double lf = a.lx[i] * a.fx[i] + a.ly[i] * a.fy[i] + a.lz[i] * a.fz[i];
-        a.gr[i] = -3.0 * a.m_const * ri * ri * v[3] - lf / (a.stokes * ri * ri);
+        a.gr[i] = -3.0 * a.m_const * ri * ri * sums[3 * (size_t)n + i] - lf / (a.stokes * ri * ri);
     }
 }
 
-// j chunks such that the (i block, chunk) grid holds >= 8 CTAs per SM
-static VjpSplit vjp_split(const dem_ctx *ctx, int n) {
-    const int iblocks = ceil_div(n, VJP_THREADS);
-    const int want = max(1, ceil_div(8 * ctx->sm_count, iblocks));
-    int chunk = ceil_div(ceil_div(n, want), VJP_TILE) * VJP_TILE;
-    if (chunk < VJP_TILE) chunk = VJP_TILE;
-    VjpSplit sp;
-    sp.chunk = chunk;
-    sp.splits = max(1, ceil_div(n, chunk));
-    return sp;
+struct VjpShape {
+    int warps, ipt, B, nb;
+    int rows;      // block rows per launch
+    size_t bytes;  // records of one launch and the sums
+};
+
+// Records of a launch stay below this; a larger n goes through its block rows in several launches.
+constexpr size_t VJP_RECORD_BYTES = size_t(2) << 30;
+
+// Blocks of 32 droplets fill the SMs with a small box's block pairs, blocks of 64 (two droplets per lane
+// share the loads and shuffles) are faster from n ~ 2,000 on, and one CTA of four warps on a block of 128
+// halves the records of a large n.  Both passes, periodic, us, with 32 / 64 / 128: n = 1,000: 45 / 64 / 70;
+// 2,000: 73 / 70 / 75; 3,000: 114 / 95 / 120; 8,000: 460 / 412 / 430; 16,384: 1,792 / 1,554 / 1,589.
+static VjpShape vjp_shape(int n) {
+    VjpShape s;
+    s.warps = n > 32768 ? 4 : 1;
+    s.ipt = n >= 2000 && n <= 32768 ? 2 : 1;
+    s.B = 32 * s.warps * s.ipt;
+    s.nb = ceil_div(n, s.B);
+    const size_t item = sizeof(double) * 8 * s.B;
+    s.rows = s.nb;
+    while (s.rows > 1 && (size_t)pairs_before(s.nb, s.rows) * item > VJP_RECORD_BYTES) s.rows = (s.rows + 1) / 2;
+    s.bytes = (size_t)pairs_before(s.nb, s.rows) * item + sizeof(double) * 4 * n;
+    return s;
+}
+
+template <int W, int IPT>
+static void launch_rows(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, int row0, int row1, double *records,
+                        cudaStream_t s) {
+    const VjpBlocks b{sh.nb, row0, pairs_before(sh.nb, row0)};
+    const unsigned grid = (unsigned)(pairs_before(sh.nb, row1) - b.item0);
+    if (pair) {
+        if (per)
+            vjp_pair_kernel<W, IPT, true><<<grid, 32 * W, 0, counted(s)>>>(a, b, records);
+        else
+            vjp_pair_kernel<W, IPT, false><<<grid, 32 * W, 0, counted(s)>>>(a, b, records);
+    } else {
+        if (per)
+            vjp_oseen_kernel<W, IPT, true>
+                <<<grid, 32 * W, 0, counted(s)>>>(a.n, a.x, a.y, a.z, a.lx, a.ly, a.lz, a.L, a.halfL, b, records);
+        else
+            vjp_oseen_kernel<W, IPT, false>
+                <<<grid, 32 * W, 0, counted(s)>>>(a.n, a.x, a.y, a.z, a.lx, a.ly, a.lz, a.L, a.halfL, b, records);
+    }
+}
+
+// One O(N^2) pass (mu or pair terms) into sums[3 or 4][n].
+static void vjp_pass(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, double *records, double *sums,
+                     cudaStream_t s) {
+    for (int row0 = 0; row0 < sh.nb; row0 += sh.rows) {
+        const int row1 = min(sh.nb, row0 + sh.rows);
+        if (sh.warps == 4)
+            launch_rows<4, 1>(sh, a, per, pair, row0, row1, records, s);
+        else if (sh.ipt == 2)
+            launch_rows<1, 2>(sh, a, per, pair, row0, row1, records, s);
+        else
+            launch_rows<1, 1>(sh, a, per, pair, row0, row1, records, s);
+        if (pair)
+            vjp_sum_kernel<4><<<ceil_div(4LL * a.n, 128), 128, 0, counted(s)>>>(a.n, sh.B, sh.nb, row0, row1, records,
+                                                                               sums);
+        else
+            vjp_sum_kernel<3><<<ceil_div(3LL * a.n, 128), 128, 0, counted(s)>>>(a.n, sh.B, sh.nb, row0, row1, records,
+                                                                               sums);
+    }
 }
 
 int launch_direct_vjp(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, const double *r,
@@ -294,28 +401,21 @@ int launch_direct_vjp(dem_ctx *ctx, int n, const double *x, const double *y, con
                       double *mx, double *my, double *mz, double *gx, double *gy, double *gz, double *gr,
                       cudaStream_t s) {
     if (n == 0) return DEM_OK;
-    const VjpSplit sp = vjp_split(ctx, n);
-    // partial sums: [splits][7][n] doubles in the context's [splits][3][capacity] array
-    int rc = dem_ensure_partials(ctx, ceil_div(7 * sp.splits, 3));
+    const VjpShape sh = vjp_shape(n);
+    // the context's partial sums, [splits][3][capacity]: the sums, then the records
+    int rc = dem_ensure_partials(ctx, ceil_div((int64_t)(sh.bytes / sizeof(double)), 3LL * ctx->capacity));
     if (rc) return rc;
-    double *part = ctx->partial;
-    const dim3 grid(ceil_div(n, VJP_THREADS), sp.splits);
+    double *sums = ctx->partial, *records = sums + 4 * (size_t)n;
     const int egrid = min(ceil_div(n, 256), 8 * ctx->sm_count);
-    // mu = eta (Oseen pass applied to lambda) + lambda / (gamma r)
-    if (periodic)
-        vjp_oseen_kernel<true><<<grid, VJP_THREADS, 0, counted(s)>>>(n, x, y, z, lx, ly, lz, L, 0.5 * L, sp, part);
-    else
-        vjp_oseen_kernel<false><<<grid, VJP_THREADS, 0, counted(s)>>>(n, x, y, z, lx, ly, lz, L, 0.5 * L, sp, part);
-    vjp_mu_kernel<<<egrid, 256, 0, counted(s)>>>(n, sp.splits, part, r, lx, ly, lz, eta, stokes, mx, my, mz);
+    const VjpArgs a{n, x, y, z, r, fx, fy, fz, lx, ly, lz, mx, my, mz, m_const, eta, stokes, L, 0.5 * L, gx, gy, gz, gr};
+    dem_prof_begin(ctx, "vjp_mu_pass", s);
+    vjp_pass(sh, a, periodic != 0, false, records, sums, s);
+    vjp_mu_kernel<<<egrid, 256, 0, counted(s)>>>(n, sums, r, lx, ly, lz, eta, stokes, mx, my, mz);
+    dem_prof_end(ctx, s);
     if ((rc = dem_check_launch(ctx, "vjp mu"))) return rc;
-    VjpArgs a{n, x, y, z, r, fx, fy, fz, lx, ly, lz, mx, my, mz, m_const, eta, stokes, L, 0.5 * L, gx, gy, gz, gr,
-              sp, part};
     dem_prof_begin(ctx, "vjp_pass", s);
-    if (periodic)
-        vjp_pair_kernel<true><<<grid, VJP_THREADS, 0, counted(s)>>>(a);
-    else
-        vjp_pair_kernel<false><<<grid, VJP_THREADS, 0, counted(s)>>>(a);
-    vjp_finish_kernel<<<egrid, 256, 0, counted(s)>>>(a);
+    vjp_pass(sh, a, periodic != 0, true, records, sums, s);
+    vjp_finish_kernel<<<egrid, 256, 0, counted(s)>>>(a, sums);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "vjp pair pass");
 }
