@@ -100,7 +100,8 @@ DEM_API int dem_profile_reset(dem_ctx *ctx);
                                        minimum image and the tests) */
 
 /* Tuning of the mixed-precision direct kernels (0 keeps the current value).
- *   i_per_thread  i-particles register-blocked per thread (1, 2, 4 or 8;
+ *   i_per_thread  i-particles register-blocked per thread (1, 2, 4 or 8; an
+ *                 upper bound where the split schedule chooses its j-chunks;
  *                 the symmetric schedule uses 1, 2 or 4)
  *   threads       threads per CTA of the split schedule (64..512, multiple of 32)
  *   j_splits      number of j-chunks of the split schedule (>=1; 0 = auto)

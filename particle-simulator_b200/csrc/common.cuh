@@ -58,6 +58,12 @@ struct dem_ctx {
     } sym_order;
     bool sym_reuse_order = false;
     int partial_splits = 0;
+    // mixed, split schedule: resident CTAs per SM for this thread count, [force][periodic][1, 2, 4, 8 rows] (0: not
+    // asked yet)
+    struct {
+        int threads = 0;
+        int ctas[2][2][4] = {};
+    } split_occ;
     double *dscratch = nullptr;     // 8 doubles: reductions (max radius, ...)
     int32_t *cell_hash = nullptr;   // hash bucket per particle
     int32_t *cell_xyz = nullptr;    // cell coordinates per particle, [3][capacity] (the count pass)

@@ -25,7 +25,7 @@ extern "C" void dem_count_replayed_launches(unsigned long long k) { dem_count_la
 namespace dem {
 int sym_sorted_prepare(dem_ctx *ctx);
 int direct_fp64_prepare(dem_ctx *ctx);
-int direct_plan(const dem_ctx *ctx, int n, int periodic, int *schedule, int *i_per_thread, int *threads,
+int direct_plan(dem_ctx *ctx, int n, int periodic, int *schedule, int *i_per_thread, int *threads,
                 long long *ctas, int *j_splits);
 }
 
@@ -289,7 +289,7 @@ int dem_direct_get_tuning(const dem_ctx *ctx, int *i_per_thread, int *threads, i
 int dem_direct_plan(const dem_ctx *ctx, int n, int periodic, int *schedule, int *i_per_thread, int *threads,
                     long long *ctas, int *j_splits) {
     if (!ctx || n < 0 || !schedule || !i_per_thread || !threads || !ctas || !j_splits) return DEM_E_INVALID;
-    return dem::direct_plan(ctx, n, periodic, schedule, i_per_thread, threads, ctas, j_splits);
+    return dem::direct_plan(const_cast<dem_ctx *>(ctx), n, periodic, schedule, i_per_thread, threads, ctas, j_splits);
 }
 
 }  // extern "C"

@@ -18,7 +18,7 @@ constexpr double MIC_MARGIN = 1.0 / 262144.0;  // 2^-18
 
 struct MixedArgs {
     int n;
-    int j_chunk;  // j per split (multiple of TJ)
+    int j_chunk;  // j per split (multiple of FLUSH)
     const float4 *pos4;  // (x, y, z, r^3) scaled / (x, y, z, -)
     const float *krf;    // force pass: k_f * r (scaled)
     const float4 *frc4;  // convection pass: (F scaled, k_o * r scaled)
@@ -170,17 +170,29 @@ static __global__ void maxabs_kernel(int n, const double *__restrict__ a, const 
     if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
 }
 
+__device__ __forceinline__ void pack_position(int i, const double *__restrict__ x, const double *__restrict__ y,
+                                              const double *__restrict__ z, const double *__restrict__ r, double center,
+                                              double s, double k_near, float4 *__restrict__ pos4,
+                                              float *__restrict__ kr) {
+    const double rs = r[i] * s;
+    pos4[i] = make_float4((float)((x[i] - center) * s), (float)((y[i] - center) * s), (float)((z[i] - center) * s),
+                          (float)(rs * rs * rs));
+    if (kr) kr[i] = (float)(k_near * rs);
+}
+
+__device__ __forceinline__ void pack_force(int i, const double *__restrict__ fx, const double *__restrict__ fy,
+                                           const double *__restrict__ fz, const double *__restrict__ r, double s,
+                                           double q, double k_near, float4 *__restrict__ frc4) {
+    frc4[i] = make_float4((float)(fx[i] * q), (float)(fy[i] * q), (float)(fz[i] * q), (float)(k_near * r[i] * s));
+}
+
 static __global__ void prep_positions_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
                                       const double *__restrict__ z, const double *__restrict__ r, double center,
                                       const unsigned long long *__restrict__ scales, double k_near,
                                       float4 *__restrict__ pos4, float *__restrict__ kr) {
     const double s = pow2_inv_of(scales[0]);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double rs = r[i] * s;
-        pos4[i] = make_float4((float)((x[i] - center) * s), (float)((y[i] - center) * s), (float)((z[i] - center) * s),
-                              (float)(rs * rs * rs));
-        if (kr) kr[i] = (float)(k_near * rs);
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        pack_position(i, x, y, z, r, center, s, k_near, pos4, kr);
 }
 
 static __global__ void prep_forces_kernel(int n, const double *__restrict__ fx, const double *__restrict__ fy,
@@ -190,7 +202,7 @@ static __global__ void prep_forces_kernel(int n, const double *__restrict__ fx, 
     const double s = pow2_inv_of(scales[0]);
     const double q = pow2_inv_of(scales[1]);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        frc4[i] = make_float4((float)(fx[i] * q), (float)(fy[i] * q), (float)(fz[i] * q), (float)(k_near * r[i] * s));
+        pack_force(i, fx, fy, fz, r, s, q, k_near, frc4);
 }
 
 // out_c[i] = factor_i * sum_s partial[s][c][i]
