@@ -47,6 +47,8 @@
 // derivatives of |d|^-n are n(n+2) [S_abc r^-(n+4) - (n+4) x_a x_b x_c r^-(n+6)]
 // and those of dz^2 |d|^-5 follow from the product rule; contracted with Q they
 // give the closed form of quad_force below.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -229,53 +231,182 @@ __global__ void __launch_bounds__(RS_T) rs_hist_kernel(int n, const uint32_t *__
     hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
+// The lanes of `live` whose 8-bit digit equals this lane's: one vote per bit.  (match.any, which took its
+// place, is serial in the distinct digits: scatter passes at n = 285,000 10.4 -> 5.8 us, at 2^20 21 -> 16.)
+__device__ __forceinline__ unsigned digit_peers(int d, unsigned live) {
+    unsigned peers = live;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1;
+        const unsigned ones = __ballot_sync(0xffffffffu, one);
+        peers &= one ? ones : ~ones;
+    }
+    return peers;
+}
+
 // Stable scatter: warp w ranks items [w * 256, (w + 1) * 256) of the tile in
-// order, 32 at a time, grouping equal digits with match.any.
+// order, 32 at a time, grouping equal digits by votes (digit_peers).
 __global__ void __launch_bounds__(RS_T) rs_scatter_kernel(int n, const uint32_t *__restrict__ kin,
                                                           const int32_t *__restrict__ vin, uint32_t *__restrict__ kout,
                                                           int32_t *__restrict__ vout, int shift, int tiles,
                                                           const int32_t *__restrict__ off) {
     constexpr int W = RS_T / 32;
     __shared__ int cnt[W][256];
-    __shared__ int run[W][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int d = threadIdx.x; d < W * 256; d += RS_T) (&cnt[0][0])[d] = 0;
     __syncthreads();
     const int base = blockIdx.x * RS_TILE + w * (32 * RS_ITEMS);
     const unsigned lt = (1u << lane) - 1u;
+    uint32_t key[RS_ITEMS];
+    int val[RS_ITEMS], pos[RS_ITEMS];
+#pragma unroll
     for (int r = 0; r < RS_ITEMS; ++r) {
         const int i = base + r * 32 + lane;
-        const bool valid = i < n;
-        const int d = valid ? (int)((kin[i] >> shift) & 255u) : 256 + lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        if (valid && (peers & lt) == 0) cnt[w][d] += __popc(peers);
+        key[r] = i < n ? kin[i] : 0u;
+        val[r] = i < n ? vin[i] : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; ++r) {
+        const bool valid = base + r * 32 + lane < n;
+        const int d = (int)((key[r] >> shift) & 255u);
+        const unsigned peers = digit_peers(d, __ballot_sync(0xffffffffu, valid));
+        const int before = cnt[w][d];
         __syncwarp();
+        if (valid && (peers & lt) == 0) cnt[w][d] = before + __popc(peers);
+        __syncwarp();
+        pos[r] = before + __popc(peers & lt);
     }
     __syncthreads();
     {
         const int d = threadIdx.x;  // RS_T == 256 digits
         int acc = off[d * tiles + blockIdx.x];
         for (int ww = 0; ww < W; ++ww) {
-            run[ww][d] = acc;
-            acc += cnt[ww][d];
+            const int c = cnt[ww][d];
+            cnt[ww][d] = acc;
+            acc += c;
         }
     }
     __syncthreads();
+#pragma unroll
     for (int r = 0; r < RS_ITEMS; ++r) {
-        const int i = base + r * 32 + lane;
-        const bool valid = i < n;
-        const uint32_t key = valid ? kin[i] : 0u;
-        const int d = valid ? (int)((key >> shift) & 255u) : 256 + lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        int pos = 0;
-        if (valid) pos = run[w][d] + __popc(peers & lt);
-        __syncwarp();
-        if (valid) {
-            kout[pos] = key;
-            vout[pos] = vin[i];
-            if ((peers & lt) == 0) run[w][d] += __popc(peers);
+        if (base + r * 32 + lane < n) {
+            const int p = cnt[w][(key[r] >> shift) & 255u] + pos[r];
+            kout[p] = key[r];
+            vout[p] = val[r];
         }
-        __syncwarp();
+    }
+}
+
+// The sort of up to RC_MAX pairs in one launch: a cluster of 8 CTAs, each on its contiguous eighth of the
+// sequence (warp w of a CTA on its contiguous share, `items` rounds of 32), PASSES stable 8-bit passes from
+// `shift` on.  Per pass a warp counts and ranks its digits (digit_peers), a CTA its warps, and the cluster
+// its CTAs, whose 256 totals each CTA reads over distributed shared memory; the pairs are scattered through
+// global memory between the two buffers.  The 20 launches it replaces (histogram, three scan kernels, scatter
+// per pass) took 82 us of kernel time at n = 16,384 and 91 at 65,536, each a few microseconds of latency on a
+// handful of CTAs; this takes 20 us at 8,192, 27 at 16,384 and 64 at 65,536 (8 SMs: its votes and shared-memory
+// ranking; level with the tiled passes there).  A symmetric force + convection call at 8,192: 586 -> 507 us.
+constexpr int RC_T = 1024, RC_CTAS = 8, RC_ITEMS = 8, RC_MAX = RC_T * RC_CTAS * RC_ITEMS;
+
+template <int PASSES>
+__global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(RC_T)
+    rs_cluster_kernel(int n, int items, int shift, uint32_t *k0, int32_t *v0, uint32_t *k1, int32_t *v1) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int W = RC_T / 32, PARTS = RC_T / 256;
+    __shared__ int cnt[W][256];       // a warp's digit counts, then the CTA's pairs before it with that digit
+    __shared__ int part[PARTS][256];  // the same of W / PARTS warps
+    __shared__ int hist[256];         // the CTA's digit counts (read by the cluster)
+    __shared__ int base[256];         // first position of the CTA's pairs with a digit
+    __shared__ int wsum[8];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, rank = (int)cluster.block_rank();
+    const unsigned lt = (1u << lane) - 1u;
+    const int first = (rank * W + w) * 32 * items + lane;
+    for (int pass = 0; pass < PASSES; ++pass, shift += 8) {
+        const uint32_t *kin = pass & 1 ? k1 : k0;
+        const int32_t *vin = pass & 1 ? v1 : v0;
+        uint32_t *kout = pass & 1 ? k0 : k1;
+        int32_t *vout = pass & 1 ? v0 : v1;
+        uint32_t key[RC_ITEMS];
+        int val[RC_ITEMS], pos[RC_ITEMS];
+#pragma unroll
+        for (int r = 0; r < RC_ITEMS; ++r) {
+            const int i = first + 32 * r;
+            const bool valid = r < items && i < n;
+            key[r] = valid ? kin[i] : 0u;
+            val[r] = valid ? vin[i] : 0;
+        }
+        for (int d = tid; d < W * 256; d += RC_T) (&cnt[0][0])[d] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RC_ITEMS; ++r) {
+            if (r >= items) break;
+            const bool valid = first + 32 * r < n;
+            const int d = (int)((key[r] >> shift) & 255u);
+            const unsigned peers = digit_peers(d, __ballot_sync(0xffffffffu, valid));
+            const int before = cnt[w][d];
+            __syncwarp();
+            if (valid && (peers & lt) == 0) cnt[w][d] = before + __popc(peers);
+            __syncwarp();
+            pos[r] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        const int d = tid & 255, q = tid >> 8;
+        {
+            int run = 0;
+#pragma unroll
+            for (int k = 0; k < W / PARTS; ++k) {
+                const int c = cnt[q * (W / PARTS) + k][d];
+                cnt[q * (W / PARTS) + k][d] = run;
+                run += c;
+            }
+            part[q][d] = run;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            int run = 0;
+#pragma unroll
+            for (int p = 0; p < PARTS; ++p) {
+                const int c = part[p][d];
+                part[p][d] = run;
+                run += c;
+            }
+            hist[d] = run;
+        }
+        cluster.sync();
+        int total = 0, before = 0, inc = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int c = 0; c < RC_CTAS; ++c) {
+                const int h = cluster.map_shared_rank(hist, c)[d];
+                total += h;
+                before += c < rank ? h : 0;
+            }
+            inc = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            if (lane == 31) wsum[w] = inc;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            int b = inc - total + before;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) b += k < w ? wsum[k] : 0;
+            base[d] = b;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RC_ITEMS; ++r) {
+            if (r < items && first + 32 * r < n) {
+                const int dd = (int)((key[r] >> shift) & 255u);
+                const int p = base[dd] + part[w / (W / PARTS)][dd] + cnt[w][dd] + pos[r];
+                kout[p] = key[r];
+                vout[p] = val[r];
+            }
+        }
+        cluster.sync();  // the pairs are in place, and nobody reads this pass's counts any more
     }
 }
 
@@ -1186,9 +1317,16 @@ int morton_order(dem_ctx *ctx, int n, const double *x, const double *y, const do
     return radix_sort_pairs(ctx, n, w, s);
 }
 
+static int rc_items(int n) { return std::max(1, (n + RC_T * RC_CTAS - 1) / (RC_T * RC_CTAS)); }
+
 int radix_pass(dem_ctx *ctx, int n, const uint32_t *kin, const int32_t *vin, uint32_t *kout, int32_t *vout, int shift,
                int32_t *hist, cudaStream_t s) {
     const int tiles = (n + RS_TILE - 1) / RS_TILE;
+    if (n <= RC_MAX) {
+        rs_cluster_kernel<1><<<RC_CTAS, RC_T, 0, counted(s)>>>(n, rc_items(n), shift, const_cast<uint32_t *>(kin),
+                                                               const_cast<int32_t *>(vin), kout, vout);
+        return dem_check_launch(ctx, "radix pass");
+    }
     int32_t *off = hist + 256 * (size_t)tiles + 1;
     rs_hist_kernel<<<tiles, RS_T, 0, counted(s)>>>(n, kin, shift, tiles, hist);
     int rc = exclusive_scan<int32_t, int32_t>(ctx, hist, off, 256LL * tiles, s);
@@ -1198,6 +1336,11 @@ int radix_pass(dem_ctx *ctx, int n, const uint32_t *kin, const int32_t *vin, uin
 }
 
 int radix_sort_pairs(dem_ctx *ctx, int n, const MortonWs &w, cudaStream_t s) {
+    if (n <= RC_MAX) {
+        rs_cluster_kernel<4><<<RC_CTAS, RC_T, 0, counted(s)>>>(n, rc_items(n), 0, w.keys[0], w.idx[0], w.keys[1],
+                                                               w.idx[1]);
+        return dem_check_launch(ctx, "morton order");
+    }
     const int tiles = (n + RS_TILE - 1) / RS_TILE;
     int32_t *hist = w.hist, *off = w.hist + 256 * (size_t)tiles + 1;
     int cur = 0, rc;
