@@ -270,14 +270,13 @@ def hbm_peak():
 # Algorithmic bytes of the memory-bound kernels (what a kernel that touches
 # every input and output once would move):
 #   hash detection (csrc/hash.cu): per droplet its position and radius (32 B
-#     read), its bucket id (4 B written, 4 B read) and bucket slot (4 B written,
-#     4 B read); per table slot its start (4 B written, 4 B read); 8 B per pair.
+#     read); 8 B per pair.
 #   Morton build (csrc/bh.cu): per droplet positions (24 B read), key (4 B
 #     written), 4 radix passes over (key, index) (16 B each), the gather of
 #     position and radius into key order (32 B read, 32 B written); per node its
 #     records (~140 B written).
-def hash_bytes(n, table, pairs):
-    return 48 * n + 8 * table + 8 * pairs
+def hash_bytes(n, pairs):
+    return 32 * n + 8 * pairs
 
 
 def morton_build_bytes(n, nodes):
@@ -967,9 +966,8 @@ def report_tree(args, res):
     peak_b, src_b = hbm_peak()
     mb = []
     if "hash_detect" in res["kern"]:
-        table = 1 << max(int(2 * n - 1).bit_length(), 0)
-        mb.append(hbm_entry("hash detection", res["kern"]["hash_detect"], hash_bytes(n, table, 0), peak_b, src_b,
-                            "48 N + 8 table + 8 pairs"))
+        mb.append(hbm_entry("hash detection", res["kern"]["hash_detect"], hash_bytes(n, 0), peak_b, src_b,
+                            "32 N + 8 pairs"))
     if "bh_build" in res["kern"]:
         mb.append(hbm_entry("Morton octree build (keys, radix sort, gather, levels, node moments)",
                             res["kern"]["bh_build"], morton_build_bytes(n, st["node_count"]), peak_b, src_b,
@@ -1481,11 +1479,10 @@ def main():
                                           f"x {n} columns, extrapolated ({c['sample_s']:.1f} s of CPU work)"}
     if "hash_detect" in kern:
         peak_b, src_b = hbm_peak()
-        table = 1 << max(int(2 * n - 1).bit_length(), 0)
         n_det = int(round(sum(nt) / len(nt)))  # droplets per detection in the timed window
-        line["memory_bound"] = [hbm_entry("hash detection (assign, scans, scatter, bucket records, count, write)",
-                                          kern["hash_detect"][0] / kern["hash_detect"][1], hash_bytes(n_det, table, 0),
-                                          peak_b, src_b, "48 N + 8 table + 8 pairs")]
+        line["memory_bound"] = [hbm_entry("hash detection (radii, search cells, scatter, search, row scan, rows)",
+                                          kern["hash_detect"][0] / kern["hash_detect"][1], hash_bytes(n_det, 0),
+                                          peak_b, src_b, "32 N + 8 pairs")]
     if "fp64" in res:
         f64 = res["fp64"]
         fp64_sps = 1000.0 / f64["ms_per_step"]

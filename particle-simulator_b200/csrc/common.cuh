@@ -23,6 +23,14 @@ struct dem_mixed_tuning {
     int schedule = 0;  // DEM_SCHED_AUTO / DEM_SCHED_SPLIT / DEM_SCHED_SYMMETRIC
 };
 
+constexpr int SEARCH_MISC_WORDS = 8;
+// Buckets of the collision search for n particles: a power of two >= 2 n.
+inline uint32_t search_buckets(int64_t n) {
+    uint32_t b = 1024;
+    while (b < 2 * (uint64_t)n && b < 0x80000000u) b <<= 1;
+    return b;
+}
+
 struct dem_prof_rec {
     const char *name;
     cudaEvent_t start, stop;
@@ -65,17 +73,16 @@ struct dem_ctx {
         int ctas[2][2][4] = {};
     } split_occ;
     double *dscratch = nullptr;     // 8 doubles: reductions (max radius, ...)
-    int32_t *cell_hash = nullptr;   // hash bucket per particle
-    int32_t *cell_xyz = nullptr;    // cell coordinates per particle, [3][capacity] (the count pass)
-    int32_t *bucket_count = nullptr;  // table
-    int32_t *bucket_start = nullptr;  // table (exclusive scan)
-    int32_t *bucket_cursor = nullptr; // table
-    int32_t *sorted_idx = nullptr;    // particles grouped by bucket
-    double2 *hash_pos = nullptr;      // (x, y), (z, r) of the particles in bucket order (2 per particle)
-    float4 *hash_pos32 = nullptr;     // (x, y, z, r) rounded to FP32, bucket order (the far test)
-    int32_t *pair_count = nullptr;    // per particle (capacity + 1)
+    // collision detection (hash.cu): zeroed words (SEARCH_MISC_WORDS, row counts, bucket counts), per particle
+    // (bucket, rank in it, cell id), (first slot, particles) per bucket, FP32 records with (particle, cell id) in
+    // bucket order (2 each), the pair list and its rows (search_list_cap each)
+    int32_t *search_zero = nullptr;
+    int4 *search_key = nullptr;
+    int2 *search_bucket = nullptr;
+    float4 *search_rec = nullptr;
+    int2 *search_list = nullptr;
+    uint32_t search_list_cap = 0;
     int64_t *pair_offset = nullptr;   // per particle (capacity + 1), exclusive scan
-    int64_t table_capacity = 0;
     int32_t *flags = nullptr;       // merge: 1 = consumed
     int32_t *keep_off = nullptr;    // merge: exclusive scan of survivors (capacity + 1)
     double *merged_buf = nullptr;   // merge: 4 doubles per merged droplet
@@ -92,7 +99,6 @@ cudaStream_t counted(cudaStream_t s);
 int dem_set_error(dem_ctx *ctx, int code, const std::string &msg);
 int dem_check_cuda(dem_ctx *ctx, cudaError_t e, const char *where);
 int dem_check_launch(dem_ctx *ctx, const char *where);
-int dem_ensure_table(dem_ctx *ctx, int64_t table_size);
 int dem_ensure_partials(dem_ctx *ctx, int splits);
 int dem_ensure_sym_partials(dem_ctx *ctx, size_t bytes);
 // Records a CUDA event before/after a kernel launch when profiling is on.

@@ -1,4 +1,5 @@
 // ctx.cu -- context, workspace and error handling of libdem_b200.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -46,16 +47,6 @@ static int grow(dem_ctx *ctx, T **p, size_t count, const char *what) {
     if (*p) cudaFree(*p);
     *p = nullptr;
     return dem_check_cuda(ctx, cudaMalloc((void **)p, sizeof(T) * (count > 0 ? count : 1)), what);
-}
-
-int dem_ensure_table(dem_ctx *ctx, int64_t table_size) {
-    if (table_size <= ctx->table_capacity) return DEM_OK;
-    int rc;
-    if ((rc = grow(ctx, &ctx->bucket_count, (size_t)table_size, "hash table"))) return rc;
-    if ((rc = grow(ctx, &ctx->bucket_start, (size_t)table_size + 1, "hash table"))) return rc;
-    if ((rc = grow(ctx, &ctx->bucket_cursor, (size_t)table_size, "hash table"))) return rc;
-    ctx->table_capacity = table_size;
-    return DEM_OK;
 }
 
 int dem_ensure_partials(dem_ctx *ctx, int splits) {
@@ -174,12 +165,13 @@ int dem_ctx_reserve(dem_ctx *ctx, int capacity) {
     const size_t n = (size_t)capacity;
     if ((rc = grow(ctx, &ctx->pack_a, n, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->pack_b, n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->cell_hash, n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->cell_xyz, 3 * n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->sorted_idx, n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->hash_pos, 2 * n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->hash_pos32, n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->pair_count, n + 1, "workspace"))) return rc;
+    const size_t buckets = search_buckets((int64_t)n);
+    if ((rc = grow(ctx, &ctx->search_zero, SEARCH_MISC_WORDS + n + buckets, "workspace"))) return rc;
+    if ((rc = grow(ctx, &ctx->search_key, n, "workspace"))) return rc;
+    if ((rc = grow(ctx, &ctx->search_bucket, buckets, "workspace"))) return rc;
+    if ((rc = grow(ctx, &ctx->search_rec, 2 * n, "workspace"))) return rc;
+    ctx->search_list_cap = (uint32_t)std::min<size_t>(2 * n + 65536, 0x7fffffffu);
+    if ((rc = grow(ctx, &ctx->search_list, 2 * (size_t)ctx->search_list_cap, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->pair_offset, n + 1, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->flags, n + 1, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->keep_off, n + 1, "workspace"))) return rc;
@@ -227,8 +219,8 @@ void dem_ctx_destroy(dem_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     void *ptrs[] = {ctx->d_err,         ctx->pack_a,      ctx->pack_b,     ctx->partial,    ctx->dscratch,
-                    ctx->cell_hash,     ctx->cell_xyz, ctx->bucket_count, ctx->bucket_start, ctx->bucket_cursor, ctx->sorted_idx, ctx->hash_pos, ctx->hash_pos32,
-                    ctx->pair_count,    ctx->pair_offset, ctx->flags,      ctx->keep_off,   ctx->merged_buf,
+                    ctx->search_zero,   ctx->search_key,  ctx->search_bucket, ctx->search_rec, ctx->search_list,
+                    ctx->pair_offset,   ctx->flags,       ctx->keep_off,   ctx->merged_buf,
                     ctx->merged_cnt,    ctx->scan_tmp,    ctx->sym_partial};
     for (void *p : ptrs)
         if (p) cudaFree(p);

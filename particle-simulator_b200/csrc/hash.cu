@@ -5,24 +5,31 @@
 //   _hash_cell :74-76, _assign_cells :79-112, _prefix_sum :115-123,
 //   _scatter_particles :126-132, _detect_collisions :135-229, detect :233-316.
 //
-// Pipeline (all on the device, no host synchronisation):
-//   1. max radius            -> cell = 2 max r, grid = max(1, ceil(L / cell))
-//   2. bucket of every droplet, bucket counts (atomics)
-//   3. exclusive scan of the counts (bucket starts), scatter into buckets
-//   4. per droplet i: the distinct hash buckets of its 27 neighbour cells; count
-//      the j > i in them with MIC distance <= r_i + r_j (threads take the
-//      droplets in bucket order, so the lanes of a warp share candidate lists)
-//   5. exclusive scan of the per-i counts -> pair offsets (lexicographic order)
-//   6. per droplet i: write its pairs, sort its j's ascending
+// The reference compares a droplet i with every j > i in the hash buckets of the
+// 27 cells around its own, cells of twice the LARGEST radius: ~120 candidates per
+// droplet for lognormal radii at 2 % volume fraction, of which one in 250 touches
+// something.  Its pair set is {touching pairs} intersected with {pairs whose
+// bucket the 27 cells reach}; the second condition is a property of two droplets
+// alone, so it is checked for touching pairs only and these are found on a search
+// grid of their own (hashed cells of 4.5 MEAN radii):
+//   1. maximum and mean radius; the last CTA derives both grids
+//   2. search cell of every droplet, rank in its bucket (atomics)
+//   3. bucket starts (any order: one CTA-wide scan and one atomic per CTA)
+//   4. FP32 records in bucket order
+//   5. per droplet i: the search cells within 2 r_i (i is the pair's larger droplet,
+//      ties by index, so this covers the contact distance); candidates pass an FP32
+//      far test, then the reference's contact test in FP64, then the reachability
+//      test: list of pairs, pairs per row, raw hits
+//   6. exclusive scan of the row counts, pairs into their rows, rows sorted by rank
+// A droplet reads ~6 cells and ~2 candidates at 2 % volume fraction.
 // Memory roofline: the chain is bounded by HBM and latency, not arithmetic.  Its
-// algorithmic bytes per detection are 48 N + 8 T + 8 K (N droplets, T table
-// slots, K pairs): position and radius read once (32 B), bucket id and bucket
-// slot written and read (16 B), bucket starts written and read (8 B per slot),
-// 8 B per pair written.
-// The candidate set of a droplet is exactly the reference's (the same buckets,
-// including buckets shared by aliased cells), and the distance test is the
-// same IEEE expression (this file is compiled with -fmad=false), so the pair
-// set is bit-identical to the reference's np.unique output.
+// algorithmic bytes per detection are 32 N + 8 K (N droplets, K pairs): position and
+// radius read once, 8 B per pair written.  Kernels, periodic, before (27 buckets per
+// droplet) -> now: N = 2^20 765 -> 240 us (the search 580 -> 138, bound by L2
+// latency), N = 2,000 118 -> 55, of which most are gaps between short kernels.
+// The contact test is the same IEEE expression as the reference's (this file is
+// compiled with -fmad=false) and does not depend on the order of the two droplets,
+// so the pair set is bit-identical to the reference's np.unique output.
 #include "common.cuh"
 #include "scan.cuh"
 
@@ -63,9 +70,7 @@ __global__ void max_kernel(int n, const double *__restrict__ r, unsigned long lo
 // reference's pair set, kept bit-exact).  even_cells = 1 (the generator's own
 // use): grid = floor(L / (2 max r)) whole cells of side L / grid >= 2 max r, so
 // every touching pair is compared across the periodic faces too.
-__global__ void hash_params_kernel(const unsigned long long *__restrict__ slot, double L, int even_cells,
-                                   HashParams *__restrict__ hp) {
-    const double max_radius = from_ordered_bits(*slot);
+__device__ __forceinline__ HashParams hash_params(double max_radius, double L, int even_cells) {
     double cell = 2.0 * max_radius;  // :258
     HashParams p;
     p.valid = cell > 0 ? 1 : 0;  // :259-260
@@ -75,7 +80,11 @@ __global__ void hash_params_kernel(const unsigned long long *__restrict__ slot, 
     if (even_cells && p.valid) cell = L / g;
     p.cell = cell;
     p.grid = (int32_t)g;  // :262
-    *hp = p;
+    return p;
+}
+
+__global__ void hash_params_kernel(const unsigned long long *__restrict__ slot, double L, HashParams *__restrict__ hp) {
+    *hp = hash_params(from_ordered_bits(*slot), L, 0);
 }
 
 __device__ __forceinline__ int32_t hash_cell(int32_t ix, int32_t iy, int32_t iz, int32_t mask) {
@@ -102,8 +111,7 @@ __device__ __forceinline__ int32_t cell_coord(double p, double cell, int32_t gri
 
 __global__ void assign_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
                               const double *__restrict__ z, const HashParams *__restrict__ hp, int periodic,
-                              int32_t mask, int32_t *__restrict__ cell_hash, int32_t *__restrict__ bucket_count,
-                              int32_t *__restrict__ cell_xyz) {
+                              int32_t mask, int32_t *__restrict__ cell_hash, int32_t *__restrict__ bucket_count) {
     const HashParams p = *hp;
     if (!p.valid) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -112,11 +120,6 @@ __global__ void assign_kernel(int n, const double *__restrict__ x, const double 
         const int32_t iz = cell_coord(z[i], p.cell, p.grid, periodic);
         const int32_t h = hash_cell(ix, iy, iz, mask);
         cell_hash[i] = h;
-        if (cell_xyz) {  // [3][n], for the count pass
-            cell_xyz[i] = ix;
-            cell_xyz[n + i] = iy;
-            cell_xyz[2 * (size_t)n + i] = iz;
-        }
         atomicAdd(&bucket_count[h], 1);
     }
 }
@@ -145,80 +148,28 @@ __device__ __forceinline__ bool contact_rn(double d2, double s) {
 }
 
 // Visits every candidate j > i of droplet i (the distinct buckets of its 27
-// neighbour cells) and calls f(j, multiplicity) for those in contact.
-// PACKED: the droplets' (x, y), (z, r) in bucket order are in P (two double2
-// per bucket slot, slot ti holding droplet i), so a bucket's candidates are
-// read as contiguous 32-byte records instead of four scattered gathers, and
-// their FP32 roundings in P32 reject the clearly separated candidates first.
-// That test only drops a candidate whose FP32 distance exceeds the contact
-// distance by far more than FP32 rounding can account for (a margin of
-// 2^-17 (max |x_i| + L) plus 2^-18 of the radii sum; the per-axis distance is
-// bounded below by the smaller of |d| and ||d| - L|, which covers either image
-// the FP64 test may take); NaNs and overflowed bounds fail the comparison and
-// go to the FP64 test, and a margin below 2^-100 turns the far test off.  So
-// every pair the FP64 test accepts is still found.
-template <bool PACKED, typename F>
-__device__ __forceinline__ void for_each_contact(int i, int ti, const double *__restrict__ x,
-                                                 const double *__restrict__ y, const double *__restrict__ z,
-                                                 const double *__restrict__ r, const double2 *__restrict__ P,
-                                                 const float4 *__restrict__ P32,
+// neighbour cells) and calls f(j) for those in contact (the allocation-free
+// detector).
+template <typename F>
+__device__ __forceinline__ void for_each_contact(int i, const double *__restrict__ x, const double *__restrict__ y,
+                                                 const double *__restrict__ z, const double *__restrict__ r,
                                                  const HashParams &p, int periodic, double L, double halfL,
                                                  int32_t mask, int n, const int32_t *__restrict__ bstart,
                                                  const int32_t *__restrict__ sorted_idx, F &&f) {
-    double xi, yi, zi, ri;
-    if (PACKED) {
-        const double2 a = P[2 * ti], b = P[2 * ti + 1];
-        xi = a.x;
-        yi = a.y;
-        zi = b.x;
-        ri = b.y;
-    } else {
-        xi = x[i];
-        yi = y[i];
-        zi = z[i];
-        ri = r[i];
-    }
+    const double xi = x[i], yi = y[i], zi = z[i], ri = r[i];
     const int32_t cx = cell_coord(xi, p.cell, p.grid, periodic);
     const int32_t cy = cell_coord(yi, p.cell, p.grid, periodic);
     const int32_t cz = cell_coord(zi, p.cell, p.grid, periodic);
-    float4 qi = make_float4(0.f, 0.f, 0.f, 0.f);
-    float Lf = 0.f, marg = 0.f;
-    if (PACKED) {
-        qi = P32[ti];
-        Lf = (float)L;
-        marg = (float)(0x1p-17 * (fmax(fabs(xi), fmax(fabs(yi), fabs(zi))) + fabs(L)));
-        qi.w = qi.w * (1.f + 0x1p-18f) + marg;  // r_i, widened: the far test adds r_j (1 + 2^-18)
-        if (!(marg >= 0x1p-100f)) qi.w = INFINITY;  // coordinates near FP32's subnormal range: no far test
-    }
-    auto bucket = [&](const double xj, const double yj, const double zj, const double rj, int32_t j, int m) {
-        double dx = xj - xi, dy = yj - yi, dz = zj - zi;
+    auto candidate = [&](int32_t s, int m) {
+        const int32_t j = sorted_idx[s];
+        if (!(i < j)) return;
+        double dx = x[j] - xi, dy = y[j] - yi, dz = z[j] - zi;
         if (periodic) {
             dx = mic64(dx, L, halfL);
             dy = mic64(dy, L, halfL);
             dz = mic64(dz, L, halfL);
         }
-        if (contact_rn(dx * dx + dy * dy + dz * dz, ri + rj)) f(j, m);  // dist <= r_i + r_j
-    };
-    // PACKED: the slot's index and FP32 record are loaded together (one round of loads per candidate)
-    auto candidate = [&](int32_t s, int m) {
-        const int32_t j = sorted_idx[s];
-        if (PACKED) {
-            const float4 q = P32[s];
-            if (!(i < j)) return;
-            float ax = fabsf(q.x - qi.x), ay = fabsf(q.y - qi.y), az = fabsf(q.z - qi.z);
-            if (periodic) {
-                ax = fminf(ax, fabsf(ax - Lf));
-                ay = fminf(ay, fabsf(ay - Lf));
-                az = fminf(az, fabsf(az - Lf));
-            }
-            const float sf = fmaf(q.w, 1.f + 0x1p-18f, qi.w);
-            if (fmaf(ax, ax, fmaf(ay, ay, az * az)) > sf * sf) return;  // clearly apart
-            const double2 a = P[2 * s], b = P[2 * s + 1];
-            bucket(a.x, a.y, b.x, b.y, j, m);
-        } else {
-            if (!(i < j)) return;
-            bucket(x[j], y[j], z[j], r[j], j, m);
-        }
+        if (contact_rn(dx * dx + dy * dy + dz * dz, ri + r[j])) f(j, m);  // dist <= r_i + r_j
     };
     // Neighbour cell c = 9 (di + 1) + 3 (dj + 1) + (dk + 1): its bucket, or -1 outside an open box.
     auto cell_hash = [&](int c) -> int32_t {
@@ -243,42 +194,13 @@ __device__ __forceinline__ void for_each_contact(int i, int ti, const double *__
 #pragma unroll
             for (int m = 0; m < c; ++m) dup |= h[c] >= 0 && h[c] == h[m];
         if (!dup) {
-            if (PACKED) {
-                // the next cell's bucket range is loaded while this cell's candidates are tested, and
-                // candidates are taken two at a time: the loop is bound by load latency, not arithmetic
-                int32_t start = 0, end = 0;
-                if (h[0] >= 0) {
-                    start = bstart[h[0]];
-                    end = bstart[h[0] + 1];
-                }
-#pragma unroll 1
-                for (int c = 0; c < 27; ++c) {
-                    int32_t ns = 0, ne = 0;
-                    const int32_t hn = c + 1 < 27 ? cell_hash(c + 1) : -1;
-                    if (hn >= 0) {
-                        ns = bstart[hn];
-                        ne = bstart[hn + 1];
-                    }
-                    if (end > n) end = n;  // :199-201
-                    int32_t s = start;
-#pragma unroll 1
-                    for (; s + 1 < end; s += 2) {
-                        candidate(s, 1);
-                        candidate(s + 1, 1);
-                    }
-                    if (s < end) candidate(s, 1);
-                    start = ns;
-                    end = ne;
-                }
-            } else {
-                for (int c = 0; c < 27; ++c) {
-                    const int32_t hc = cell_hash(c);
-                    if (hc < 0) continue;
-                    const int32_t start = bstart[hc];
-                    int32_t end = bstart[hc + 1];
-                    if (end > n) end = n;  // :199-201
-                    for (int32_t s = start; s < end; ++s) candidate(s, 1);
-                }
+            for (int c = 0; c < 27; ++c) {
+                const int32_t hc = cell_hash(c);
+                if (hc < 0) continue;
+                const int32_t start = bstart[hc];
+                int32_t end = bstart[hc + 1];
+                if (end > n) end = n;  // :199-201
+                for (int32_t s = start; s < end; ++s) candidate(s, 1);
             }
             return;
         }
@@ -318,25 +240,8 @@ __device__ __forceinline__ void for_each_contact(int i, int ti, const double *__
     }
 }
 
-// The droplets' positions and radii in bucket order: P[2 s] = (x, y), P[2 s + 1] = (z, r) of sorted_idx[s].
-__global__ void bucket_positions_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
-                                        const double *__restrict__ z, const double *__restrict__ r,
-                                        const HashParams *__restrict__ hp, const int32_t *__restrict__ sorted_idx,
-                                        double2 *__restrict__ P, float4 *__restrict__ P32) {
-    if (!hp->valid) return;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const int j = sorted_idx[s];
-        const double xj = x[j], yj = y[j], zj = z[j], rj = r[j];
-        P[2 * s] = make_double2(xj, yj);
-        P[2 * s + 1] = make_double2(zj, rj);
-        P32[s] = make_float4((float)xj, (float)yj, (float)zj, (float)rj);
-    }
-}
-
-template <bool PACKED>
 __global__ void count_pairs_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
                                    const double *__restrict__ z, const double *__restrict__ r,
-                                   const double2 *__restrict__ P, const float4 *__restrict__ P32,
                                    const HashParams *__restrict__ hp, int periodic,
                                    double L, int32_t mask, const int32_t *__restrict__ bstart,
                                    const int32_t *__restrict__ sorted_idx, int32_t *__restrict__ pair_count,
@@ -347,224 +252,19 @@ __global__ void count_pairs_kernel(int n, const double *__restrict__ x, const do
         const int i = p.valid ? sorted_idx[t] : t;  // bucket order (the buckets are filled when valid)
         int32_t c = 0;
         if (p.valid) {
-            for_each_contact<PACKED>(i, t, x, y, z, r, P, P32, p, periodic, L, 0.5 * L, mask, n, bstart,
-                                     sorted_idx, [&](int32_t, int m) {
-                                         ++c;
-                                         local_raw += (unsigned long long)m;
-                                     });
+            for_each_contact(i, x, y, z, r, p, periodic, L, 0.5 * L, mask, n, bstart, sorted_idx,
+                             [&](int32_t, int m) {
+                                 ++c;
+                                 local_raw += (unsigned long long)m;
+                             });
         }
         pair_count[i] = c;
     }
     if (local_raw) atomicAdd(raw, local_raw);
 }
 
-// Count pass of the context entry point: one warp per occupied bucket.  The
-// droplets of a bucket share their 27 neighbour buckets when they lie in one
-// cell (the usual case), so the warp loads the 27 bucket ranges once, lays
-// their candidates out as one list and tests 32 candidates at a time, each lane
-// against every droplet of the bucket (staged in shared memory): the lanes stay
-// converged and each candidate is read once per bucket, not once per droplet.
-// A bucket holding droplets of several cells (hash aliasing) is taken one cell
-// at a time.  The tests are for_each_contact's (the FP32 far test, then the same
-// FP64 contact test); a cell with a neighbour bucket seen from two of its
-// neighbour cells, and a bucket of more than 32 droplets, take for_each_contact
-// per droplet.  Counts per droplet do not depend on the order.
-constexpr int CB_WARPS = 4;
-constexpr int CB_LIST = 256;  // candidate slots staged per warp (more: found by search)
-#ifndef CB_MIN_CTAS
-#define CB_MIN_CTAS 8  // resident CTAs per SM the count pass is compiled for (latency-bound: more warps)
-#endif
-
-__global__ void __launch_bounds__(32 * CB_WARPS, CB_MIN_CTAS)
-    count_pairs_bucket_kernel(int n, int table, const double *__restrict__ x, const double *__restrict__ y,
-                              const double *__restrict__ z, const double *__restrict__ r,
-                              const double2 *__restrict__ P, const float4 *__restrict__ P32,
-                              const HashParams *__restrict__ hp, int periodic, double L, int32_t mask,
-                              const int32_t *__restrict__ bstart, const int32_t *__restrict__ sorted_idx,
-                              const int32_t *__restrict__ cell_xyz, int32_t *__restrict__ pair_count,
-                              unsigned long long *__restrict__ raw) {
-    __shared__ float4 s_q[CB_WARPS][32];                       // FP32 record, radius widened (far test)
-    __shared__ double2 s_a[CB_WARPS][32], s_b[CB_WARPS][32];  // FP64 (x, y), (z, r)
-    __shared__ int s_i[CB_WARPS][32], s_cnt[CB_WARPS][32], s_st[CB_WARPS][32], s_pre[CB_WARPS][32];
-    __shared__ int s_list[CB_WARPS][CB_LIST];  // the cell's candidate slots (when they fit)
-    const HashParams p = *hp;
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    if (!p.valid) {
-        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) pair_count[t] = 0;
-        return;
-    }
-    const double halfL = 0.5 * L;
-    const float Lf = (float)L;
-    unsigned long long local_raw = 0;
-    const int warps_total = gridDim.x * CB_WARPS;
-    for (long long g = (long long)blockIdx.x * CB_WARPS + wp; g * 32 < table; g += warps_total) {
-        const long long bb = g * 32 + lane;
-        int t0 = 0, m = 0;
-        if (bb < table) {
-            t0 = bstart[bb];
-            m = bstart[bb + 1] - t0;
-        }
-        unsigned occ = __ballot_sync(0xffffffffu, m > 0);
-        while (occ) {
-            const int src = __ffs(occ) - 1;
-            occ &= occ - 1;
-            const int bt0 = __shfl_sync(0xffffffffu, t0, src), bm = __shfl_sync(0xffffffffu, m, src);
-            if (bm > 32) {  // a crowded bucket: per droplet
-                for (int k = lane; k < bm; k += 32) {
-                    const int t = bt0 + k;
-                    const int ii = sorted_idx[t];
-                    int32_t c = 0;
-                    for_each_contact<true>(ii, t, x, y, z, r, P, P32, p, periodic, L, halfL, mask, n, bstart,
-                                           sorted_idx, [&](int32_t, int mult) {
-                                               ++c;
-                                               local_raw += (unsigned long long)mult;
-                                           });
-                    pair_count[ii] = c;
-                }
-                continue;
-            }
-            // the bucket's droplets, one per lane, grouped by cell (a bucket can hold several cells)
-            int i = -1;
-            int32_t cx = 0, cy = 0, cz = 0;
-            double2 a = make_double2(0.0, 0.0), b = a;
-            if (lane < bm) {
-                const int t = bt0 + lane;
-                i = sorted_idx[t];
-                a = P[2 * t];
-                b = P[2 * t + 1];
-                cx = cell_xyz[i];  // cell_coord of the droplet (assign_kernel)
-                cy = cell_xyz[n + i];
-                cz = cell_xyz[2 * (size_t)n + i];
-            }
-            // lanes of the same cell (cell coordinates are >= 0; idle lanes get distinct negative x)
-            const unsigned same_cell = __match_any_sync(0xffffffffu, lane < bm ? cx : -1 - lane) &
-                                       __match_any_sync(0xffffffffu, cy) & __match_any_sync(0xffffffffu, cz);
-            unsigned todo = __ballot_sync(0xffffffffu, lane < bm);
-            while (todo) {
-                const int leader = __ffs(todo) - 1;
-                const unsigned grp = __shfl_sync(0xffffffffu, same_cell, leader);
-                todo &= ~grp;
-                const bool mine = (grp >> lane) & 1u;
-                const int32_t cx0 = __shfl_sync(0xffffffffu, cx, leader), cy0 = __shfl_sync(0xffffffffu, cy, leader),
-                              cz0 = __shfl_sync(0xffffffffu, cz, leader);
-                // neighbour cell c = lane: 9 (di + 1) + 3 (dj + 1) + (dk + 1), as in for_each_contact
-                int32_t h = -1;
-                if (lane < 27) {
-                    int32_t nx = cx0 + lane / 9 - 1, ny = cy0 + (lane / 3) % 3 - 1, nz = cz0 + lane % 3 - 1;
-                    if (periodic) {
-                        h = hash_cell(wrap1(nx, p.grid), wrap1(ny, p.grid), wrap1(nz, p.grid), mask);
-                    } else if (!(nx < 0 || ny < 0 || nz < 0 || nx >= p.grid || ny >= p.grid || nz >= p.grid)) {
-                        h = hash_cell(nx, ny, nz, mask);
-                    }
-                }
-                const unsigned peers = __match_any_sync(0xffffffffu, lane < 27 ? h : -2 - lane);
-                if (__any_sync(0xffffffffu, lane < 27 && h >= 0 && __popc(peers) > 1)) {
-                    // a neighbour bucket seen from two cells: per droplet, with multiplicities
-                    if (mine) {
-                        const int t = bt0 + lane;
-                        int32_t c = 0;
-                        for_each_contact<true>(i, t, x, y, z, r, P, P32, p, periodic, L, halfL, mask, n, bstart,
-                                               sorted_idx, [&](int32_t, int mult) {
-                                                   ++c;
-                                                   local_raw += (unsigned long long)mult;
-                                               });
-                        pair_count[i] = c;
-                    }
-                    continue;
-                }
-                int st = 0, len = 0;
-                if (h >= 0) {
-                    st = bstart[h];
-                    int e = bstart[h + 1];
-                    if (e > n) e = n;  // :199-201
-                    len = e > st ? e - st : 0;
-                }
-                int inc = len;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
-                }
-                const int total = __shfl_sync(0xffffffffu, inc, 31);
-                const int gm = __popc(grp);
-                s_st[wp][lane] = st;
-                s_pre[wp][lane] = inc - len;
-                const bool listed = total <= CB_LIST;
-                if (listed)
-                    for (int e = 0; e < len; ++e) s_list[wp][inc - len + e] = st + e;
-                if (mine) {  // the group's droplets at slots 0 .. gm - 1
-                    const int slot = __popc(grp & ((1u << lane) - 1u));
-                    const float marg = (float)(0x1p-17 * (fmax(fabs(a.x), fmax(fabs(a.y), fabs(b.x))) + fabs(L)));
-                    float4 q = P32[bt0 + lane];
-                    q.w = q.w * (1.f + 0x1p-18f) + marg;  // as for_each_contact's qi
-                    if (!(marg >= 0x1p-100f)) q.w = INFINITY;
-                    s_q[wp][slot] = q;
-                    s_a[wp][slot] = a;
-                    s_b[wp][slot] = b;
-                    s_i[wp][slot] = i;
-                    s_cnt[wp][slot] = 0;
-                }
-                __syncwarp();
-                const int *wi = s_i[wp];
-                const float4 *wq = s_q[wp];
-                for (int t = lane; t - lane < total; t += 32) {  // every lane takes the same number of rounds
-                    if (t >= total) continue;
-                    int sl;
-                    if (listed) {
-                        sl = s_list[wp][t];
-                    } else {  // the neighbour bucket holding list entry t: the last c with s_pre[c] <= t
-                        int lo = 0, hi = 26;
-                        while (lo < hi) {
-                            const int mid = (lo + hi + 1) >> 1;
-                            if (s_pre[wp][mid] <= t)
-                                lo = mid;
-                            else
-                                hi = mid - 1;
-                        }
-                        sl = s_st[wp][lo] + (t - s_pre[wp][lo]);
-                    }
-                    const int32_t j = sorted_idx[sl];
-                    const float4 q = P32[sl];
-                    const float qw = q.w * (1.f + 0x1p-18f);
-#pragma unroll 4
-                    for (int k = 0; k < gm; ++k) {
-                        const float4 qi = wq[k];
-                        float ax = fabsf(q.x - qi.x), ay = fabsf(q.y - qi.y), az = fabsf(q.z - qi.z);
-                        if (periodic) {
-                            ax = fminf(ax, fabsf(ax - Lf));
-                            ay = fminf(ay, fabsf(ay - Lf));
-                            az = fminf(az, fabsf(az - Lf));
-                        }
-                        const float sf = qw + qi.w;
-                        // i < j, and not clearly apart: the exact test (rare)
-                        if (!(wi[k] < j) || fmaf(ax, ax, fmaf(ay, ay, az * az)) > sf * sf) continue;
-                        const double2 ca = P[2 * sl], cb = P[2 * sl + 1];
-                        const double2 ka = s_a[wp][k], kb = s_b[wp][k];
-                        double dx = ca.x - ka.x, dy = ca.y - ka.y, dz = cb.x - kb.x;
-                        if (periodic) {
-                            dx = mic64(dx, L, halfL);
-                            dy = mic64(dy, L, halfL);
-                            dz = mic64(dz, L, halfL);
-                        }
-                        if (contact_rn(dx * dx + dy * dy + dz * dz, kb.y + cb.y)) {  // dist <= r_i + r_j
-                            atomicAdd(&s_cnt[wp][k], 1);
-                            ++local_raw;
-                        }
-                    }
-                }
-                __syncwarp();
-                if (lane < gm) pair_count[s_i[wp][lane]] = s_cnt[wp][lane];
-                __syncwarp();  // shared memory is rewritten by the next group
-            }
-        }
-    }
-    if (local_raw) atomicAdd(raw, local_raw);
-}
-
-template <bool PACKED>
 __global__ void write_pairs_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
                                    const double *__restrict__ z, const double *__restrict__ r,
-                                   const double2 *__restrict__ P, const float4 *__restrict__ P32,
                                    const HashParams *__restrict__ hp, int periodic, double L, int32_t mask,
                                    const int32_t *__restrict__ bstart, const int32_t *__restrict__ sorted_idx,
                                    const int64_t *__restrict__ offset, int32_t *__restrict__ pairs, int64_t cap,
@@ -586,8 +286,7 @@ __global__ void write_pairs_kernel(int n, const double *__restrict__ x, const do
         // pairs[o0 .. o0 + len); once the run holds m entries the largest drops out, so a cut row
         // keeps its m smallest j and the buffer holds the lexicographically first cap pairs
         int64_t len = 0;
-        for_each_contact<PACKED>(i, t, x, y, z, r, P, P32, p, periodic, L, 0.5 * L, mask, n, bstart, sorted_idx,
-                                 [&](int32_t j, int) {
+        for_each_contact(i, x, y, z, r, p, periodic, L, 0.5 * L, mask, n, bstart, sorted_idx, [&](int32_t j, int) {
             int64_t q;
             if (len < m) {
                 pairs[2 * (o0 + len)] = i;
@@ -602,6 +301,457 @@ __global__ void write_pairs_kernel(int n, const double *__restrict__ x, const do
             }
             pairs[2 * (o0 + q) + 1] = j;
         });
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The search of the context entry point
+// ---------------------------------------------------------------------------
+struct SearchParams {
+    HashParams hash;   // the reference's cells
+    double inv_h;      // search cells per unit length
+    int32_t m;         // search cells per axis of a periodic box; 0: open
+    float r_max;       // rounded up
+};
+
+// Words of the workspace that a detection zeroes: these, the bucket counts, the row counts.
+struct SearchMisc {
+    unsigned long long max_bits;  // maximum radius (ordered bits)
+    float r_sum;                  // of the positive radii
+    unsigned int done;            // CTAs of radius_kernel that have finished
+    unsigned int next_slot;       // slots given out to buckets
+    unsigned int found;           // pairs in the list
+    unsigned int pad[2];
+};
+static_assert(sizeof(SearchMisc) == 4 * SEARCH_MISC_WORDS, "ctx.cu sizes the workspace by this");
+
+// Search cells: 4.5 mean radii, so that a mean droplet's reach (2 r) covers (4 / 4.5 + 1)^3 ~ 6.7 cells, that
+// a cell holds ~0.4 droplets at 2 % volume fraction and ~6 at 30 %; not below half the largest radius (whose
+// droplet then searches at most 10^3 cells) nor above 4.5 of it.  Periodic boxes: whole cells, at most
+// 1,024 per axis (cell_id tells the cells of one search apart).
+__global__ void radius_kernel(int n, const double *__restrict__ r, double L, int periodic, int even_cells,
+                              SearchMisc *__restrict__ misc, SearchParams *__restrict__ out) {
+    __shared__ bool last;
+    unsigned long long m = 0ull;  // below every ordered value
+    float sum = 0.f;
+#pragma unroll 4
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double v = r[i];
+        const unsigned long long o = ordered_bits(v);
+        m = o > m ? o : m;
+        sum += v > 0.0 ? (float)v : 0.f;
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, off);
+        m = t > m ? t : m;
+        sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&misc->max_bits, m);
+        atomicAdd(&misc->r_sum, sum);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&misc->done, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    __threadfence();
+    SearchParams p;
+    p.hash = hash_params(from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits), L, even_cells);
+    const double r_max = from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits);
+    const double mean = (double)*(volatile float *)&misc->r_sum / n;
+    double h = fmax(4.5 * mean, 0.5 * r_max);
+    h = h <= 4.5 * r_max ? h : 4.5 * r_max;
+    p.r_max = __double2float_ru(r_max);
+    p.m = 0;
+    p.inv_h = 1.0 / h;
+    if (periodic) {
+        const double cells = floor(L / h);
+        p.m = cells >= 1024.0 ? 1024 : cells >= 1.0 ? (int32_t)cells : 1;
+        p.inv_h = p.m / L;
+    }
+    *out = p;
+}
+
+__device__ __forceinline__ int32_t search_floor(double v) {  // floor, kept within +-2^30
+    return (int32_t)fmin(fmax(floor(v), -0x1p30), 0x1p30);
+}
+__device__ __forceinline__ int32_t search_coord(double v, const SearchParams &p) {
+    const int32_t c = search_floor(v * p.inv_h);
+    return p.m ? floor_mod(c, p.m) : c;
+}
+__device__ __forceinline__ uint32_t search_bucket(int32_t cx, int32_t cy, int32_t cz, uint32_t mask) {
+    uint32_t h = (uint32_t)cx * 0x9E3779B1u ^ (uint32_t)cy * 0x85EBCA77u ^ (uint32_t)cz * 0xC2B2AE3Du;
+    h ^= h >> 15;
+    return (h * 0x2C1B3C6Du >> 7) & mask;
+}
+// Tells the cells of one droplet's search apart: their coordinates differ by less than 512 per axis (open
+// boxes: at most 10) or are the distinct residues below 1,024 of a periodic box.
+__device__ __forceinline__ int32_t cell_id(int32_t cx, int32_t cy, int32_t cz) {
+    return (int32_t)((uint32_t)cx + ((uint32_t)cy << 10) + ((uint32_t)cz << 20));
+}
+
+__global__ void search_assign_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
+                                     const double *__restrict__ z, const SearchParams *__restrict__ sp, uint32_t mask,
+                                     int32_t *__restrict__ count, int4 *__restrict__ key) {
+    const SearchParams p = *sp;
+    if (!p.hash.valid) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int32_t cx = search_coord(x[i], p), cy = search_coord(y[i], p), cz = search_coord(z[i], p);
+        const uint32_t b = search_bucket(cx, cy, cz, mask);
+        key[i] = make_int4((int)b, atomicAdd(&count[b], 1), cell_id(cx, cy, cz), 0);
+    }
+}
+
+// bucket[b] = (first slot, droplets): the CTA scans its buckets and takes its slots with one atomic, so
+// buckets of different CTAs follow one another in any order.
+constexpr int SB_T = 256, SB_ITEMS = 8;
+__global__ void __launch_bounds__(SB_T) search_starts_kernel(uint32_t buckets, const int32_t *__restrict__ count,
+                                                             SearchMisc *__restrict__ misc,
+                                                             const SearchParams *__restrict__ sp,
+                                                             int2 *__restrict__ bucket) {
+    if (!sp->hash.valid) return;
+    __shared__ int wsum[SB_T / 32], base;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t first = (blockIdx.x * SB_T + threadIdx.x) * SB_ITEMS;
+    int c[SB_ITEMS], own = 0;
+#pragma unroll
+    for (int k = 0; k < SB_ITEMS; ++k) {
+        c[k] = first + k < buckets ? count[first + k] : 0;
+        own += c[k];
+    }
+    int inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+        for (int k = 0; k < SB_T / 32; ++k) {
+            const int v = wsum[k];
+            wsum[k] = total;
+            total += v;
+        }
+        base = (int)atomicAdd(&misc->next_slot, (unsigned int)total);
+    }
+    __syncthreads();
+    int at = base + wsum[w] + inc - own;
+#pragma unroll
+    for (int k = 0; k < SB_ITEMS; ++k) {
+        if (first + k < buckets) bucket[first + k] = make_int2(at, c[k]);
+        at += c[k];
+    }
+}
+
+__global__ void search_scatter_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
+                                      const double *__restrict__ z, const double *__restrict__ r,
+                                      const SearchParams *__restrict__ sp, const int4 *__restrict__ key,
+                                      const int2 *__restrict__ bucket, float4 *__restrict__ rec) {
+    if (!sp->hash.valid) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int4 k = key[i];
+        const size_t s = bucket[k.x].x + k.y;
+        rec[2 * s] = make_float4((float)x[i], (float)y[i], (float)z[i], (float)r[i]);
+        rec[2 * s + 1] = make_float4(__int_as_float(i), __int_as_float(k.z), 0.f, 0.f);
+    }
+}
+
+struct SearchArgs {
+    int n;
+    const double *x, *y, *z, *r;
+    const SearchParams *sp;
+    int periodic;
+    double L, halfL;
+    int32_t hash_mask;   // the reference's table
+    uint32_t mask;       // search buckets - 1
+    const int2 *bucket;
+    const float4 *rec;   // per slot: (x, y, z, r), (droplet, cell id, -, -)
+    SearchMisc *misc;
+    int32_t *row_count;
+    int2 *list, *tmp;
+    uint32_t list_cap;
+    unsigned long long *raw;
+};
+
+// How many of the 27 cells around droplet i's cell map to droplet j's bucket (:160-201): 0 when the
+// reference does not compare i with j > i.
+__device__ __noinline__ int reference_hits(const SearchArgs &a, const HashParams &p, int i, int j) {
+    const bool per = a.periodic;
+    const int32_t cx = cell_coord(a.x[i], p.cell, p.grid, per), cy = cell_coord(a.y[i], p.cell, p.grid, per),
+                  cz = cell_coord(a.z[i], p.cell, p.grid, per);
+    const int32_t hj = hash_cell(cell_coord(a.x[j], p.cell, p.grid, per), cell_coord(a.y[j], p.cell, p.grid, per),
+                                 cell_coord(a.z[j], p.cell, p.grid, per), a.hash_mask);
+    int hits = 0;
+    for (int c = 0; c < 27; ++c) {
+        int32_t nx = cx + c / 9 - 1, ny = cy + (c / 3) % 3 - 1, nz = cz + c % 3 - 1;
+        if (per) {
+            nx = wrap1(nx, p.grid);
+            ny = wrap1(ny, p.grid);
+            nz = wrap1(nz, p.grid);
+        } else if (nx < 0 || ny < 0 || nz < 0 || nx >= p.grid || ny >= p.grid || nz >= p.grid) {
+            continue;
+        }
+        hits += hash_cell(nx, ny, nz, a.hash_mask) == hj;
+    }
+    return hits;
+}
+
+// The reference's contact test of two droplets (:203-219).
+__device__ __forceinline__ bool in_contact(const SearchArgs &a, int i, int j) {
+    double dx = a.x[j] - a.x[i], dy = a.y[j] - a.y[i], dz = a.z[j] - a.z[i];
+    if (a.periodic) {
+        dx = mic64(dx, a.L, a.halfL);
+        dy = mic64(dy, a.L, a.halfL);
+        dz = mic64(dz, a.L, a.halfL);
+    }
+    return contact_rn(dx * dx + dy * dy + dz * dz, a.r[i] + a.r[j]);  // dist <= r_i + r_j
+}
+
+// FP32 record q of a droplet, its radius widened for far_apart: by 2^-17 (max |x_i| + L) plus 2^-18 of the radii
+// sum, far more than FP32 rounding of either record can account for.  A margin below 2^-100 turns the far
+// test off.
+__device__ __forceinline__ float4 widened(float4 q, double L) {
+    const float marg = 0x1p-17f * (fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))) + fabsf((float)L));
+    q.w = marg >= 0x1p-100f ? q.w * (1.f + 0x1p-18f) + marg : INFINITY;
+    return q;
+}
+// Clearly not in contact (c: the candidate's record).  The per-axis distance is bounded below by the smaller of
+// |d| and ||d| - L|, which covers either image the FP64 test may take; NaNs and overflowed bounds fail the
+// comparison and go to the FP64 test, so every pair that test accepts is still found.
+__device__ __forceinline__ bool far_apart(const float4 &q, const float4 &c, bool periodic, float Lf) {
+    float ax = fabsf(c.x - q.x), ay = fabsf(c.y - q.y), az = fabsf(c.z - q.z);
+    if (periodic) {
+        ax = fminf(ax, fabsf(ax - Lf));
+        ay = fminf(ay, fabsf(ay - Lf));
+        az = fminf(az, fabsf(az - Lf));
+    }
+    const float s = fmaf(c.w, 1.f + 0x1p-18f, q.w);
+    return fmaf(ax, ax, fmaf(ay, ay, az * az)) > s * s;
+}
+
+// The search cells within `reach` of a coordinate, per axis: first cell and how many (periodic: wrapped, each
+// cell once).  `slack` covers the rounding of v and of the cell coordinates.
+struct Span {
+    int32_t first, len;
+};
+__device__ __forceinline__ Span span_of(double v, double reach, double slack, const SearchParams &p) {
+    const double wide = reach * (1.0 + 0x1p-18) + slack;
+    const int32_t lo = search_floor((v - wide) * p.inv_h), hi = search_floor((v + wide) * p.inv_h);
+    const long long len = (long long)hi - lo + 1;
+    if (!p.m) return {lo, (int32_t)len};  // len <= ~20: cells are at least half the largest radius
+    return len >= p.m ? Span{0, p.m} : Span{floor_mod(lo, p.m), (int32_t)len};
+}
+// From an FP32 coordinate (rounded by 2^-24 of itself), unless that is coarse against the cells or the cells
+// are near FP32's subnormal range.
+__device__ __forceinline__ Span span_of32(float v, const double *__restrict__ exact, int i, double reach, double L,
+                                          const SearchParams &p) {
+    const double slack = 0x1p-20 * (fabs((double)v) + (p.m ? fabs(L) : 0.0));
+    if (slack * p.inv_h < 0.125 && p.inv_h < 0x1p100) return span_of((double)v, reach, slack, p);
+    const double e = exact[i];
+    return span_of(e, reach, 1e-14 * (fabs(e) + (p.m ? fabs(L) : 0.0)), p);
+}
+__device__ __forceinline__ int32_t span_cell(const Span &s, int k, const SearchParams &p) {
+    const int32_t c = s.first + k;
+    return p.m && c >= p.m ? c - p.m : c;
+}
+
+// `group` <= 32 droplets (bucket order) per warp.  Their search cells form one list, 32 of which the warp looks up
+// at a time, and the droplets found in them another, of which it tests 32 at a time: a droplet has 1 to 27 cells,
+// rarely thousands, and 0 to a few candidates in each, so loops per lane would mostly wait for the longest
+// lane's loads (436 us at N = 2^20; this form 139).
+constexpr int SP_WARPS = 4;
+__global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __grid_constant__ SearchArgs a, int group) {
+    __shared__ float4 s_q[SP_WARPS][32];                // widened record
+    __shared__ float s_r[SP_WARPS][32];                 // radius
+    __shared__ int s_i[SP_WARPS][32];                   // droplet
+    __shared__ Span s_span[SP_WARPS][3][32];
+    __shared__ int s_first[SP_WARPS][32];               // the droplet's first entry in the list of cells
+    __shared__ int2 s_queue[SP_WARPS][64];              // candidates: slot, (cell id)
+    __shared__ unsigned char s_owner[SP_WARPS][64];     // and whose
+    const SearchParams p = *a.sp;
+    if (!p.hash.valid) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = (blockIdx.x * SP_WARPS + w) * group + lane;
+    const float Lf = (float)a.L;
+    unsigned long long raw = 0;
+    int cells = 0;
+    if (lane < group && t < a.n) {
+        const float4 q = a.rec[2 * (size_t)t];
+        const int i = __float_as_int(a.rec[2 * (size_t)t + 1].x);
+        s_q[w][lane] = widened(q, a.L);
+        s_r[w][lane] = q.w;
+        s_i[w][lane] = i;
+        // The partner's radius is at most this droplet's (by the FP32 order), so 2 r covers the contact
+        // distance; where FP32 radii are not normal numbers their order says nothing and r_max bounds it.
+        const double reach = q.w > 0x1p-100f && q.w < 0x1p100f ? 2.0 * q.w : a.r[i] + p.r_max;
+        if (reach >= 0.0) {  // (a pair of negative radii never touches)
+            const Span sx = span_of32(q.x, a.x, i, reach, a.L, p), sy = span_of32(q.y, a.y, i, reach, a.L, p),
+                       sz = span_of32(q.z, a.z, i, reach, a.L, p);
+            s_span[w][0][lane] = sx;
+            s_span[w][1][lane] = sy;
+            s_span[w][2][lane] = sz;
+            cells = sx.len * sy.len * sz.len;
+        }
+    }
+    int end = cells;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    s_first[w][lane] = end - cells;
+    __syncwarp();
+
+    // Entry e of the list of cells: its owner, its cell's id and bucket.
+    auto look_up = [&](int e, int &owner, int &id) -> int2 {
+        if (e >= total) return make_int2(0, 0);
+        int lo = 0;
+#pragma unroll
+        for (int step = 16; step; step >>= 1)  // the last lane whose first entry is <= e (an empty lane shares the next one's)
+            if (lo + step < 32 && s_first[w][lo + step] <= e) lo += step;
+        owner = lo;
+        const Span sx = s_span[w][0][lo], sy = s_span[w][1][lo], sz = s_span[w][2][lo];
+        const int k = e - s_first[w][lo], kxy = k / sz.len;
+        const int32_t cz = span_cell(sz, k - kxy * sz.len, p), kx = kxy / sy.len;
+        const int32_t cy = span_cell(sy, kxy - kx * sy.len, p), cx = span_cell(sx, kx, p);
+        id = cell_id(cx, cy, cz);
+        return a.bucket[search_bucket(cx, cy, cz, a.mask)];
+    };
+    // The first `k` <= 32 queued candidates: the smaller droplets (ties: the smaller index) of their cells.
+    auto test = [&](int k) {
+        if (lane < k) {
+            const int2 c = s_queue[w][lane];
+            const int o = s_owner[w][lane];
+            const float4 q = a.rec[2 * (size_t)c.x], r = a.rec[2 * (size_t)c.x + 1];
+            const int i = s_i[w][o], j = __float_as_int(r.x);
+            const bool smaller = q.w < s_r[w][o] || (q.w == s_r[w][o] && j < i);
+            if (smaller && __float_as_int(r.y) == c.y && !far_apart(s_q[w][o], q, a.periodic, Lf) &&
+                in_contact(a, i, j)) {
+                const int hits = reference_hits(a, p.hash, min(i, j), max(i, j));
+                if (hits) {
+                    raw += hits;
+                    atomicAdd(&a.row_count[min(i, j)], 1);
+                    const unsigned at = atomicAdd(&a.misc->found, 1u);
+                    if (at < a.list_cap) a.list[at] = make_int2(min(i, j), max(i, j));
+                }
+            }
+        }
+        __syncwarp();
+    };
+    int queued = 0;
+    int owner = 0, id = 0;
+    int2 b = look_up(lane, owner, id);
+    for (int e = lane; e - lane < total; e += 32) {
+        int next_owner = 0, next_id = 0;
+        const int2 next = look_up(e + 32, next_owner, next_id);  // in flight while this round's are queued
+        for (int k = 0; __any_sync(0xffffffffu, k < b.y); ++k) {
+            const unsigned live = __ballot_sync(0xffffffffu, k < b.y);
+            if (k < b.y) {
+                const int at = queued + __popc(live & ((1u << lane) - 1u));
+                s_queue[w][at] = make_int2(b.x + k, id);
+                s_owner[w][at] = (unsigned char)owner;
+            }
+            queued += __popc(live);
+            __syncwarp();
+            if (queued >= 32) {
+                test(32);
+                queued -= 32;
+                const int2 c = s_queue[w][32 + lane];
+                const unsigned char o = s_owner[w][32 + lane];
+                __syncwarp();
+                s_queue[w][lane] = c;
+                s_owner[w][lane] = o;
+                __syncwarp();
+            }
+        }
+        b = next;
+        owner = next_owner;
+        id = next_id;
+    }
+    test(queued);
+    if (raw) atomicAdd(a.raw, raw);
+}
+
+// The listed pairs into their rows (any order within a row).
+__global__ void place_pairs_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset) {
+    if (!a.sp->hash.valid || a.misc->found > a.list_cap) return;
+    const unsigned k = a.misc->found;
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
+        const int2 e = a.list[q];
+        a.tmp[offset[e.x] + atomicSub(&a.row_count[e.x], 1) - 1] = e;
+    }
+}
+
+// The rows sorted by j: a pair goes to its rank in its row; entries at or past `cap` are dropped, so the
+// buffer holds the lexicographically first cap pairs.  More pairs than the list holds: every droplet i
+// searches its reach r_i + r_max for its row and inserts each j > i into the row's sorted run, the largest
+// dropping out of a row that the capacity cuts.
+__global__ void write_rows_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset, int32_t *__restrict__ pairs,
+                                  int64_t cap, int64_t *__restrict__ counts, uint32_t *err) {
+    const SearchParams p = *a.sp;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    if (tid == 0) {
+        counts[0] = p.hash.valid ? offset[a.n] : 0;
+        if (p.hash.valid && offset[a.n] > cap) raise_device_error(err, DEM_DEVERR_PAIR_OVERFLOW);
+    }
+    if (!p.hash.valid) return;
+    if (a.misc->found <= a.list_cap) {
+        for (int64_t q = tid; q < (int64_t)a.misc->found; q += threads) {
+            const int2 e = a.tmp[q];
+            const int64_t o0 = offset[e.x], o1 = offset[e.x + 1];
+            int64_t to = o0;
+            for (int64_t w = o0; w < o1; ++w) to += a.tmp[w].y < e.y;
+            if (to < cap) {
+                pairs[2 * to] = e.x;
+                pairs[2 * to + 1] = e.y;
+            }
+        }
+        return;
+    }
+    const float Lf = (float)a.L;
+    for (int t = tid; t < a.n; t += threads) {
+        const float4 q = a.rec[2 * (size_t)t];
+        const int i = __float_as_int(a.rec[2 * (size_t)t + 1].x);
+        const int64_t o0 = offset[i], o1 = offset[i + 1];
+        const int64_t m = (o1 < cap ? o1 : cap) - o0;
+        const double reach = a.r[i] + p.r_max;
+        if (m <= 0 || !(reach >= 0.0)) continue;
+        const float4 qw = widened(q, a.L);
+        const Span sx = span_of32(q.x, a.x, i, reach, a.L, p), sy = span_of32(q.y, a.y, i, reach, a.L, p),
+                   sz = span_of32(q.z, a.z, i, reach, a.L, p);
+        int64_t len = 0;
+        for (int c = 0; c < sx.len * sy.len * sz.len; ++c) {
+            const int cxy = c / sz.len;
+            const int32_t cx = span_cell(sx, cxy / sy.len, p), cy = span_cell(sy, cxy % sy.len, p),
+                          cz = span_cell(sz, c % sz.len, p);
+            const int2 b = a.bucket[search_bucket(cx, cy, cz, a.mask)];
+            const int32_t id = cell_id(cx, cy, cz);
+            for (int s = b.x; s < b.x + b.y; ++s) {
+                const float4 r = a.rec[2 * (size_t)s + 1];
+                const int j = __float_as_int(r.x);
+                if (j <= i || __float_as_int(r.y) != id || far_apart(qw, a.rec[2 * (size_t)s], a.periodic, Lf) ||
+                    !in_contact(a, i, j) || !reference_hits(a, p.hash, i, j))
+                    continue;
+                int64_t at;
+                if (len < m) {
+                    pairs[2 * (o0 + len)] = i;
+                    at = len++;
+                } else {
+                    if (j >= pairs[2 * (o0 + m - 1) + 1]) continue;
+                    at = m - 1;
+                }
+                while (at > 0 && pairs[2 * (o0 + at - 1) + 1] > j) {
+                    pairs[2 * (o0 + at) + 1] = pairs[2 * (o0 + at - 1) + 1];
+                    --at;
+                }
+                pairs[2 * (o0 + at) + 1] = j;
+            }
+        }
     }
 }
 
@@ -621,46 +771,59 @@ __global__ void pair_bin_kernel(const int32_t *__restrict__ pairs, const int64_t
 int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, const double *r,
                        double L, int periodic, int table_size, int32_t *pairs, int64_t cap, int64_t *counts,
                        cudaStream_t s, int even_cells) {
-    int rc = dem_ensure_table(ctx, table_size);
+    if (table_size > (int64_t)SCAN_MAX_BLOCKS * SCAN_TILE)
+        return dem_set_error(ctx, DEM_E_CAPACITY, "scan: too many elements");
+    int rc = dem_check_cuda(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(int64_t), s), "memset");
+    if (rc || n == 0) return rc;
+    const uint32_t buckets = search_buckets(n);
+    // zeroed together: misc, row counts, bucket counts
+    SearchMisc *misc = reinterpret_cast<SearchMisc *>(ctx->search_zero);
+    int32_t *row_count = ctx->search_zero + SEARCH_MISC_WORDS, *bucket_count = row_count + n;
+    SearchParams *sp = reinterpret_cast<SearchParams *>(ctx->dscratch + 2);
+    static_assert(sizeof(SearchParams) <= 6 * sizeof(double), "dscratch[2..7]");
+    rc = dem_check_cuda(ctx, cudaMemsetAsync(misc, 0, sizeof(int32_t) * (SEARCH_MISC_WORDS + (size_t)n + buckets), s),
+                        "memset");
     if (rc) return rc;
-    unsigned long long *slot = reinterpret_cast<unsigned long long *>(ctx->dscratch) + 2;
-    HashParams *hp = reinterpret_cast<HashParams *>(ctx->dscratch + 4);
-    const int32_t mask = table_size - 1;
     const int grid = max(1, min(ceil_div(n, 256), 8 * ctx->sm_count));
-    rc = dem_check_cuda(ctx, cudaMemsetAsync(slot, 0, sizeof(unsigned long long), s), "memset");
-    if (!rc) rc = dem_check_cuda(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(int64_t), s), "memset");
-    if (!rc) rc = dem_check_cuda(ctx, cudaMemsetAsync(ctx->bucket_count, 0, sizeof(int32_t) * table_size, s), "memset");
-    if (rc) return rc;
-    if (n == 0) return DEM_OK;
     dem_prof_begin(ctx, "hash_detect", s);
-    max_kernel<<<grid, 256, 0, counted(s)>>>(n, r, slot);
-    hash_params_kernel<<<1, 1, 0, counted(s)>>>(slot, L, even_cells, hp);
-    assign_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, hp, periodic, mask, ctx->cell_hash, ctx->bucket_count,
-                                                ctx->cell_xyz);
-    rc = dem_check_launch(ctx, "hash assign");
+    radius_kernel<<<max(1, min(ceil_div(n, 1024), 4 * ctx->sm_count)), 256, 0, counted(s)>>>(n, r, L, periodic, even_cells,
+                                                                                         misc, sp);
+    search_assign_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, sp, buckets - 1, bucket_count, ctx->search_key);
+    search_starts_kernel<<<ceil_div(buckets, SB_T * SB_ITEMS), SB_T, 0, counted(s)>>>(buckets, bucket_count, misc, sp,
+                                                                                     ctx->search_bucket);
+    search_scatter_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, r, sp, ctx->search_key, ctx->search_bucket,
+                                                        ctx->search_rec);
+    if ((rc = dem_check_launch(ctx, "hash search grid"))) return rc;
+    SearchArgs a{};
+    a.n = n;
+    a.x = x;
+    a.y = y;
+    a.z = z;
+    a.r = r;
+    a.sp = sp;
+    a.periodic = periodic;
+    a.L = L;
+    a.halfL = 0.5 * L;
+    a.hash_mask = table_size - 1;
+    a.mask = buckets - 1;
+    a.bucket = ctx->search_bucket;
+    a.rec = ctx->search_rec;
+    a.misc = misc;
+    a.row_count = row_count;
+    a.list = ctx->search_list;
+    a.tmp = ctx->search_list + ctx->search_list_cap;
+    a.list_cap = ctx->search_list_cap;
+    a.raw = reinterpret_cast<unsigned long long *>(counts + 1);
+    // few droplets: fewer per warp, so that ~8 warps per SM share the search (N = 2,000: 14.7 -> 7.6 us with 4)
+    int group = 32;
+    while (group > 4 && ceil_div(n, group) < 8 * ctx->sm_count) group >>= 1;
+    search_pairs_kernel<<<ceil_div(n, group * SP_WARPS), 32 * SP_WARPS, 0, counted(s)>>>(a, group);
+    if ((rc = dem_check_launch(ctx, "hash search"))) return rc;
+    rc = exclusive_scan<int32_t, int64_t>(ctx, row_count, ctx->pair_offset, n, s);
     if (rc) return rc;
-    rc = exclusive_scan<int32_t, int32_t>(ctx, ctx->bucket_count, ctx->bucket_start, table_size, s);
-    if (rc) return rc;
-    rc = dem_check_cuda(ctx, cudaMemcpyAsync(ctx->bucket_cursor, ctx->bucket_start, sizeof(int32_t) * table_size,
-                                             cudaMemcpyDeviceToDevice, s),
-                        "cursor copy");
-    if (rc) return rc;
-    scatter_kernel<<<grid, 256, 0, counted(s)>>>(n, ctx->cell_hash, hp, ctx->bucket_cursor, ctx->sorted_idx);
-    bucket_positions_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, r, hp, ctx->sorted_idx, ctx->hash_pos,
-                                                          ctx->hash_pos32);
-    const int dgrid = ceil_div(n, 128);
-    const int cgrid = max(1, min(ceil_div(table_size, 32 * CB_WARPS), 32 * ctx->sm_count));
-    count_pairs_bucket_kernel<<<cgrid, 32 * CB_WARPS, 0, counted(s)>>>(
-        n, table_size, x, y, z, r, ctx->hash_pos, ctx->hash_pos32, hp, periodic, L, mask, ctx->bucket_start,
-        ctx->sorted_idx, ctx->cell_xyz, ctx->pair_count, reinterpret_cast<unsigned long long *>(counts + 1));
-    rc = dem_check_launch(ctx, "hash count");
-    if (rc) return rc;
-    rc = exclusive_scan<int32_t, int64_t>(ctx, ctx->pair_count, ctx->pair_offset, n, s);
-    if (rc) return rc;
-    write_pairs_kernel<true><<<dgrid, 128, 0, counted(s)>>>(n, x, y, z, r, ctx->hash_pos, ctx->hash_pos32, hp,
-                                                            periodic, L, mask,
-                                                            ctx->bucket_start, ctx->sorted_idx, ctx->pair_offset,
-                                                            pairs, cap, counts, ctx->d_err);
+    const int pgrid = max(1, min(ceil_div(n, 256), 2 * ctx->sm_count));
+    place_pairs_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset);
+    write_rows_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset, pairs, cap, counts, ctx->d_err);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "hash write");
 }
@@ -765,8 +928,8 @@ extern "C" int dem_hash_detect_noalloc(int n, const double *x, const double *y, 
     if (cudaMemsetAsync(bucket_count, 0, sizeof(int32_t) * table_size, s) != cudaSuccess) return DEM_E_CUDA;
     if (n == 0) return DEM_OK;
     max_kernel<<<grid, 256, 0, counted(s)>>>(n, r, slot);
-    hash_params_kernel<<<1, 1, 0, counted(s)>>>(slot, L, 0, hp);
-    assign_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, hp, periodic, mask, cell_hash, bucket_count, nullptr);
+    hash_params_kernel<<<1, 1, 0, counted(s)>>>(slot, L, hp);
+    assign_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, hp, periodic, mask, cell_hash, bucket_count);
     if (cudaGetLastError() != cudaSuccess) return DEM_E_CUDA;
     if (exclusive_scan_into<int32_t, int32_t>(bucket_count, bucket_start, table_size, static_cast<int32_t *>(sums),
                                               s) != cudaSuccess)
@@ -776,14 +939,14 @@ extern "C" int dem_hash_detect_noalloc(int n, const double *x, const double *y, 
         return DEM_E_CUDA;
     scatter_kernel<<<grid, 256, 0, counted(s)>>>(n, cell_hash, hp, bucket_cursor, sorted_idx);
     const int dgrid = ceil_div(n, 128);
-    count_pairs_kernel<false><<<dgrid, 128, 0, counted(s)>>>(n, x, y, z, r, nullptr, nullptr, hp, periodic, L, mask,
+    count_pairs_kernel<<<dgrid, 128, 0, counted(s)>>>(n, x, y, z, r, hp, periodic, L, mask,
                                                              bucket_start, sorted_idx, pair_count,
                                                              reinterpret_cast<unsigned long long *>(counts + 1));
     if (cudaGetLastError() != cudaSuccess) return DEM_E_CUDA;
     if (exclusive_scan_into<int32_t, int64_t>(pair_count, pair_offset, n, static_cast<int64_t *>(sums), s) !=
         cudaSuccess)
         return DEM_E_CUDA;
-    write_pairs_kernel<false><<<dgrid, 128, 0, counted(s)>>>(n, x, y, z, r, nullptr, nullptr, hp, periodic, L, mask,
+    write_pairs_kernel<<<dgrid, 128, 0, counted(s)>>>(n, x, y, z, r, hp, periodic, L, mask,
                                                              bucket_start, sorted_idx, pair_offset, pairs,
                                                              pair_capacity, counts, err);
     return cudaGetLastError() == cudaSuccess ? DEM_OK : DEM_E_CUDA;
