@@ -81,6 +81,19 @@ DEM_API unsigned long long dem_launch_count(void);
  * that the caller captured (a replay does not pass through the library). */
 DEM_API void dem_count_replayed_launches(unsigned long long k);
 
+/* The library calls between the two as a CUDA graph: dem_graph_begin puts
+ * `stream` (not the legacy default stream) into capture, dem_graph_end ends it
+ * and instantiates what was captured; dem_graph_launch replays it.  Nothing
+ * runs during the capture.  The calls must have run once before with the same
+ * sizes, so that no workspace has to grow; the graph keeps their pointers.
+ * dem_graph_end leaves capture mode even when it fails.  No reference
+ * counterpart. */
+typedef struct dem_graph dem_graph;
+DEM_API int dem_graph_begin(dem_ctx *ctx, void *stream);
+DEM_API int dem_graph_end(dem_ctx *ctx, void *stream, dem_graph **out);
+DEM_API int dem_graph_launch(dem_ctx *ctx, dem_graph *graph, void *stream);
+DEM_API void dem_graph_destroy(dem_graph *graph);
+
 /* Opt-in kernel timing: while enabled, CUDA events are recorded on the launch
  * stream around the main kernels ("mixed_force_pass", "mixed_convection_pass",
  * "fp64_force_pass", "fp64_convection_pass", "hash_detect").
@@ -242,6 +255,14 @@ DEM_API int dem_batch_replay(dem_batch *batch, int steps, void *stream);
 DEM_API int dem_aos_to_soa(dem_ctx *ctx, int n, const double *aos, double *x, double *y, double *z, void *stream);
 DEM_API int dem_soa_to_aos(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, double *aos,
                            void *stream);
+
+/* A trajectory frame: (x, y, z) to (n, 3) rows in aos_dev on `stream`, then a
+ * copy of them to host memory aos_host (pinned) on `copy_stream`, which waits for
+ * the first.  The cudaEvent_t's `ready` and `done` are recorded after the rows
+ * and after the copy.  Replaces the synchronous copy of a saved frame,
+ * dem/solution/droplet_solution.py:63-92. */
+DEM_API int dem_frame_copy(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, double *aos_dev,
+                           double *aos_host, void *stream, void *copy_stream, void *ready, void *done);
 
 /* ---- direct O(N^2) passes --------------------------------------------- */
 /* Dipole force on every droplet.

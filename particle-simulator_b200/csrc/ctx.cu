@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <new>
 
 #include "common.cuh"
 #include "scan.cuh"
@@ -121,6 +122,45 @@ int dem_kernel_binary_version(int device, int *version) {
     }
     *version = a.binaryVersion;
     return DEM_OK;
+}
+
+struct dem_graph {
+    cudaGraphExec_t exec = nullptr;
+};
+
+int dem_graph_begin(dem_ctx *ctx, void *stream) {
+    if (!ctx) return DEM_E_INVALID;
+    return dem_check_cuda(ctx, cudaStreamBeginCapture((cudaStream_t)stream, cudaStreamCaptureModeThreadLocal),
+                          "begin capture");
+}
+
+int dem_graph_end(dem_ctx *ctx, void *stream, dem_graph **out) {
+    if (!ctx || !out) return DEM_E_INVALID;
+    *out = nullptr;
+    cudaGraph_t g = nullptr;
+    int rc = dem_check_cuda(ctx, cudaStreamEndCapture((cudaStream_t)stream, &g), "end capture");
+    cudaGraphExec_t exec = nullptr;
+    if (!rc) rc = dem_check_cuda(ctx, cudaGraphInstantiate(&exec, g, 0), "instantiate graph");
+    if (g) cudaGraphDestroy(g);
+    if (rc) {
+        cudaGetLastError();  // a failed capture leaves no error behind for the next call
+        return rc;
+    }
+    *out = new (std::nothrow) dem_graph{exec};
+    if (*out) return DEM_OK;
+    cudaGraphExecDestroy(exec);
+    return dem_set_error(ctx, DEM_E_CAPACITY, "out of host memory");
+}
+
+int dem_graph_launch(dem_ctx *ctx, dem_graph *graph, void *stream) {
+    if (!ctx || !graph) return DEM_E_INVALID;
+    return dem_check_cuda(ctx, cudaGraphLaunch(graph->exec, (cudaStream_t)stream), "graph launch");
+}
+
+void dem_graph_destroy(dem_graph *graph) {
+    if (!graph) return;
+    cudaGraphExecDestroy(graph->exec);
+    delete graph;
 }
 
 int dem_profile_enable(dem_ctx *ctx, int enable) {

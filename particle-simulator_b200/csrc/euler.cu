@@ -156,4 +156,18 @@ int dem_soa_to_aos(dem_ctx *ctx, int n, const double *x, const double *y, const 
     return dem_check_launch(ctx, "soa_to_aos");
 }
 
+int dem_frame_copy(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, double *aos_dev,
+                   double *aos_host, void *stream, void *copy_stream, void *ready, void *done) {
+    if (!ctx || !ready || !done || n < 0) return DEM_E_INVALID;
+    if (n > 0 && !aos_host) return dem_set_error(ctx, DEM_E_INVALID, "null pointer");
+    int rc = n > 0 ? dem_soa_to_aos(ctx, n, x, y, z, aos_dev, stream) : DEM_OK;
+    if (!rc) rc = dem_check_cuda(ctx, cudaEventRecord((cudaEvent_t)ready, (cudaStream_t)stream), "frame copy");
+    if (!rc) rc = dem_check_cuda(ctx, cudaStreamWaitEvent((cudaStream_t)copy_stream, (cudaEvent_t)ready, 0), "frame copy");
+    if (!rc && n > 0)
+        rc = dem_check_cuda(ctx, cudaMemcpyAsync(aos_host, aos_dev, 3 * sizeof(double) * (size_t)n,
+                                                 cudaMemcpyDeviceToHost, (cudaStream_t)copy_stream), "frame copy");
+    if (!rc) rc = dem_check_cuda(ctx, cudaEventRecord((cudaEvent_t)done, (cudaStream_t)copy_stream), "frame copy");
+    return rc;
+}
+
 }  // extern "C"

@@ -30,14 +30,22 @@ class Stager:
         self.torch = ctx.torch
 
     # -- inputs ---------------------------------------------------------------
+    def _rows(self, t):
+        """A CUDA tensor as contiguous float64 (n, 3) rows (itself when it is)."""
+        f64 = self.torch.float64
+        if t.dtype is f64 and t.dim() == 2 and t.shape[1] == 3 and t.is_contiguous():
+            return t
+        return t.to(dtype=f64).reshape(-1, 3).contiguous()
+
     def positions(self, positions, radii, tag="in") -> tuple[DeviceState, bool]:
         """Returns the device state and whether the inputs were CUDA tensors."""
         torch = self.torch
         if N.is_cuda_tensor(positions):
-            pos = positions.to(dtype=torch.float64).reshape(-1, 3).contiguous()
+            pos = self._rows(positions)
             n = pos.shape[0]
             r = radii if N.is_cuda_tensor(radii) else torch.as_tensor(np.asarray(radii), device=pos.device)
-            r = r.to(dtype=torch.float64).reshape(-1).contiguous()
+            if not (r.dtype is torch.float64 and r.dim() == 1 and r.is_contiguous()):
+                r = r.to(dtype=torch.float64).reshape(-1).contiguous()
             soa = self.buf.dev(tag + "_soa", (3, n))
             self.ctx.aos_to_soa(n, pos, soa)
             return DeviceState(n, soa, r, pos), True
@@ -60,9 +68,8 @@ class Stager:
 
     def vectors(self, arr, n, tag) -> tuple:
         """(N, 3) numpy or CUDA tensor -> SoA device tensor."""
-        torch = self.torch
         if N.is_cuda_tensor(arr):
-            a = arr.to(dtype=torch.float64).reshape(-1, 3).contiguous()
+            a = self._rows(arr)
         else:
             h = self.buf.host(tag + "_h", (n, 3))
             h.numpy()[...] = np.ascontiguousarray(arr, dtype=np.float64).reshape(-1, 3)

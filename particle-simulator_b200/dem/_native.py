@@ -9,6 +9,8 @@ the classes raise instead of computing elsewhere.
 from __future__ import annotations
 
 import ctypes as C
+import math
+import sys
 import threading
 from pathlib import Path
 
@@ -51,6 +53,11 @@ SIGNATURES = {
     "dem_ctx_reserve": (_i, [_vp, _i]),
     "dem_ctx_capacity": (_i, [_vp]),
     "dem_last_error": (C.c_char_p, [_vp]),
+    "dem_graph_begin": (_i, [_vp, _vp]),
+    "dem_graph_end": (_i, [_vp, _vp, C.POINTER(_vp)]),
+    "dem_graph_launch": (_i, [_vp, _vp, _vp]),
+    "dem_graph_destroy": (None, [_vp]),
+    "dem_frame_copy": (_i, [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "dem_device_errors": (_i, [_vp, C.POINTER(C.c_uint32), _vp]),
     "dem_profile_enable": (_i, [_vp, _i]),
     "dem_profile_read": (_i, [_vp, C.c_char_p, C.POINTER(_d), C.POINTER(_i)]),
@@ -181,6 +188,17 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def xyz(t) -> tuple:
+    """The three component pointers of an SoA vector: a (3, n) tensor (from its base and row stride:
+    no view per component) or a sequence of three tensors."""
+    if isinstance(t, (list, tuple)):
+        return t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr()
+    if t.shape[0] < 3:
+        raise IndexError("an SoA vector has three components")
+    p, step = t.data_ptr(), t.stride(0) * t.element_size()
+    return p, p + step, p + 2 * step
+
+
 class Context:
     """One ``dem_ctx`` (device workspace) bound to a CUDA device."""
 
@@ -190,6 +208,9 @@ class Context:
         if device is None:
             device = torch.cuda.current_device()
         self.device = torch.device("cuda", torch.device(device).index if not isinstance(device, int) else device)
+        # the handle without a Stream object per call (2.2 -> 0.1 us), where this torch offers it
+        self._raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda index: torch.cuda.current_stream(index).cuda_stream)
         self.handle = _vp()
         with torch.cuda.device(self.device):
             self._check(lib().dem_ctx_create(self.device.index, max(int(capacity), 1), C.byref(self.handle)), "create")
@@ -215,7 +236,8 @@ class Context:
         raise DemError(f"{what}: {msg} (code {rc})")
 
     def stream(self):
-        return self.torch.cuda.current_stream(self.device).cuda_stream
+        """The current stream of this context's device, as a raw handle."""
+        return self._raw_stream(self.device.index)
 
     @property
     def capacity(self) -> int:
@@ -284,75 +306,78 @@ class Context:
 
     # -- thin wrappers over the C ABI (torch CUDA tensors in, no allocation) --
     def aos_to_soa(self, n, aos, soa):
-        self._check(lib().dem_aos_to_soa(self.handle, n, ptr(aos), ptr(soa[0]), ptr(soa[1]), ptr(soa[2]), self.stream()),
+        self._check(lib().dem_aos_to_soa(self.handle, n, ptr(aos), *xyz(soa), self.stream()),
                     "aos_to_soa")
 
     def soa_to_aos(self, n, soa, aos):
-        self._check(lib().dem_soa_to_aos(self.handle, n, ptr(soa[0]), ptr(soa[1]), ptr(soa[2]), ptr(aos), self.stream()),
+        self._check(lib().dem_soa_to_aos(self.handle, n, *xyz(soa), ptr(aos), self.stream()),
                     "soa_to_aos")
+
+    def frame_copy(self, n, soa, aos_dev, aos_host, copy_stream, ready, done):
+        """SoA positions -> aos_dev on the current stream -> aos_host (pinned) on copy_stream; `ready` and
+        `done` (torch events that have been recorded before) are recorded after the two."""
+        self._check(lib().dem_frame_copy(self.handle, n, *xyz(soa), ptr(aos_dev), ptr(aos_host), self.stream(),
+                                         copy_stream.cuda_stream, ready.cuda_event, done.cuda_event), "frame_copy")
 
     def direct_forces(self, n, pos, r, m_const, L, periodic, precision, out):
         self._check(
-            lib().dem_direct_forces(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), float(m_const),
-                                    float(L), int(periodic), int(precision), ptr(out[0]), ptr(out[1]), ptr(out[2]),
+            lib().dem_direct_forces(self.handle, n, *xyz(pos), ptr(r), float(m_const),
+                                    float(L), int(periodic), int(precision), *xyz(out),
                                     self.stream()),
             "direct_forces",
         )
 
     def direct_convection(self, n, pos, r, F, eta_const, L, periodic, precision, out):
         self._check(
-            lib().dem_direct_convection(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), ptr(F[0]),
-                                        ptr(F[1]), ptr(F[2]), float(eta_const), float(L), int(periodic),
-                                        int(precision), ptr(out[0]), ptr(out[1]), ptr(out[2]), self.stream()),
+            lib().dem_direct_convection(self.handle, n, *xyz(pos), ptr(r), *xyz(F), float(eta_const), float(L),
+                                        int(periodic),
+                                        int(precision), *xyz(out), self.stream()),
             "direct_convection",
         )
 
     def direct_forces_and_convection(self, n, pos, r, m_const, eta_const, L, periodic, precision, F, V):
         self._check(
-            lib().dem_direct_forces_and_convection(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
+            lib().dem_direct_forces_and_convection(self.handle, n, *xyz(pos), ptr(r),
                                                    float(m_const), float(eta_const), float(L), int(periodic),
-                                                   int(precision), ptr(F[0]), ptr(F[1]), ptr(F[2]), ptr(V[0]),
-                                                   ptr(V[1]), ptr(V[2]), self.stream()),
+                                                   int(precision), *xyz(F), *xyz(V), self.stream()),
             "direct_forces_and_convection",
         )
 
     def direct_convection_corr(self, corr: "Correction", n, pos, r, F, eta_const, L, periodic, precision, out):
         self._check(
-            lib().dem_direct_convection_corr(self.handle, corr.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]),
-                                             ptr(r), ptr(F[0]), ptr(F[1]), ptr(F[2]), float(eta_const), float(L),
-                                             int(periodic), int(precision), ptr(out[0]), ptr(out[1]),
-                                             ptr(out[2]), self.stream()),
+            lib().dem_direct_convection_corr(self.handle, corr.handle, n, *xyz(pos),
+                                             ptr(r), *xyz(F), float(eta_const), float(L),
+                                             int(periodic), int(precision), *xyz(out), self.stream()),
             "direct_convection_corr",
         )
 
     def direct_vjp(self, n, pos, r, F, lam, m_const, eta_const, stokes, L, periodic, mu, g, gr):
         self._check(
-            lib().dem_direct_vjp(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), ptr(F[0]), ptr(F[1]),
-                                 ptr(F[2]), ptr(lam[0]), ptr(lam[1]), ptr(lam[2]), float(m_const), float(eta_const),
-                                 float(stokes), float(L), int(periodic), ptr(mu[0]), ptr(mu[1]), ptr(mu[2]),
-                                 ptr(g[0]), ptr(g[1]), ptr(g[2]), ptr(gr), self.stream()),
+            lib().dem_direct_vjp(self.handle, n, *xyz(pos), ptr(r), *xyz(F), *xyz(lam), float(m_const),
+                                 float(eta_const),
+                                 float(stokes), float(L), int(periodic), *xyz(mu),
+                                 *xyz(g), ptr(gr), self.stream()),
             "direct_vjp",
         )
 
     def euler_update(self, n, pos, r, F, V, stokes, dt, L, periodic, out):
         self._check(
-            lib().dem_euler_update(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), ptr(F[0]), ptr(F[1]),
-                                   ptr(F[2]), ptr(V[0]), ptr(V[1]), ptr(V[2]), float(stokes), float(dt), float(L),
-                                   int(periodic), ptr(out[0]), ptr(out[1]), ptr(out[2]), self.stream()),
+            lib().dem_euler_update(self.handle, n, *xyz(pos), ptr(r), *xyz(F), *xyz(V), float(stokes), float(dt),
+                                   float(L),
+                                   int(periodic), *xyz(out), self.stream()),
             "euler_update",
         )
 
     def euler_update_total(self, n, pos, V, dt, L, periodic, out):
         self._check(
-            lib().dem_euler_update_total(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(V[0]), ptr(V[1]),
-                                         ptr(V[2]), float(dt), float(L), int(periodic), ptr(out[0]), ptr(out[1]),
-                                         ptr(out[2]), self.stream()),
+            lib().dem_euler_update_total(self.handle, n, *xyz(pos), *xyz(V), float(dt), float(L), int(periodic),
+                                         *xyz(out), self.stream()),
             "euler_update_total",
         )
 
     def hash_detect(self, n, pos, r, L, periodic, table_size, pairs, capacity, counts):
         self._check(
-            lib().dem_hash_detect(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), float(L),
+            lib().dem_hash_detect(self.handle, n, *xyz(pos), ptr(r), float(L),
                                   int(periodic), int(table_size), ptr(pairs), int(capacity), ptr(counts),
                                   self.stream()),
             "hash_detect",
@@ -360,7 +385,7 @@ class Context:
 
     def overlap_pairs(self, n, pos, r, L, periodic, table_size, pairs, capacity, counts):
         self._check(
-            lib().dem_overlap_pairs(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), float(L),
+            lib().dem_overlap_pairs(self.handle, n, *xyz(pos), ptr(r), float(L),
                                     int(periodic), int(table_size), ptr(pairs), int(capacity), ptr(counts),
                                     self.stream()),
             "overlap_pairs",
@@ -371,7 +396,7 @@ class Context:
         self._check(
             lib().dem_generate_droplets(self.handle, int(n), int(seed) & 0xFFFFFFFFFFFFFFFF, float(lo), float(hi),
                                         float(rmin), float(rmax), float(minimum_distance), int(bool(periodic)),
-                                        int(max_rounds), ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
+                                        int(max_rounds), *xyz(pos), ptr(r),
                                         C.byref(rounds), self.stream()),
             "generate_droplets",
         )
@@ -383,8 +408,8 @@ class Context:
 
     def merge(self, n, pos, r, pairs, num_pairs, out_pos, out_r, n_out, merged=None):
         self._check(
-            lib().dem_merge(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), ptr(pairs), ptr(num_pairs),
-                            ptr(out_pos[0]), ptr(out_pos[1]), ptr(out_pos[2]), ptr(out_r), ptr(n_out), ptr(merged),
+            lib().dem_merge(self.handle, n, *xyz(pos), ptr(r), ptr(pairs), ptr(num_pairs),
+                            *xyz(out_pos), ptr(out_r), ptr(n_out), ptr(merged),
                             self.stream()),
             "merge",
         )
@@ -451,21 +476,21 @@ class Tree:
             self.handle = None
 
     def build(self, n, pos, r, L, periodic, mpl):
-        self.ctx._check(lib().dem_tree_build(self.handle, n, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r), float(L),
+        self.ctx._check(lib().dem_tree_build(self.handle, n, *xyz(pos), ptr(r), float(L),
                                              int(bool(periodic)), int(mpl), self.ctx.stream()), "tree_build")
 
     def forces(self, m_const, theta_sq, out):
-        self.ctx._check(lib().dem_tree_forces(self.handle, float(m_const), float(theta_sq), ptr(out[0]), ptr(out[1]),
-                                              ptr(out[2]), self.ctx.stream()), "tree_forces")
+        self.ctx._check(lib().dem_tree_forces(self.handle, float(m_const), float(theta_sq), *xyz(out),
+                                              self.ctx.stream()), "tree_forces")
 
     def propagate_forces(self, F=None):
-        a = (None, None, None) if F is None else (ptr(F[0]), ptr(F[1]), ptr(F[2]))
+        a = (None, None, None) if F is None else xyz(F)
         self.ctx._check(lib().dem_tree_propagate_forces(self.handle, *a, self.ctx.stream()), "tree_propagate")
 
     def velocity(self, F, eta_const, theta_sq, stokes_factor, out):
-        a = (None, None, None) if F is None else (ptr(F[0]), ptr(F[1]), ptr(F[2]))
+        a = (None, None, None) if F is None else xyz(F)
         self.ctx._check(lib().dem_tree_velocity(self.handle, *a, float(eta_const), float(theta_sq),
-                                                float(stokes_factor), ptr(out[0]), ptr(out[1]), ptr(out[2]),
+                                                float(stokes_factor), *xyz(out),
                                                 self.ctx.stream()), "tree_velocity")
 
     def collision_matrix(self, bins, nbins, out):
@@ -511,18 +536,18 @@ class MortonTree:
             self.handle = None
 
     def build(self, n, pos, r, L, periodic, leaf_size):
-        self.ctx._check(lib().dem_bh_build(self.handle, int(n), ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
+        self.ctx._check(lib().dem_bh_build(self.handle, int(n), *xyz(pos), ptr(r),
                                            float(L), int(bool(periodic)), int(leaf_size), self.ctx.stream()),
                         "bh_build")
 
     def forces(self, m_const, theta, out):
-        self.ctx._check(lib().dem_bh_forces(self.handle, float(m_const), float(theta), ptr(out[0]), ptr(out[1]),
-                                            ptr(out[2]), self.ctx.stream()), "bh_forces")
+        self.ctx._check(lib().dem_bh_forces(self.handle, float(m_const), float(theta), *xyz(out),
+                                            self.ctx.stream()), "bh_forces")
 
     def velocity(self, F, eta_const, theta, stokes_factor, out):
-        a = (None, None, None) if F is None else (ptr(F[0]), ptr(F[1]), ptr(F[2]))
+        a = (None, None, None) if F is None else xyz(F)
         self.ctx._check(lib().dem_bh_velocity(self.handle, *a, float(eta_const), float(theta), float(stokes_factor),
-                                              ptr(out[0]), ptr(out[1]), ptr(out[2]), self.ctx.stream()),
+                                              *xyz(out), self.ctx.stream()),
                         "bh_velocity")
 
     def set_window(self, window_level):
@@ -579,33 +604,33 @@ class Batch:
         return dict(i_per_thread=a.value, ctas=b.value)
 
     def forces(self, pos, r, m_const, out):
-        self.ctx._check(lib().dem_batch_forces(self.handle, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
-                                               float(m_const), ptr(out[0]), ptr(out[1]), ptr(out[2]),
+        self.ctx._check(lib().dem_batch_forces(self.handle, *xyz(pos), ptr(r),
+                                               float(m_const), *xyz(out),
                                                self.ctx.stream()), "batch_forces")
 
     def convection(self, pos, r, F, eta_const, out):
-        self.ctx._check(lib().dem_batch_convection(self.handle, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
-                                                   ptr(F[0]), ptr(F[1]), ptr(F[2]), float(eta_const), ptr(out[0]),
-                                                   ptr(out[1]), ptr(out[2]), self.ctx.stream()), "batch_convection")
+        self.ctx._check(lib().dem_batch_convection(self.handle, *xyz(pos), ptr(r),
+                                                   *xyz(F), float(eta_const), *xyz(out), self.ctx.stream()),
+                                                   "batch_convection")
 
     def step(self, pos, r, m_const, eta_const, stokes, dt, F, V):
-        self.ctx._check(lib().dem_batch_step(self.handle, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
-                                             float(m_const), float(eta_const), float(stokes), float(dt), ptr(F[0]),
-                                             ptr(F[1]), ptr(F[2]), ptr(V[0]), ptr(V[1]), ptr(V[2]),
+        self.ctx._check(lib().dem_batch_step(self.handle, *xyz(pos), ptr(r),
+                                             float(m_const), float(eta_const), float(stokes), float(dt), *xyz(F),
+                                             *xyz(V),
                                              self.ctx.stream()), "batch_step")
 
     def autotune(self, pos, r, m_const, eta_const, F, V, reps=3):
         best = _d()
-        self.ctx._check(lib().dem_batch_autotune(self.handle, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
-                                                 float(m_const), float(eta_const), ptr(F[0]), ptr(F[1]), ptr(F[2]),
-                                                 ptr(V[0]), ptr(V[1]), ptr(V[2]), int(reps), self.ctx.stream(),
+        self.ctx._check(lib().dem_batch_autotune(self.handle, *xyz(pos), ptr(r),
+                                                 float(m_const), float(eta_const), *xyz(F),
+                                                 *xyz(V), int(reps), self.ctx.stream(),
                                                  C.byref(best)), "batch_autotune")
         return float(best.value)
 
     def capture(self, pos, r, m_const, eta_const, stokes, dt, F, V):
-        self.ctx._check(lib().dem_batch_capture(self.handle, ptr(pos[0]), ptr(pos[1]), ptr(pos[2]), ptr(r),
+        self.ctx._check(lib().dem_batch_capture(self.handle, *xyz(pos), ptr(r),
                                                 float(m_const), float(eta_const), float(stokes), float(dt),
-                                                ptr(F[0]), ptr(F[1]), ptr(F[2]), ptr(V[0]), ptr(V[1]), ptr(V[2])),
+                                                *xyz(F), *xyz(V)),
                         "batch_capture")
 
     def replay(self, steps):
@@ -620,34 +645,62 @@ class Buffers:
 
         self.torch = torch
         self.device = device
-        self._dev = {}
-        self._host = {}
+        self._dev, self._host = {}, {}  # name -> flat buffer
+        self._dev_views, self._host_views = {}, {}  # name -> (shape, the view last handed out)
+
+    def _view(self, store, views, name, shape, dtype, make):
+        dtype = dtype or self.torch.float64
+        known = views.get(name)
+        if known is not None and known[0] == shape and known[1].dtype == dtype:
+            return known[1]
+        numel = math.prod(shape)
+        t = store.get(name)
+        if t is None or t.numel() < numel or t.dtype != dtype:
+            t = store[name] = make(max(numel, 1), dtype)
+        v = t[:numel].view(*shape)
+        views[name] = (shape, v)
+        return v
 
     def dev(self, name, shape, dtype=None):
-        torch = self.torch
-        dtype = dtype or torch.float64
-        numel = int(np.prod(shape))
-        t = self._dev.get(name)
-        if t is None or t.numel() < numel or t.dtype != dtype:
-            t = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
-            self._dev[name] = t
-        return t[:numel].view(*shape)
+        return self._view(self._dev, self._dev_views, name, shape, dtype,
+                          lambda n, d: self.torch.empty(n, dtype=d, device=self.device))
 
     def host(self, name, shape, dtype=None):
-        torch = self.torch
-        dtype = dtype or torch.float64
-        numel = int(np.prod(shape))
-        t = self._host.get(name)
-        if t is None or t.numel() < numel or t.dtype != dtype:
-            t = torch.empty(max(numel, 1), dtype=dtype, pin_memory=True)
-            self._host[name] = t
-        return t[:numel].view(*shape)
+        return self._view(self._host, self._host_views, name, shape, dtype,
+                          lambda n, d: self.torch.empty(n, dtype=d, pin_memory=True))
+
+
+class Graph:
+    """The library calls of one function as a CUDA graph, captured natively on a stream of its own
+    (nothing runs) and replayed on the current stream.  ``launches``: kernels in it."""
+
+    def __init__(self, ctx: Context, stream, body):
+        self.ctx = ctx
+        self.handle = _vp()
+        before = launch_count()
+        with ctx.torch.cuda.stream(stream):
+            ctx._check(lib().dem_graph_begin(ctx.handle, ctx.stream()), "graph capture")
+            try:
+                body()
+            finally:  # leaves capture mode whatever happened
+                rc = lib().dem_graph_end(ctx.handle, ctx.stream(), C.byref(self.handle))
+            ctx._check(rc, "graph capture")
+        self.launches = launch_count() - before
+
+    def replay(self):
+        self.ctx._check(lib().dem_graph_launch(self.ctx.handle, self.handle, self.ctx.stream()), "graph launch")
+        count_replayed_launches(self.launches)
+
+    def __del__(self):
+        h = getattr(self, "handle", None)
+        if h is not None and h.value and _lib is not None:
+            try:
+                _lib.dem_graph_destroy(h)
+            except Exception:  # pragma: no cover - interpreter shutdown
+                pass
+            self.handle = None
 
 
 def is_cuda_tensor(a) -> bool:
-    try:
-        import torch
-
-        return isinstance(a, torch.Tensor) and a.is_cuda
-    except Exception:  # pragma: no cover
-        return False
+    torch = sys.modules.get("torch")  # a tensor exists only once torch is loaded
+    return torch is not None and isinstance(a, torch.Tensor) and a.is_cuda

@@ -61,8 +61,8 @@ class DirectTrajectory:
 
     # -- device helpers (SoA (3, n) tensors) -------------------------------------
     def velocity_parts(self, ctx, n, pos, r, m, F, V):
-        ctx.direct_forces(n, pos, r, m, self.L, self.periodic, self.precision, F)
-        ctx.direct_convection(n, pos, r, F, self.eta_const, self.L, self.periodic, self.precision, V)
+        # one call: the convection pass reuses the force pass's droplet order (same bits as two calls)
+        ctx.direct_forces_and_convection(n, pos, r, m, self.eta_const, self.L, self.periodic, self.precision, F, V)
 
     def advance(self, ctx, n, pos, r, F, V, D):
         """pos += dt u and D += dt u (no wrap), u = F / (gamma r) + V."""

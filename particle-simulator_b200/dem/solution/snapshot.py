@@ -31,6 +31,11 @@ class SnapshotWriter:
         self.ready = [torch.cuda.Event() for _ in range(self.depth)]
         self.done = [torch.cuda.Event() for _ in range(self.depth)]
         self.copy_stream = torch.cuda.Stream(device=dev)
+        for s in range(self.depth):
+            self.ready[s].record(self.copy_stream)  # creates the events the native call records
+            self.done[s].record(self.copy_stream)
+            # the allocator must not hand a slot out while the copy stream may read it
+            self.dev[s].record_stream(self.copy_stream)
         self.pending = collections.deque()  # (slot, time, n, solution), oldest first
         self.next_slot = 0
         self.frames = 0
@@ -43,17 +48,16 @@ class SnapshotWriter:
             self._append_oldest()
         s = self.next_slot
         self.next_slot = (s + 1) % self.depth
-        compute = self.torch.cuda.current_stream(self.ctx.device)
-        if n > 0:
-            self.ctx.soa_to_aos(n, pos_soa, self.dev[s])
-        self.ready[s].record(compute)
-        with self.torch.cuda.stream(self.copy_stream):
-            self.copy_stream.wait_event(self.ready[s])
-            if n > 0:
-                self.host[s][:n].copy_(self.dev[s][:n], non_blocking=True)
-            self.done[s].record(self.copy_stream)
-        self.dev[s].record_stream(self.copy_stream)  # the allocator must not hand the slot out while it is read
+        self.ctx.frame_copy(n, pos_soa, self.dev[s], self.host[s], self.copy_stream, self.ready[s], self.done[s])
         self.pending.append((s, t, n, solution))
+
+    def __del__(self):
+        # the pinned slots may go back to the allocator only once the copies into them have ended
+        if getattr(self, "pending", None):
+            try:
+                self.copy_stream.synchronize()
+            except Exception:  # pragma: no cover - interpreter shutdown
+                pass
 
     def _append_oldest(self):
         s, t, n, sol = self.pending.popleft()

@@ -194,14 +194,37 @@ class EulerDropletSolver(Solver):
         writer = SnapshotWriter(ctx, n, self.snapshot_depth) if self.snapshot_depth > 0 else None
 
         from .. import _native as N
+        from ..collision_detector import SpatialHashCollisionDetector
+        from ..force_calculator import DirectDropletForceCalculator
 
         state = {"graphs": self.graphs and not tree}
-        graphs = {}  # (n, cur, rc, detect) -> (graph, kernels in it); a key is captured on its second use
+        graphs = {}  # (n, cur, rc, detect) -> replay function; a key is captured on its second use
         seen = set()
         speculative = det is not None and hasattr(det, "detect_launch") and hasattr(det, "_pairs")
         side = torch.cuda.Stream(device=dev)  # the speculative step's detection
         clean = [0]  # consecutive detections without pairs
         pairs_ptr = [det._pairs.data_ptr() if speculative else 0]
+
+        # This package's calculator and detector allocate nothing once they have run, so their calls are captured
+        # natively (~0.1 ms; torch's capture, which tracks allocations, takes ~0.9 ms of a short run's step).
+        native = type(fc) is DirectDropletForceCalculator and (det is None or type(det) is SpatialHashCollisionDetector)
+        capture_stream = torch.cuda.Stream(device=dev)
+
+        def capture(body):
+            """`body` as a graph: a function that replays it."""
+            if native:
+                return N.Graph(ctx, capture_stream, body).replay
+            g = torch.cuda.CUDAGraph()
+            before = N.launch_count()
+            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+                body()
+            kernels = N.launch_count() - before
+
+            def replay():
+                g.replay()
+                N.count_replayed_launches(kernels)
+
+            return replay
 
         def advance(n, cur, rc, detect=False):
             """[detection of pos_bufs[cur] +] forces + convection + Euler from pos_bufs[cur]
@@ -224,21 +247,15 @@ class EulerDropletSolver(Solver):
                 body()
                 return
             if key not in graphs:
-                g = torch.cuda.CUDAGraph()
-                c0 = N.launch_count()
                 try:
-                    with torch.cuda.graph(g, capture_error_mode="thread_local"):
-                        body()
+                    graphs[key] = capture(body)
                 except RuntimeError as e:  # a calculator whose calls cannot be captured: run eagerly
                     state["graphs"] = False
                     if self.verbose:
                         print(f"CUDA graph capture unavailable ({e}); stepping without graphs")
                     body()
                     return
-                graphs[key] = (g, N.launch_count() - c0)
-            g, k = graphs[key]
-            g.replay()
-            N.count_replayed_launches(k)
+            graphs[key]()
             self.graph_replays += 1
 
         def save(tt, nn):
