@@ -205,13 +205,21 @@ int dem_ctx_reserve(dem_ctx *ctx, int capacity) {
     const size_t n = (size_t)capacity;
     if ((rc = grow(ctx, &ctx->pack_a, n, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->pack_b, n, "workspace"))) return rc;
+    // the collision search's arrays in one allocation (an allocation costs more than its bytes)
     const size_t buckets = search_buckets((int64_t)n);
-    if ((rc = grow(ctx, &ctx->search_zero, SEARCH_MISC_WORDS + n + buckets, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->search_key, n, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->search_bucket, buckets, "workspace"))) return rc;
-    if ((rc = grow(ctx, &ctx->search_rec, 2 * n, "workspace"))) return rc;
-    ctx->search_list_cap = (uint32_t)std::min<size_t>(2 * n + 65536, 0x7fffffffu);
-    if ((rc = grow(ctx, &ctx->search_list, 2 * (size_t)ctx->search_list_cap, "workspace"))) return rc;
+    const uint32_t list_cap = (uint32_t)std::min<size_t>(2 * n + 65536, 0x7fffffffu);
+    auto part = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    const size_t zero_b = part(4 * (SEARCH_MISC_WORDS + n + buckets)), key_b = part(sizeof(int4) * n),
+                 bucket_b = part(sizeof(int2) * buckets), rec_b = part(sizeof(float4) * 2 * n),
+                 list_b = part(sizeof(int2) * 2 * (size_t)list_cap);
+    if ((rc = grow(ctx, &ctx->search_mem, zero_b + key_b + bucket_b + rec_b + list_b, "workspace"))) return rc;
+    char *at = ctx->search_mem;
+    ctx->search_zero = reinterpret_cast<int32_t *>(at);
+    ctx->search_key = reinterpret_cast<int4 *>(at += zero_b);
+    ctx->search_bucket = reinterpret_cast<int2 *>(at += key_b);
+    ctx->search_rec = reinterpret_cast<float4 *>(at += bucket_b);
+    ctx->search_list = reinterpret_cast<int2 *>(at += rec_b);
+    ctx->search_list_cap = list_cap;
     if ((rc = grow(ctx, &ctx->pair_offset, n + 1, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->flags, n + 1, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->keep_off, n + 1, "workspace"))) return rc;
@@ -259,7 +267,7 @@ void dem_ctx_destroy(dem_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     void *ptrs[] = {ctx->d_err,         ctx->pack_a,      ctx->pack_b,     ctx->partial,    ctx->dscratch,
-                    ctx->search_zero,   ctx->search_key,  ctx->search_bucket, ctx->search_rec, ctx->search_list,
+                    ctx->search_mem,
                     ctx->pair_offset,   ctx->flags,       ctx->keep_off,   ctx->merged_buf,
                     ctx->merged_cnt,    ctx->scan_tmp,    ctx->sym_partial};
     for (void *p : ptrs)

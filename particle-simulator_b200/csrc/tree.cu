@@ -22,6 +22,9 @@
 #include "corr.cuh"
 #include "scan.cuh"
 
+constexpr int WALK_T = 128;  // threads per CTA of the walks
+constexpr size_t WALK_REC_BYTES = 64, WALK_DIP_BYTES = 80;
+
 struct dem_tree {
     dem_ctx *ctx = nullptr;  // must outlive the tree while kernels run; destroy does not touch it
     int device = 0;
@@ -44,6 +47,12 @@ struct dem_tree {
     double *p = nullptr;                   // [4][N]: x, y, z, r
     double *pf = nullptr;                  // [3][N]: forces of the last force walk
     int32_t *part_node = nullptr, *part_oct = nullptr, *leaf_idx = nullptr;
+    // walk records (walk_records_kernel) and droplets in leaf-slot order
+    char *rec_f = nullptr, *rec_v = nullptr, *rec_d = nullptr;  // [M]
+    double2 *slot_p = nullptr, *slot_f = nullptr;               // [N][2]: (x, y), (z, r); (Fx, Fy), (Fz, -)
+    int32_t *roots = nullptr;              // [2]: where the force / velocity walk starts
+    bool built = false;                    // the last build completed
+    bool vel_records = false;              // rec_v / rec_d belong to this build
     int32_t *h_total = nullptr;            // pinned
     const dem_corr *corr = nullptr;        // periodic-image correction (borrowed), or none
 };
@@ -58,6 +67,9 @@ struct TreeDev {
     int32_t *first_child, *next, *leaf_start, *count, *child_cnt, *parents, *parent_fc, *flag, *rank, *fill;
     double *p, *pf;
     int32_t *part_node, *part_oct, *leaf_idx;
+    char *rec_f, *rec_v, *rec_d;
+    double2 *slot_p, *slot_f;
+    int32_t *roots;
     uint32_t *err;
 };
 
@@ -89,6 +101,12 @@ static TreeDev view(const dem_tree *t) {
     v.part_node = t->part_node;
     v.part_oct = t->part_oct;
     v.leaf_idx = t->leaf_idx;
+    v.rec_f = t->rec_f;
+    v.rec_v = t->rec_v;
+    v.rec_d = t->rec_d;
+    v.slot_p = t->slot_p;
+    v.slot_f = t->slot_f;
+    v.roots = t->roots;
     v.err = t->ctx->d_err;
     return v;
 }
@@ -383,97 +401,190 @@ __global__ void sweep_forces_kernel(TreeDev t, int a, int b) {
         for (int u = 0; u < 12; ++u) t.fs[u * M + parent] = acc[u];
     }
 }
+// ---------------------------------------------------------------------------
+// Walk records.  A walk visits a node through one 64-byte record: the size
+// squared and the centre (the same expressions the reference evaluates at every
+// visit, :466-520, evaluated once), what the accepted node needs, and two links
+// that leave out the nodes the walk passes over without a term (empty, R^3 sum
+// below 1e-30 :861, squared force sum below 1e-60 :1155; half the nodes of a tree
+// of one droplet per leaf): the first of its children that is not passed over
+// (or what follows them), and the next node when it is done.  Links: -1 the end;
+// child <= -2 marks a leaf whose first slot is -2 - child.
+// ---------------------------------------------------------------------------
+struct __align__(16) ForceRec {
+    double s2, cx, cy, cz, r3;
+    int32_t child, next, count, pad[3];
+};
+struct __align__(16) VelRec {
+    double s2, cx, cy, cz;
+    int32_t child, next;
+    double fx, fy, fz;
+};
+// Dipole D_ab = P_ab - c_a F_b about the centre (:1215-1230) and its trace.
+struct __align__(16) DipRec {
+    double d[9], tr;
+};
+static_assert(sizeof(ForceRec) == WALK_REC_BYTES && sizeof(VelRec) == WALK_REC_BYTES && sizeof(DipRec) == WALK_DIP_BYTES,
+              "the tree's allocation");
 
-// ---------------------------------------------------------------------------
-// walks
-// ---------------------------------------------------------------------------
+template <bool FORCE>
+__device__ __forceinline__ bool passed_over(const TreeDev &t, int k) {
+    if (t.count[k] == 0) return true;
+    if (FORCE) return t.R3[k] < 1e-30;
+    const size_t M = t.max_nodes;
+    const double fx = t.fs[k], fy = t.fs[M + k], fz = t.fs[2 * M + k];
+    return fx * fx + fy * fy + fz * fz < 1e-60;
+}
+
+// The first node from k on that has a term or is opened (a walk that met k, or any node it passes over).
+template <bool FORCE>
+__device__ __forceinline__ int first_kept(const TreeDev &t, int k) {
+    for (int steps = 0; k >= 0 && passed_over<FORCE>(t, k); k = t.next[k])
+        if (++steps > t.node_count) return -1;  // broken links: the walk's own bound reports them
+    return k;
+}
+
+template <bool FORCE>
+__global__ void walk_records_kernel(TreeDev t, int nc, int32_t *__restrict__ root) {
+    const int M = t.max_nodes;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *root = first_kept<FORCE>(t, 0);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nc; k += gridDim.x * blockDim.x) {
+        if (passed_over<FORCE>(t, k)) continue;  // no walk loads its record
+        const double s = node_size(t.mn, t.mx, M, k);
+        double cx, cy, cz;
+        node_center(t.mn, t.mx, t.R3, M, k, cx, cy, cz);
+        const int fc = t.first_child[k];
+        const int child = fc < 0 ? -2 - t.leaf_start[k] : first_kept<FORCE>(t, fc);
+        const int next = first_kept<FORCE>(t, t.next[k]);
+        if (FORCE) {
+            ForceRec *const o = reinterpret_cast<ForceRec *>(t.rec_f) + k;
+            *o = ForceRec{s * s, cx, cy, cz, t.R3[k], child, next, t.count[k], {0, 0, 0}};
+        } else {
+            const double Fx = t.fs[k], Fy = t.fs[M + k], Fz = t.fs[2 * (size_t)M + k];
+            reinterpret_cast<VelRec *>(t.rec_v)[k] = VelRec{s * s, cx, cy, cz, child, next, Fx, Fy, Fz};
+            const double *P = t.fs + 3 * (size_t)M;
+            DipRec d;
+            const double c[3] = {cx, cy, cz}, F[3] = {Fx, Fy, Fz};
+#pragma unroll
+            for (int q = 0; q < 9; ++q) d.d[q] = P[(size_t)q * M + k] - c[q / 3] * F[q % 3];
+            d.tr = d.d[0] + d.d[4] + d.d[8];
+            reinterpret_cast<DipRec *>(t.rec_d)[k] = d;
+        }
+    }
+}
+
+// Droplets (x, y, z, r) in leaf-slot order; with fx: their forces.
+__global__ void slot_droplets_kernel(TreeDev t, int n) {
+    const size_t N = t.cap;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const int j = t.leaf_idx[s];
+        t.slot_p[2 * (size_t)s] = make_double2(t.p[j], t.p[N + j]);
+        t.slot_p[2 * (size_t)s + 1] = make_double2(t.p[2 * N + j], t.p[3 * N + j]);
+    }
+}
+__global__ void slot_forces_kernel(TreeDev t, int n, const double *__restrict__ fx, const double *__restrict__ fy,
+                                   const double *__restrict__ fz) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const int j = t.leaf_idx[s];
+        t.slot_f[2 * (size_t)s] = make_double2(fx[j], fy[j]);
+        t.slot_f[2 * (size_t)s + 1] = make_double2(fz[j], 0.0);
+    }
+}
+
+// The walks.  One thread per target, in leaf-slot order (a permutation of all n particles: every particle
+// ends in a leaf), so the lanes of a warp walk neighbouring targets along nearly the same path; each
+// target's sums are its own thread's, in the reference's order, whatever order the targets are taken in.
+// A lane first goes on to its next term -- an accepted node or a pair of a leaf -- and the warp then
+// evaluates the lanes' terms together (a node's and a pair's force have the same form).
+//
+// Bound: latency (a visit's record, a chain of FP64 operations) and divergence (13 of 32 lanes active on
+// average): 21 warps per SM are all there is at N = 100,000.  N = 100,003, one droplet per leaf, open, force /
+// total-velocity walk: 2.00 / 3.54 ms with 11 to 23 scattered loads and a division per visit, half of the
+// visits on empty nodes; 1.24 / 2.13 ms now; 16 droplets per leaf, periodic: 11.5 / 15.0 -> 5.5 / 7.7.
+// (Loading the next node's record before a term is evaluated: 1.39 / 2.22, the loads wait all the same.)
+template <bool PER>
+__device__ __forceinline__ void image64x3(double &dx, double &dy, double &dz, double L, double halfL) {
+    if (PER) {
+        dx = mic64(dx, L, halfL);
+        dy = mic64(dy, L, halfL);
+        dz = mic64(dz, L, halfL);
+    }
+}
+
 // _compute_forces_kernel :783-894
 template <bool PER>
-__global__ void __launch_bounds__(128) force_walk_kernel(TreeDev t, double m_const, double theta_sq,
-                                                         double *__restrict__ fx, double *__restrict__ fy,
-                                                         double *__restrict__ fz) {
-    const int M = t.max_nodes, N = t.cap, n = t.n;
+__global__ void __launch_bounds__(WALK_T) force_walk_kernel(TreeDev t, double m_const, double theta_sq,
+                                                            double *__restrict__ fx, double *__restrict__ fy,
+                                                            double *__restrict__ fz) {
+    const int N = t.cap, n = t.n;
     const double L = t.L, halfL = 0.5 * t.L;
-    // targets in leaf-slot order (a permutation of all n particles: every particle ends in a leaf), so
-    // the lanes of a warp walk neighbouring targets along nearly the same path; each target's sums
-    // are its own thread's, in the reference's order, whatever order the targets are taken in
-    for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n; slot += gridDim.x * blockDim.x) {
-        const int i = t.leaf_idx[slot];
-        const double xi = t.p[i], yi = t.p[N + i], zi = t.p[2 * N + i], ri = t.p[3 * N + i];
-        const double ri3 = ipow3(ri);
-        double Fx = 0, Fy = 0, Fz = 0;
-        int node = 0;
-        int steps = 0;  // every node is visited at most once; more means broken links
-        while (node >= 0) {
-            if (++steps > t.node_count + 1) {
-                raise_device_error(t.err, DEM_DEVERR_NODE_OVERFLOW);
+    const ForceRec *__restrict__ rec = reinterpret_cast<const ForceRec *>(t.rec_f);
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n) return;
+    const int i = t.leaf_idx[slot];
+    const double2 pa = t.slot_p[2 * (size_t)slot], pb = t.slot_p[2 * (size_t)slot + 1];
+    const double xi = pa.x, yi = pa.y, zi = pb.x, ri = pb.y;
+    const double mri3 = m_const * ipow3(ri);
+    double Fx = 0, Fy = 0, Fz = 0;
+    int node = t.roots[0], k = 0, kend = 0;
+    int steps = 0;  // every node is visited at most once; more means broken links
+    while (true) {
+        double dx, dy, dz, d_sq, w;
+        bool term = false;
+        while (k < kend || node >= 0) {
+            if (k < kend) {
+                const int s = k++;
+                if (s == slot) continue;
+                const double2 qa = t.slot_p[2 * (size_t)s], qb = t.slot_p[2 * (size_t)s + 1];
+                dx = qa.x - xi, dy = qa.y - yi, dz = qb.x - zi;
+                image64x3<PER>(dx, dy, dz, L, halfL);
+                d_sq = dx * dx + dy * dy + dz * dz;
+                const double r_sum = ri + qb.y;
+                if (!(d_sq >= r_sum * r_sum)) continue;
+                w = ipow3(qb.y);
+                term = true;
                 break;
             }
-            const int cnt = t.count[node];
-            if (cnt == 0 || t.R3[node] < 1e-30) {
-                node = t.next[node];
+            if (++steps > t.node_count + 1) {
+                raise_device_error(t.err, DEM_DEVERR_NODE_OVERFLOW);
+                node = -1;
+                break;
+            }
+            const ForceRec &q = rec[node];
+            const int child = q.child;
+            if (child <= -2) {
+                k = -2 - child;
+                kend = k + q.count;
+                node = q.next;
                 continue;
             }
-            if (t.first_child[node] < 0) {
-                const int l0 = t.leaf_start[node];
-                for (int k = 0; k < cnt; ++k) {
-                    const int j = t.leaf_idx[l0 + k];
-                    if (j >= 0 && j != i) {
-                        double dx = t.p[j] - xi, dy = t.p[N + j] - yi, dz = t.p[2 * N + j] - zi;
-                        if (PER) {
-                            dx = mic64(dx, L, halfL);
-                            dy = mic64(dy, L, halfL);
-                            dz = mic64(dz, L, halfL);
-                        }
-                        const double r_sq = dx * dx + dy * dy + dz * dz;
-                        const double rj = t.p[3 * N + j];
-                        const double r_sum = ri + rj;
-                        if (r_sq >= r_sum * r_sum) {
-                            const double rr = sqrt(r_sq);
-                            const double r7 = r_sq * r_sq * r_sq * rr;
-                            const double factor = m_const * ri3 * ipow3(rj) / r7;
-                            const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
-                            const double ang = 4.0 * dz2 - dx2 - dy2;
-                            Fx += factor * dx * ang;
-                            Fy += factor * dy * ang;
-                            Fz += factor * dz * (2.0 * dz2 - 3.0 * dx2 - 3.0 * dy2);
-                        }
-                    }
-                }
-                node = t.next[node];
-                continue;
+            dx = q.cx - xi, dy = q.cy - yi, dz = q.cz - zi;
+            image64x3<PER>(dx, dy, dz, L, halfL);
+            d_sq = dx * dx + dy * dy + dz * dz;
+            if (q.s2 < theta_sq * d_sq && d_sq > 0.0) {
+                w = q.r3;
+                node = q.next;
+                term = true;
+                break;
             }
-            const double s = node_size(t.mn, t.mx, M, node);
-            double cx, cy, cz;
-            node_center(t.mn, t.mx, t.R3, M, node, cx, cy, cz);
-            double dx = cx - xi, dy = cy - yi, dz = cz - zi;
-            if (PER) {
-                dx = mic64(dx, L, halfL);
-                dy = mic64(dy, L, halfL);
-                dz = mic64(dz, L, halfL);
-            }
-            const double D_sq = dx * dx + dy * dy + dz * dz;
-            if (s * s < theta_sq * D_sq && D_sq > 0.0) {
-                const double rr = sqrt(D_sq);
-                const double r7 = D_sq * D_sq * D_sq * rr;
-                const double factor = m_const * ri3 * t.R3[node] / r7;
-                const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
-                const double ang = 4.0 * dz2 - dx2 - dy2;
-                Fx += factor * dx * ang;
-                Fy += factor * dy * ang;
-                Fz += factor * dz * (2.0 * dz2 - 3.0 * dx2 - 3.0 * dy2);
-                node = t.next[node];
-            } else {
-                node = t.first_child[node];
-            }
+            node = child;
         }
-        fx[i] = Fx;
-        fy[i] = Fy;
-        fz[i] = Fz;
-        t.pf[i] = Fx;
-        t.pf[N + i] = Fy;
-        t.pf[2 * N + i] = Fz;
+        if (!term) break;
+        const double rr = sqrt(d_sq);
+        const double r7 = d_sq * d_sq * d_sq * rr;
+        const double factor = mri3 * w / r7;
+        const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
+        const double ang = 4.0 * dz2 - dx2 - dy2;
+        Fx += factor * dx * ang;
+        Fy += factor * dy * ang;
+        Fz += factor * dz * (2.0 * dz2 - 3.0 * dx2 - 3.0 * dy2);
     }
+    fx[i] = Fx;
+    fy[i] = Fy;
+    fz[i] = Fz;
+    t.pf[i] = Fx;
+    t.pf[N + i] = Fy;
+    t.pf[2 * (size_t)N + i] = Fz;
 }
 
 // _compute_stokeslet_kernel :1000-1280 (stokes <= 0) and
@@ -481,126 +592,110 @@ __global__ void __launch_bounds__(128) force_walk_kernel(TreeDev t, double m_con
 // periodic-image correction after every leaf pair (:1070-1131) and accepted
 // node (:1171-1213), and the self term of the Stokeslet walk (:1271-1276).
 template <bool PER, bool CORR>
-__global__ void __launch_bounds__(128) velocity_walk_kernel(TreeDev t, const double *__restrict__ Fx_,
-                                                            const double *__restrict__ Fy_,
-                                                            const double *__restrict__ Fz_, double eta,
-                                                            double theta_sq, double stokes, CorrDev corr,
-                                                            double *__restrict__ vx, double *__restrict__ vy,
-                                                            double *__restrict__ vz) {
-    const int M = t.max_nodes, N = t.cap, n = t.n;
+__global__ void __launch_bounds__(WALK_T) velocity_walk_kernel(TreeDev t, const double *__restrict__ Fx_,
+                                                               const double *__restrict__ Fy_,
+                                                               const double *__restrict__ Fz_, double eta,
+                                                               double theta_sq, double stokes, CorrDev corr,
+                                                               double *__restrict__ vx, double *__restrict__ vy,
+                                                               double *__restrict__ vz) {
+    const int N = t.cap, n = t.n;
     const double L = t.L, halfL = 0.5 * t.L;
-    // targets in leaf-slot order, as in force_walk_kernel
-    for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n; slot += gridDim.x * blockDim.x) {
-        const int i = t.leaf_idx[slot];
-        const double xi = t.p[i], yi = t.p[N + i], zi = t.p[2 * N + i], ri = t.p[3 * N + i];
-        double ux = 0, uy = 0, uz = 0;
-        if (stokes > 0) {
-            const double inv_stokes_r = 1.0 / (stokes * ri);
-            ux = t.pf[i] * inv_stokes_r;
-            uy = t.pf[N + i] * inv_stokes_r;
-            uz = t.pf[2 * N + i] * inv_stokes_r;
-        }
-        int node = 0;
-        int steps = 0;
-        while (node >= 0) {
-            if (++steps > t.node_count + 1) {
-                raise_device_error(t.err, DEM_DEVERR_NODE_OVERFLOW);
+    const VelRec *__restrict__ rec = reinterpret_cast<const VelRec *>(t.rec_v);
+    const DipRec *__restrict__ dip = reinterpret_cast<const DipRec *>(t.rec_d);
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n) return;
+    const int i = t.leaf_idx[slot];
+    const double2 pa = t.slot_p[2 * (size_t)slot], pb = t.slot_p[2 * (size_t)slot + 1];
+    const double xi = pa.x, yi = pa.y, zi = pb.x, ri = pb.y;
+    double ux = 0, uy = 0, uz = 0;
+    if (stokes > 0) {
+        const double inv_stokes_r = 1.0 / (stokes * ri);
+        ux = t.pf[i] * inv_stokes_r;
+        uy = t.pf[N + i] * inv_stokes_r;
+        uz = t.pf[2 * (size_t)N + i] * inv_stokes_r;
+    }
+    int node = t.roots[1], k = 0, kend = 0;
+    int steps = 0;
+    while (true) {
+        double dx, dy, dz, d_sq, Fx, Fy, Fz;
+        int accepted = -1;
+        bool term = false;
+        while (k < kend || node >= 0) {
+            if (k < kend) {
+                const int s = k++;
+                if (s == slot) continue;
+                const double2 qa = t.slot_p[2 * (size_t)s], qb = t.slot_p[2 * (size_t)s + 1];
+                dx = xi - qa.x, dy = yi - qa.y, dz = zi - qb.x;
+                image64x3<PER>(dx, dy, dz, L, halfL);
+                d_sq = dx * dx + dy * dy + dz * dz;
+                const double r_sum = ri + qb.y;
+                if (!(d_sq >= r_sum * r_sum)) continue;
+                const double2 fa = t.slot_f[2 * (size_t)s];
+                Fx = fa.x, Fy = fa.y, Fz = t.slot_f[2 * (size_t)s + 1].x;
+                term = true;
                 break;
             }
-            const int cnt = t.count[node];
-            const double fsx = t.fs[node], fsy = t.fs[M + node], fsz = t.fs[2 * M + node];
-            const double fs2 = fsx * fsx + fsy * fsy + fsz * fsz;
-            if (cnt == 0 || fs2 < 1e-60) {
-                node = t.next[node];
+            if (++steps > t.node_count + 1) {
+                raise_device_error(t.err, DEM_DEVERR_NODE_OVERFLOW);
+                node = -1;
+                break;
+            }
+            const VelRec &q = rec[node];
+            const int child = q.child;
+            if (child <= -2) {
+                k = -2 - child;
+                kend = k + t.count[node];
+                node = q.next;
                 continue;
             }
-            if (t.first_child[node] < 0) {
-                const int l0 = t.leaf_start[node];
-                for (int k = 0; k < cnt; ++k) {
-                    const int j = t.leaf_idx[l0 + k];
-                    if (j >= 0 && j != i) {
-                        double dx = xi - t.p[j], dy = yi - t.p[N + j], dz = zi - t.p[2 * N + j];
-                        if (PER) {
-                            dx = mic64(dx, L, halfL);
-                            dy = mic64(dy, L, halfL);
-                            dz = mic64(dz, L, halfL);
-                        }
-                        const double r_sq = dx * dx + dy * dy + dz * dz;
-                        const double r_sum = ri + t.p[3 * N + j];
-                        if (r_sq >= r_sum * r_sum) {
-                            const double rr = sqrt(r_sq);
-                            const double inv_r = 1.0 / rr;
-                            const double inv_r2 = inv_r * inv_r;
-                            const double Fx = Fx_[j], Fy = Fy_[j], Fz = Fz_[j];
-                            const double dot = dx * Fx + dy * Fy + dz * Fz;
-                            const double coeff = eta * inv_r;
-                            ux += coeff * (Fx + dx * inv_r2 * dot);
-                            uy += coeff * (Fy + dy * inv_r2 * dot);
-                            uz += coeff * (Fz + dz * inv_r2 * dot);
-                            if (CORR) corr_pair64(corr, dx, dy, dz, Fx, Fy, Fz, ux, uy, uz);
-                        }
-                    }
-                }
-                node = t.next[node];
-                continue;
+            dx = xi - q.cx, dy = yi - q.cy, dz = zi - q.cz;
+            image64x3<PER>(dx, dy, dz, L, halfL);
+            d_sq = dx * dx + dy * dy + dz * dz;
+            if (q.s2 < theta_sq * d_sq && d_sq > 0.0) {
+                Fx = q.fx, Fy = q.fy, Fz = q.fz;
+                accepted = node;
+                node = q.next;
+                term = true;
+                break;
             }
-            const double s = node_size(t.mn, t.mx, M, node);
-            double cx, cy, cz;
-            node_center(t.mn, t.mx, t.R3, M, node, cx, cy, cz);
-            double dx = xi - cx, dy = yi - cy, dz = zi - cz;
-            if (PER) {
-                dx = mic64(dx, L, halfL);
-                dy = mic64(dy, L, halfL);
-                dz = mic64(dz, L, halfL);
-            }
-            const double D_sq = dx * dx + dy * dy + dz * dz;
-            if (s * s < theta_sq * D_sq && D_sq > 0.0) {
-                const double rr = sqrt(D_sq);
-                const double inv_r = 1.0 / rr;
-                const double inv_r2 = inv_r * inv_r;
-                const double Fx = fsx, Fy = fsy, Fz = fsz;
-                const double dot = dx * Fx + dy * Fy + dz * Fz;
-                const double coeff = eta * inv_r;
-                ux += coeff * (Fx + dx * inv_r2 * dot);
-                uy += coeff * (Fy + dy * inv_r2 * dot);
-                uz += coeff * (Fz + dz * inv_r2 * dot);
-                if (CORR) corr_pair64(corr, dx, dy, dz, Fx, Fy, Fz, ux, uy, uz);
-                // dipole correction :1215-1265, R^3-weighted centre (same as get_center)
-                const double cmx = cx, cmy = cy, cmz = cz;
-                const double *P = t.fs + 3 * (size_t)M;
-                const double Dxx = P[node] - cmx * Fx, Dxy = P[M + node] - cmx * Fy, Dxz = P[2 * M + node] - cmx * Fz;
-                const double Dyx = P[3 * M + node] - cmy * Fx, Dyy = P[4 * M + node] - cmy * Fy,
-                             Dyz = P[5 * M + node] - cmy * Fz;
-                const double Dzx = P[6 * M + node] - cmz * Fx, Dzy = P[7 * M + node] - cmz * Fy,
-                             Dzz = P[8 * M + node] - cmz * Fz;
-                const double rx = dx, ry = dy, rz = dz;
-                const double Ux = Dxx * rx + Dyx * ry + Dzx * rz;
-                const double Uy = Dxy * rx + Dyy * ry + Dzy * rz;
-                const double Uz = Dxz * rx + Dyz * ry + Dzz * rz;
-                const double wx = Dxx * rx + Dxy * ry + Dxz * rz;
-                const double wy = Dyx * rx + Dyy * ry + Dyz * rz;
-                const double wz = Dzx * rx + Dzy * ry + Dzz * rz;
-                const double s_tr = Dxx + Dyy + Dzz;
-                const double q = rx * wx + ry * wy + rz * wz;
-                const double inv_r3 = inv_r * inv_r2;
-                const double inv_r5 = inv_r3 * inv_r2;
-                ux += eta * (inv_r3 * (Ux - wx - s_tr * rx) + 3.0 * rx * q * inv_r5);
-                uy += eta * (inv_r3 * (Uy - wy - s_tr * ry) + 3.0 * ry * q * inv_r5);
-                uz += eta * (inv_r3 * (Uz - wz - s_tr * rz) + 3.0 * rz * q * inv_r5);
-                node = t.next[node];
-            } else {
-                node = t.first_child[node];
-            }
+            node = child;
         }
-        if (CORR && !(stokes > 0)) {  // self term, Stokeslet walk only
-            ux += corr.g_self * Fx_[i];
-            uy += corr.g_self * Fy_[i];
-            uz += corr.g_self * Fz_[i];
+        if (!term) break;
+        const double rr = sqrt(d_sq);
+        const double inv_r = 1.0 / rr;
+        const double inv_r2 = inv_r * inv_r;
+        const double dot = dx * Fx + dy * Fy + dz * Fz;
+        const double coeff = eta * inv_r;
+        ux += coeff * (Fx + dx * inv_r2 * dot);
+        uy += coeff * (Fy + dy * inv_r2 * dot);
+        uz += coeff * (Fz + dz * inv_r2 * dot);
+        if (CORR) corr_pair64(corr, dx, dy, dz, Fx, Fy, Fz, ux, uy, uz);
+        if (accepted >= 0) {  // dipole correction :1215-1265, R^3-weighted centre (same as get_center)
+            const DipRec D = dip[accepted];
+            const double rx = dx, ry = dy, rz = dz;
+            const double Ux = D.d[0] * rx + D.d[3] * ry + D.d[6] * rz;
+            const double Uy = D.d[1] * rx + D.d[4] * ry + D.d[7] * rz;
+            const double Uz = D.d[2] * rx + D.d[5] * ry + D.d[8] * rz;
+            const double wx = D.d[0] * rx + D.d[1] * ry + D.d[2] * rz;
+            const double wy = D.d[3] * rx + D.d[4] * ry + D.d[5] * rz;
+            const double wz = D.d[6] * rx + D.d[7] * ry + D.d[8] * rz;
+            const double s_tr = D.tr;
+            const double q = rx * wx + ry * wy + rz * wz;
+            const double inv_r3 = inv_r * inv_r2;
+            const double inv_r5 = inv_r3 * inv_r2;
+            ux += eta * (inv_r3 * (Ux - wx - s_tr * rx) + 3.0 * rx * q * inv_r5);
+            uy += eta * (inv_r3 * (Uy - wy - s_tr * ry) + 3.0 * ry * q * inv_r5);
+            uz += eta * (inv_r3 * (Uz - wz - s_tr * rz) + 3.0 * rz * q * inv_r5);
         }
-        vx[i] = ux;
-        vy[i] = uy;
-        vz[i] = uz;
     }
+    if (CORR && !(stokes > 0)) {  // self term, Stokeslet walk only
+        ux += corr.g_self * Fx_[i];
+        uy += corr.g_self * Fy_[i];
+        uz += corr.g_self * Fz_[i];
+    }
+    vx[i] = ux;
+    vy[i] = uy;
+    vz[i] = uz;
 }
 
 // TreeCollisionFrequency._count_collisions, pbm/collision_frequency/tree_collision_freq.py:62-135:
@@ -697,7 +792,8 @@ using namespace dem;
 static int tree_free(dem_tree *t) {
     void *ptrs[] = {t->mn,       t->mx,   t->R3,       t->maxr,      t->fs,   t->first_child, t->next,
                     t->leaf_start, t->count, t->child_cnt, t->parents, t->parent_fc, t->flag, t->rank,
-                    t->fill,     t->p,    t->pf,       t->part_node, t->part_oct, t->leaf_idx};
+                    t->fill,     t->p,    t->pf,       t->part_node, t->part_oct, t->leaf_idx,
+                    t->rec_f,    t->rec_v, t->rec_d,   t->slot_p,    t->slot_f,   t->roots};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (t->h_total) cudaFreeHost(t->h_total);
@@ -739,6 +835,12 @@ int dem_tree_create(dem_ctx *ctx, int capacity, int max_nodes, dem_tree **out) {
     ALLOC(part_node, int32_t, N);
     ALLOC(part_oct, int32_t, N);
     ALLOC(leaf_idx, int32_t, N);
+    ALLOC(rec_f, char, WALK_REC_BYTES * M);
+    ALLOC(rec_v, char, WALK_REC_BYTES * M);
+    ALLOC(rec_d, char, WALK_DIP_BYTES * M);
+    ALLOC(slot_p, double2, 2 * N);
+    ALLOC(slot_f, double2, 2 * N);
+    ALLOC(roots, int32_t, 2);
 #undef ALLOC
     if (e == cudaSuccess) e = cudaMallocHost((void **)&t->h_total, sizeof(int32_t) * 2);
     if (e != cudaSuccess) {
@@ -773,6 +875,7 @@ int dem_tree_build(dem_tree *t, int n, const double *x, const double *y, const d
     t->node_count = 1;
     t->parent_count = 0;
     t->pool_exhausted = 0;
+    t->built = t->vel_records = false;
     t->level_off.clear();
     dem_prof_begin(ctx, "tree_build", s);
     tree_init_kernel<<<grid_for(ctx, max(n, 1)), 256, 0, counted(s)>>>(view(t), n, L, x, y, z, r);
@@ -825,22 +928,33 @@ int dem_tree_build(dem_tree *t, int n, const double *x, const double *y, const d
     if (!rc) rc = dem_check_cuda(ctx, cudaStreamSynchronize(s), "tree build");
     if (rc) return rc;
     t->leaf_slot_count = t->h_total[1];
+    walk_records_kernel<true><<<grid_for(ctx, nc), 256, 0, counted(s)>>>(view(t), nc, t->roots);
+    slot_droplets_kernel<<<grid_for(ctx, max(n, 1)), 256, 0, counted(s)>>>(view(t), n);
     dem_prof_end(ctx, s);
-    return dem_check_launch(ctx, "tree build");
+    rc = dem_check_launch(ctx, "tree build");
+    t->built = rc == DEM_OK;
+    return rc;
 }
 
 int dem_tree_forces(dem_tree *t, double m_const, double theta_sq, double *fx, double *fy, double *fz, void *stream) {
     if (!t || !fx || !fy || !fz) return DEM_E_INVALID;
     if (t->n == 0) return DEM_OK;
+    if (!t->built) return dem_set_error(t->ctx, DEM_E_INVALID, "the tree's build did not complete");
     cudaStream_t s = (cudaStream_t)stream;
     dem_prof_begin(t->ctx, "tree_force_walk", s);
-    const int grid = ceil_div(t->n, 128);
+    const int grid = ceil_div(t->n, WALK_T);
     if (t->periodic)
-        force_walk_kernel<true><<<grid, 128, 0, counted(s)>>>(view(t), m_const, theta_sq, fx, fy, fz);
+        force_walk_kernel<true><<<grid, WALK_T, 0, counted(s)>>>(view(t), m_const, theta_sq, fx, fy, fz);
     else
-        force_walk_kernel<false><<<grid, 128, 0, counted(s)>>>(view(t), m_const, theta_sq, fx, fy, fz);
+        force_walk_kernel<false><<<grid, WALK_T, 0, counted(s)>>>(view(t), m_const, theta_sq, fx, fy, fz);
     dem_prof_end(t->ctx, s);
     return dem_check_launch(t->ctx, "tree force walk");
+}
+
+// The velocity walk's records from the node force sums.
+static void velocity_records(dem_tree *t, cudaStream_t s) {
+    walk_records_kernel<false><<<grid_for(t->ctx, t->node_count), 256, 0, counted(s)>>>(view(t), t->node_count, t->roots + 1);
+    t->vel_records = t->built;
 }
 
 int dem_tree_propagate_forces(dem_tree *t, const double *fx, const double *fy, const double *fz, void *stream) {
@@ -859,6 +973,7 @@ int dem_tree_propagate_forces(dem_tree *t, const double *fx, const double *fy, c
         const int a = t->level_off[l], b = l + 1 < nl ? t->level_off[l + 1] : t->parent_count;
         sweep_forces_kernel<<<grid_for(ctx, b - a), 256, 0, counted(s)>>>(view(t), a, b);
     }
+    velocity_records(t, s);
     return dem_check_launch(ctx, "tree propagate forces");
 }
 
@@ -866,6 +981,7 @@ int dem_tree_velocity(dem_tree *t, const double *fx, const double *fy, const dou
                       double theta_sq, double stokes_factor, double *vx, double *vy, double *vz, void *stream) {
     if (!t || !vx || !vy || !vz) return DEM_E_INVALID;
     if (t->n == 0) return DEM_OK;
+    if (!t->built) return dem_set_error(t->ctx, DEM_E_INVALID, "the tree's build did not complete");
     const int N = t->cap;
     if (!fx) {
         fx = t->pf;
@@ -873,24 +989,26 @@ int dem_tree_velocity(dem_tree *t, const double *fx, const double *fy, const dou
         fz = t->pf + 2 * (size_t)N;
     }
     cudaStream_t s = (cudaStream_t)stream;
+    if (!t->vel_records) velocity_records(t, s);  // no forces propagated on this tree: its links, the sums as they are
     dem_prof_begin(t->ctx, "tree_velocity_walk", s);
-    const int grid = ceil_div(t->n, 128);
+    const int grid = ceil_div(t->n, WALK_T);
     const TreeDev tv = view(t);
+    slot_forces_kernel<<<grid_for(t->ctx, t->n), 256, 0, counted(s)>>>(tv, t->n, fx, fy, fz);
     if (t->corr) {
         const CorrDev cv = corr_view(t->corr);
         if (t->periodic)
-            velocity_walk_kernel<true, true><<<grid, 128, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
+            velocity_walk_kernel<true, true><<<grid, WALK_T, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
                                                                            stokes_factor, cv, vx, vy, vz);
         else
-            velocity_walk_kernel<false, true><<<grid, 128, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
+            velocity_walk_kernel<false, true><<<grid, WALK_T, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
                                                                             stokes_factor, cv, vx, vy, vz);
     } else {
         const CorrDev none{};
         if (t->periodic)
-            velocity_walk_kernel<true, false><<<grid, 128, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
+            velocity_walk_kernel<true, false><<<grid, WALK_T, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
                                                                             stokes_factor, none, vx, vy, vz);
         else
-            velocity_walk_kernel<false, false><<<grid, 128, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
+            velocity_walk_kernel<false, false><<<grid, WALK_T, 0, counted(s)>>>(tv, fx, fy, fz, eta_const, theta_sq,
                                                                              stokes_factor, none, vx, vy, vz);
     }
     dem_prof_end(t->ctx, s);
