@@ -63,14 +63,9 @@ namespace dem {
 constexpr int RS_T = 256, RS_ITEMS = 8, RS_TILE = RS_T * RS_ITEMS;
 constexpr int BH_T = 128;     // threads per walk CTA (4 warps)
 constexpr int BH_STACK = 96;  // stack entries per warp (depth <= 10, <= 8 children per node)
-// resident CTAs per SM the two-target walks are compiled for (5: 94-96 registers, none spilled; 0.4 %
-// faster at N = 2^20 than 4 CTAs with 107-108 registers)
-#ifndef BH_WALK2_CTAS_FORCE
-#define BH_WALK2_CTAS_FORCE 5
-#endif
-#ifndef BH_WALK2_CTAS_VEL
-#define BH_WALK2_CTAS_VEL 5
-#endif
+// Warps per SM the two-target walks are compiled for (up to 128 registers); 20 (96 registers) and 24 (80): a few
+// per cent slower.
+constexpr int W2_WARPS = 16;
 constexpr int BH_MAX_LEVEL = 10;
 // meta.w = level | flags: the walks pass over a flagged node without a term (empty, or the reference's
 // skip tests: R^3 sum < 1e-30 m^3, flat_tree.py:861; |F sum|^2 < 1e-60 N^2, flat_tree.py:1155)
@@ -87,6 +82,9 @@ struct BhNodes {
     // walk records, one 16-byte-aligned group per node so that a visit issues vector loads:
     float4 *qr;  // [M][2] second moment Q = sum r^3 (x - c)(x - c)^T and R^3 sum:
                  //        (Qxx, Qxy, Qxz, Qyy), (Qyz, Qzz, R^3, 0)
+    // what a visit of the two-target walks reads, contiguous (scale_nodes_kernel, leaf_offsets_kernel):
+    float4 *wf;  // [M][4] force walk: meta, cs, qr
+    float4 *wv;  // [M][5] velocity walk: meta, cs, fd
     float4 *fd;  // [M][3] force sum and dipole D_ab = sum (x_a - c_a) F_b (row a, column b), as its
                  // symmetric part S = (D + D^T) / 2 and antisymmetric part A = D^T - D:
                  //        (Fx, Fy, Fz, Sxx), (Syy, Szz, 2 Sxy, 2 Sxz), (2 Syz, A01, A02, A12)
@@ -113,7 +111,7 @@ struct dem_bh {
     int32_t *bounds = nullptr;  // [9][max_nodes] child split points of the current level
     long long *bbox = nullptr;  // [6] min/max of an open box (order-preserving integers)
     double *geom = nullptr;     // [4] root cube origin x, y, z and side
-    unsigned long long *counters = nullptr;       // [2] pair and node terms of the last walk
+    unsigned long long *counters = nullptr;       // [2] pair and node terms of the last walk; then the queues
     unsigned long long *scales = nullptr;         // [2] max r, max |F| (bit patterns)
     int32_t *scan_in = nullptr, *coff = nullptr;  // [max_nodes + 1] children per node of a level, offsets
     BhNodes nd{};
@@ -689,6 +687,8 @@ struct BhWalk {
     float theta2;
     int window_level;
     double L, halfL;
+    int *queue;  // [queues] groups taken from each SM's share (two-target walks, T = 32)
+    int queues;
     unsigned long long *counters;  // [0] leaf pair terms, [1] accepted-node terms
     uint32_t *err;
     // periodic-image correction (velocity walk with CORR): FP32 grid view whose
@@ -985,11 +985,23 @@ __device__ __forceinline__ void stokeslet2(float2 ex, float2 ey, float2 ez, floa
     az = p_fma(rinv, p_fma(ez, sc, fz), az);
 }
 
-template <bool PER, bool FORCE>
-__global__ void __launch_bounds__(BH_T, FORCE ? BH_WALK2_CTAS_FORCE : BH_WALK2_CTAS_VEL)
+// Which 64 targets a warp takes.  T = 128: four consecutive groups per CTA.  T = 32: one group per CTA, from the
+// queue of the SM that runs it -- an equal, contiguous share of the groups, so that its 16 warps walk
+// neighbouring targets and share their nodes in L1 -- and, once that is empty, from the next SM's: every
+// CTA finds one group, and no warp waits for the slowest of four.  Few groups go to T = 128, whose warps
+// share an SM's caches even then.  Force / velocity walk, ms, theta 0.5 (0.7 at 262,144), before (T = 128, 20
+// warps per SM, meta, cs and moments in arrays of their own) -> T = 128 / T = 32: n = 5,000 0.67 / 0.74 ->
+// 0.63 / 0.71 | 0.81 / 0.95; 30,000 0.70 / 0.75 -> 0.65 / 0.74 | 0.81 / 0.96; 100,000 1.56 / 1.55 -> 1.40 / 1.51 |
+// 1.39 / 1.50; 262,144 1.33 / 1.31 -> 1.19 / 1.23 | 1.19 / 1.24; 2^20 9.78 / 9.70 -> 9.36 / 9.71 | 8.56 / 8.48.
+// (One group per CTA without queues: 8.85 / 8.78.  Records with every value twice, as the packed operations
+// take it: 9.6 / 11.7; the loads cost more than the moves.)
+constexpr int W2_QUEUED = 131072;  // targets from which T = 32
+
+template <bool PER, bool FORCE, int T>
+__global__ void __launch_bounds__(T, W2_WARPS * 32 / T)
     bh_walk2_kernel(const BhWalk w, double coeff, double stokes, double *__restrict__ ox, double *__restrict__ oy,
                     double *__restrict__ oz, double *__restrict__ fsort_out) {
-    __shared__ int stack[BH_T / 32][BH_STACK];
+    __shared__ int stack[T / 32][BH_STACK];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int n = w.n, cap = w.cap;
     const double inv_ell = pow2_inv_of(w.scales[0]);
@@ -999,8 +1011,27 @@ __global__ void __launch_bounds__(BH_T, FORCE ? BH_WALK2_CTAS_FORCE : BH_WALK2_C
     const float edge = (float)(w.L * inv_ell * (0.5 - 1e-6));  // leaf pairs: FP32 separations err by < 1e-6 L
     const double gox = w.geom[0], goy = w.geom[1], goz = w.geom[2];
     unsigned long long pairs = 0, nodes = 0;
-    const int warps = gridDim.x * (BH_T / 32);
-    for (int base = (blockIdx.x * (BH_T / 32) + wp) * 64; base < n; base += warps * 64) {
+    const int groups = (n + 63) / 64;
+    int group = blockIdx.x * (T / 32) + wp;
+    if (T == 32) {
+        if (lane == 0) {
+            unsigned sm;
+            asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+            const int share = (groups + w.queues - 1) / w.queues;
+            int q = (int)(sm % (unsigned)w.queues);
+            group = groups;
+            for (int tries = 0; tries < w.queues && group == groups; ++tries, q = q + 1 == w.queues ? 0 : q + 1) {
+                const int first = q * share, end = min(groups, first + share);
+                if (first < end) {
+                    const int g = first + atomicAdd(&w.queue[q], 1);
+                    if (g < end) group = g;
+                }
+            }
+        }
+        group = __shfl_sync(0xffffffffu, group, 0);
+    }
+    if (group < groups) {
+        const int base = group * 64;
         const int si0 = base + lane, si1 = base + 32 + lane;
         const bool v0 = si0 < n, v1 = si1 < n;
         const int nv = (int)v0 + (int)v1;
@@ -1028,11 +1059,12 @@ __global__ void __launch_bounds__(BH_T, FORCE ? BH_WALK2_CTAS_FORCE : BH_WALK2_C
             }
             const int node = stack[wp][--sp];
             __syncwarp();
-            const int4 mt = w.nd.meta[node];  // count, nchild, first child / droplet, level | flags
-            const float4 cs = w.nd.cs[node];
-            const float4 rec = FORCE ? w.nd.qr[2 * (size_t)node + 1] : w.nd.fd[3 * (size_t)node];
-            const float4 rq = FORCE ? w.nd.qr[2 * (size_t)node] : w.nd.fd[3 * (size_t)node + 1];
-            const float4 rd = FORCE ? make_float4(0.f, 0.f, 0.f, 0.f) : w.nd.fd[3 * (size_t)node + 2];
+            const float4 *const o = FORCE ? w.nd.wf + 4 * (size_t)node : w.nd.wv + 5 * (size_t)node;
+            const int4 mt = *reinterpret_cast<const int4 *>(o);  // count, nchild, first child / droplet, level | flags
+            const float4 cs = o[1];
+            const float4 rec = FORCE ? o[3] : o[2];
+            const float4 rq = FORCE ? o[2] : o[3];
+            const float4 rd = FORCE ? make_float4(0.f, 0.f, 0.f, 0.f) : o[4];
             const int cnt = mt.x;
             if (mt.w & (FORCE ? BH_SKIP_FORCE : BH_SKIP_VEL)) continue;  // empty, or :861 / :1155
             // force walk: D = c - x_i; velocity walk: e = x_i - c (= -D, the minimum image is odd)
@@ -1229,7 +1261,9 @@ __global__ void leaf_offsets_kernel(BhNodes nd, int nc, const double *__restrict
             loff[j] = o;
             reach = fmaxf(reach, fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z))));
         }
-        nd.qr[2 * (size_t)k + 1].w = reach;  // the leaf's largest |offset| on any axis (the walks' edge test)
+        // the leaf's largest |offset| on any axis (the walks' edge test)
+        nd.qr[2 * (size_t)k + 1].w = reach;
+        nd.wf[4 * (size_t)k + 3].w = reach;
     }
 }
 
@@ -1260,6 +1294,11 @@ __global__ void scale_nodes_kernel(BhNodes nd, int nc, const unsigned long long 
             const bool skip = cnt == 0 || (double)qr[6] < 1e-30 * s3;
             nd.meta[k] = make_int4(cnt, nch, nch ? nd.first_child[k] : nd.start[k],
                                    nd.level[k] | (skip ? BH_SKIP_FORCE : 0) | (cnt == 0 ? BH_SKIP_VEL : 0));
+            float4 *const w = nd.wf + 4 * (size_t)k;
+            *reinterpret_cast<int4 *>(w) = nd.meta[k];
+            w[1] = nd.cs[k];
+            w[2] = nd.qr[2 * (size_t)k];
+            w[3] = nd.qr[2 * (size_t)k + 1];
         } else {
             float *fd = reinterpret_cast<float *>(nd.fd + 3 * (size_t)k);  // F[0..2], then S and A (linear in D)
             for (int q = 0; q < 3; ++q) fd[q] = (float)((double)fd[q] * fsc);
@@ -1270,6 +1309,10 @@ __global__ void scale_nodes_kernel(BhNodes nd, int nc, const unsigned long long 
             const bool skip = mt.x == 0 || f2sum < 1e-60 * (fsc * fsc);
             mt.w = (mt.w & ~BH_SKIP_VEL) | (skip ? BH_SKIP_VEL : 0);
             nd.meta[k] = mt;
+            float4 *const w = nd.wv + 5 * (size_t)k;
+            *reinterpret_cast<int4 *>(w) = mt;
+            w[1] = nd.cs[k];
+            for (int q = 0; q < 3; ++q) w[2 + q] = nd.fd[3 * (size_t)k + q];
         }
     }
 }
@@ -1367,9 +1410,14 @@ static int bh_alloc(dem_ctx *ctx, T **p, size_t count, const char *what) {
     return dem_check_cuda(ctx, cudaMalloc((void **)p, sizeof(T) * (count > 0 ? count : 1)), what);
 }
 
+// Walk counters and the SMs' queues, zeroed before a walk.
+static size_t walk_counter_bytes(const dem_ctx *ctx) {
+    return sizeof(unsigned long long) * (2 + (ctx->sm_count + 1) / 2);
+}
+
 static void bh_free_nodes(BhNodes &nd) {
     void *ptrs[] = {nd.start, nd.count, nd.first_child, nd.nchild, nd.level, nd.cx, nd.cy,
-                    nd.cz,    nd.mom,   nd.cs,          nd.meta,   nd.qr,    nd.fd};
+                    nd.cz,    nd.mom,   nd.cs,          nd.meta,   nd.qr,    nd.fd,  nd.wf, nd.wv};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     nd = BhNodes{};
@@ -1388,6 +1436,8 @@ static int bh_nodes_reserve(dem_bh *b, int m, int keep, cudaStream_t s) {
         (rc = bh_alloc(ctx, &nn.cs, m, "bh nodes")) || (rc = bh_alloc(ctx, &nn.meta, m, "bh nodes")) ||
         (rc = bh_alloc(ctx, &nn.mom, 22 * (size_t)m, "bh nodes")) ||
         (rc = bh_alloc(ctx, &nn.qr, 2 * (size_t)m, "bh nodes")) ||
+        (rc = bh_alloc(ctx, &nn.wf, 4 * (size_t)m, "bh nodes")) ||
+        (rc = bh_alloc(ctx, &nn.wv, 5 * (size_t)m, "bh nodes")) ||
         (rc = bh_alloc(ctx, &nn.fd, 3 * (size_t)m, "bh nodes"))) {
         bh_free_nodes(nn);
         return rc;
@@ -1433,6 +1483,22 @@ static inline int grid_of(dem_ctx *ctx, long long work, int threads = 256) {
 // One past the last node of level l.
 static int level_end(const dem_bh *b, int l) { return l + 1 < b->nlevels ? b->level_off[l + 1] : b->node_count; }
 
+template <bool FORCE>
+static void launch_walk2(const dem_bh *b, const BhWalk &w, double coeff, double stokes, double *ox, double *oy,
+                         double *oz, double *fsort_out, cudaStream_t s) {
+    const int groups = (b->n + 63) / 64, blocks = (groups + 3) / 4;
+    if (b->n >= W2_QUEUED) {
+        if (b->periodic)
+            bh_walk2_kernel<true, FORCE, 32><<<groups, 32, 0, counted(s)>>>(w, coeff, stokes, ox, oy, oz, fsort_out);
+        else
+            bh_walk2_kernel<false, FORCE, 32><<<groups, 32, 0, counted(s)>>>(w, coeff, stokes, ox, oy, oz, fsort_out);
+    } else if (b->periodic) {
+        bh_walk2_kernel<true, FORCE, 128><<<blocks, 128, 0, counted(s)>>>(w, coeff, stokes, ox, oy, oz, fsort_out);
+    } else {
+        bh_walk2_kernel<false, FORCE, 128><<<blocks, 128, 0, counted(s)>>>(w, coeff, stokes, ox, oy, oz, fsort_out);
+    }
+}
+
 extern "C" {
 
 int dem_bh_create(dem_ctx *ctx, int capacity, dem_bh **out) {
@@ -1451,7 +1517,7 @@ int dem_bh_create(dem_ctx *ctx, int capacity, dem_bh **out) {
         (rc = bh_alloc(ctx, &b->ps, 4 * n, "bh")) || (rc = bh_alloc(ctx, &b->fsort, 3 * n, "bh")) ||
         (rc = bh_alloc(ctx, &b->loff, n, "bh")) || (rc = bh_alloc(ctx, &b->fs32, n, "bh")) ||
         (rc = bh_alloc(ctx, &b->bbox, 6, "bh")) || (rc = bh_alloc(ctx, &b->geom, 4, "bh")) ||
-        (rc = bh_alloc(ctx, &b->counters, 2, "bh")) || (rc = bh_alloc(ctx, &b->scales, 2, "bh")) ||
+        (rc = bh_alloc(ctx, &b->counters, walk_counter_bytes(ctx) / sizeof(unsigned long long), "bh")) || (rc = bh_alloc(ctx, &b->scales, 2, "bh")) ||
         (rc = bh_nodes_reserve(b, std::max(4096, capacity / 4), 0, nullptr))) {
         bh_free(b);
         return rc;
@@ -1552,6 +1618,8 @@ int dem_bh_build(dem_bh *b, int n, const double *x, const double *y, const doubl
 static BhWalk walk_args(dem_bh *b, float theta) {
     BhWalk w;
     w.n = b->n;
+    w.queue = reinterpret_cast<int *>(b->counters + 2);
+    w.queues = b->ctx->sm_count;
     w.cap = b->capacity;
     w.node_count = b->node_count;
     w.ps = b->ps;
@@ -1581,21 +1649,17 @@ static BhWalk walk_args(dem_bh *b, float theta) {
 
 static int walk_grid(dem_bh *b) { return std::max(1, (b->n + BH_T - 1) / BH_T); }
 // bh_walk2_kernel: 64 targets per warp
-static int walk2_grid(dem_bh *b) { return std::max(1, (b->n + 2 * BH_T - 1) / (2 * BH_T)); }
 
 int dem_bh_forces(dem_bh *b, double m_const, double theta, double *fx, double *fy, double *fz, void *stream) {
     if (!b || !(theta >= 0)) return DEM_E_INVALID;
     dem_ctx *ctx = b->ctx;
     cudaStream_t s = (cudaStream_t)stream;
     if (b->n == 0) return DEM_OK;
-    int rc = dem_check_cuda(ctx, cudaMemsetAsync(b->counters, 0, 2 * sizeof(unsigned long long), s), "memset");
+    int rc = dem_check_cuda(ctx, cudaMemsetAsync(b->counters, 0, walk_counter_bytes(ctx), s), "memset");
     if (rc) return rc;
     const BhWalk w = walk_args(b, (float)theta);
     dem_prof_begin(ctx, "bh_force_walk", s);
-    if (b->periodic)
-        bh_walk2_kernel<true, true><<<walk2_grid(b), BH_T, 0, counted(s)>>>(w, m_const, 0.0, fx, fy, fz, b->fsort);
-    else
-        bh_walk2_kernel<false, true><<<walk2_grid(b), BH_T, 0, counted(s)>>>(w, m_const, 0.0, fx, fy, fz, b->fsort);
+    launch_walk2<true>(b, w, m_const, 0.0, fx, fy, fz, b->fsort, s);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "bh force walk");
 }
@@ -1623,7 +1687,7 @@ int dem_bh_velocity(dem_bh *b, const double *fx, const double *fy, const double 
     }
     scale_nodes_kernel<<<grid_of(ctx, le), 256, 0, counted(s)>>>(b->nd, le, b->scales, b->geom, 1);
     scale_forces_kernel<<<grid_of(ctx, n), 256, 0, counted(s)>>>(n, b->capacity, b->fsort, b->scales, b->fs32);
-    if ((rc = dem_check_cuda(ctx, cudaMemsetAsync(b->counters, 0, 2 * sizeof(unsigned long long), s), "memset")))
+    if ((rc = dem_check_cuda(ctx, cudaMemsetAsync(b->counters, 0, walk_counter_bytes(ctx), s), "memset")))
         return rc;
     const BhWalk w = walk_args(b, (float)theta);
     dem_prof_begin(ctx, "bh_velocity_walk", s);
@@ -1634,12 +1698,8 @@ int dem_bh_velocity(dem_bh *b, const double *fx, const double *fy, const double 
         else
             bh_walk_kernel<false, false, true><<<walk_grid(b), BH_T, 0, counted(s)>>>(w, eta_const, stokes_factor, vx,
                                                                                       vy, vz, nullptr);
-    } else if (b->periodic) {
-        bh_walk2_kernel<true, false><<<walk2_grid(b), BH_T, 0, counted(s)>>>(w, eta_const, stokes_factor, vx, vy, vz,
-                                                                             nullptr);
     } else {
-        bh_walk2_kernel<false, false><<<walk2_grid(b), BH_T, 0, counted(s)>>>(w, eta_const, stokes_factor, vx, vy,
-                                                                              vz, nullptr);
+        launch_walk2<false>(b, w, eta_const, stokes_factor, vx, vy, vz, nullptr, s);
     }
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "bh velocity walk");
