@@ -317,8 +317,8 @@ DEM_API int dem_corr_info(const dem_corr *corr, int *n, double *common, double *
 
 /* Roofline probe of the FP32 correction pass (no counterpart in the
  * reference): ctas x 256 threads each read per_thread cells of the FP32 table
- * at pseudo-random positions, 96 bytes per cell in three 256-bit loads, and
- * write one float each to out (device, ctas * 256 floats).  Time it on
+ * at pseudo-random positions, 96 bytes per cell (four lanes read each other's
+ * cells in turn, 32 bytes a lane), and write one float each to out (device, ctas * 256 floats).  Time it on
  * `stream` to get the table's random-gather bandwidth. */
 DEM_API int dem_corr_gather_probe(const dem_corr *corr, int ctas, int per_thread, float *out, void *stream);
 

@@ -2,12 +2,18 @@
 // direct pass (the FP64 direct pass is fused into direct_fp64.cu, the tree
 // walks take it in tree.cu and bh.cu).
 //
-// Direct FP32 pass: one thread per target i, j in shared-memory tiles split
-// over blockIdx.y; per pair three cell lookups (three 256-bit loads each from
-// one 128-byte line; the table, (n-1)^3 x 128 B, stays in L2) and 63 FMA of
-// trilinear forms.  Runs of 32 terms
-// are summed in FP32 and added in FP64; the j-chunk partials are reduced in a
-// fixed order, so results are deterministic.
+// Direct FP32 pass: four lanes per target i, j in shared-memory tiles split
+// over blockIdx.y; per pair three cell lookups (96 bytes each of one 128-byte
+// line; the table, (n-1)^3 x 128 B, stays in L2) and 63 FMA of trilinear
+// forms.  Lane o of a target's four (the last one idle) computes component o of
+// the velocity: it needs one 32-byte component of each cell, so the four lanes'
+// 256-bit loads fall into one line.  Bound: the L1's lines per instruction.
+// With one lane per target every load of a warp touched 32 lines, a component
+// each (3.08 ms at N = 8,192 on a 48^3 grid, 12.3 at 16,384); four lanes
+// touch 8 (1.05 and 4.1 ms), for three times the index arithmetic, which the
+// issue slots have room for.  Runs of 32 terms are summed in FP32 and added in
+// FP64; the j-chunk partials are reduced in a fixed order, so results are
+// deterministic.
 //
 // The grid is not periodic (free-space Stokeslet subtracted), so a pair whose
 // minimum image flips changes its term by O(|G| |F_j|), while the sum over j
@@ -21,12 +27,17 @@
 
 namespace dem {
 
-constexpr int CORR_T = 128;      // threads (targets) per CTA
+constexpr int CORR_T = 128;      // threads per CTA
+constexpr int CORR_U = 2;        // pairs of a lane in flight; 4 are 8 % slower at N = 8,192, 1 is 40 % slower at 500
+constexpr int CORR_CTAS = 6;     // resident per SM: 80 registers; 1 asked: 1.13 ms at N = 8,192, 6: 1.05, 8 and 10:
+                                 // 1.03 and 1.05, but 26 and 28 us at 500 against 21 (loads no longer side by side)
+constexpr int CORR_OWN = CORR_T / 4;  // targets per CTA
 constexpr int CORR_TILE = 256;   // j per shared-memory tile
 constexpr int CORR_SUB = 32;     // terms per FP32 partial: the sums cancel to ~1e-3 of sum |term|
+static_assert(CORR_TILE % CORR_SUB == 0 && CORR_SUB % CORR_U == 0, "whole runs");
 
 template <bool PER>
-__global__ void __launch_bounds__(CORR_T) corr_direct_fp32_kernel(int n, int j_chunk, const double *__restrict__ x,
+__global__ void __launch_bounds__(CORR_T, CORR_CTAS) corr_direct_fp32_kernel(int n, int j_chunk, const double *__restrict__ x,
                                                                   const double *__restrict__ y,
                                                                   const double *__restrict__ z,
                                                                   const double *__restrict__ fx,
@@ -37,63 +48,72 @@ __global__ void __launch_bounds__(CORR_T) corr_direct_fp32_kernel(int n, int j_c
                                                                   double *__restrict__ partial, size_t plane) {
     __shared__ float4 sp[CORR_TILE];  // x, y, z, -
     __shared__ float4 ss[CORR_TILE];  // F_j * common
-    const int i = blockIdx.x * CORR_T + threadIdx.x;
-    const bool active = i < n;
+    const int lane4 = threadIdx.x & 3, o = min(lane4, 2);
+    const int i = blockIdx.x * CORR_OWN + (threadIdx.x >> 2);
+    const int own = min(i, n - 1);
     const int j0 = blockIdx.y * j_chunk, j1 = min(n, j0 + j_chunk);
-    float xi = 0.f, yi = 0.f, zi = 0.f;
-    if (active) {
-        xi = (float)x[i];
-        yi = (float)y[i];
-        zi = (float)z[i];
-    }
-    double Cx = 0.0, Cy = 0.0, Cz = 0.0;
+    const float xi = (float)x[own], yi = (float)y[own], zi = (float)z[own];
+    // component o of G_z, G_x, G_y: u v w, w v u, u w v
+    const float *const b1 = c.c32 + 8 * o, *const b2 = c.c32 + 8 * (2 - o), *const b3 = c.c32 + 8 * ((3 - o) % 3);
+    double C = 0.0;
     for (int t0 = j0; t0 < j1; t0 += CORR_TILE) {
         __syncthreads();
         for (int k = threadIdx.x; k < CORR_TILE; k += CORR_T) {
-            const int j = t0 + k;
-            if (j < j1) {
-                sp[k] = make_float4((float)x[j], (float)y[j], (float)z[j], 0.f);
-                ss[k] = make_float4((float)(fx[j] * common), (float)(fy[j] * common), (float)(fz[j] * common), 0.f);
-            }
+            const int j = min(t0 + k, n - 1);
+            sp[k] = make_float4((float)x[j], (float)y[j], (float)z[j], 0.f);
+            ss[k] = make_float4((float)(fx[j] * common), (float)(fy[j] * common), (float)(fz[j] * common), 0.f);
         }
         __syncthreads();
         const int cnt = min(CORR_TILE, j1 - t0);
-        if (!active) continue;
         for (int k0 = 0; k0 < cnt; k0 += CORR_SUB) {
-            float cx = 0.f, cy = 0.f, cz = 0.f;
+            float sum = 0.f;
             const int k1 = min(cnt, k0 + CORR_SUB);
-            for (int k = k0; k < k1; ++k) {
-                if (t0 + k == i) continue;
-                const float4 p = sp[k];
-                float dx = xi - p.x, dy = yi - p.y, dz = zi - p.z;
-                if (PER) {
-                    if (fabsf(fabsf(dx) - edge) < edge_tol || fabsf(fabsf(dy) - edge) < edge_tol ||
-                        fabsf(fabsf(dz) - edge) < edge_tol) {  // image decision in FP64 (rare)
-                        const int j = t0 + k;
-                        const double hL = 0.5 * Ld;
-                        dx = (float)mic64(x[i] - x[j], Ld, hL);
-                        dy = (float)mic64(y[i] - y[j], Ld, hL);
-                        dz = (float)mic64(z[i] - z[j], Ld, hL);
-                    } else {  // |d| > L/2 -> d - sign(d) L (positions in [0, L))
-                        dx = fmaf(-L, rintf(dx * invL), dx);
-                        dy = fmaf(-L, rintf(dy * invL), dy);
-                        dz = fmaf(-L, rintf(dz * invL), dz);
+            for (int k = k0; k < k1; k += CORR_U) {
+                int cell[CORR_U][3];
+                float t[CORR_U][3], g1[CORR_U][8], g2[CORR_U][8], g3[CORR_U][8];
+#pragma unroll
+                for (int q = 0; q < CORR_U; ++q) {
+                    const float4 p = sp[k + q];
+                    float dx = xi - p.x, dy = yi - p.y, dz = zi - p.z;
+                    if (PER) {
+                        if (fabsf(fabsf(dx) - edge) < edge_tol || fabsf(fabsf(dy) - edge) < edge_tol ||
+                            fabsf(fabsf(dz) - edge) < edge_tol) {  // image decision in FP64 (rare)
+                            const int j = min(t0 + k + q, n - 1);
+                            const double hL = 0.5 * Ld;
+                            dx = (float)mic64(x[own] - x[j], Ld, hL);
+                            dy = (float)mic64(y[own] - y[j], Ld, hL);
+                            dz = (float)mic64(z[own] - z[j], Ld, hL);
+                        } else {  // |d| > L/2 -> d - sign(d) L (positions in [0, L))
+                            dx = fmaf(-L, rintf(dx * invL), dx);
+                            dy = fmaf(-L, rintf(dy * invL), dy);
+                            dz = fmaf(-L, rintf(dz * invL), dz);
+                        }
                     }
+                    corr_axis32(c, dx, cell[q][0], t[q][0]);
+                    corr_axis32(c, dy, cell[q][1], t[q][1]);
+                    corr_axis32(c, dz, cell[q][2], t[q][2]);
                 }
-                const float4 s = ss[k];
-                corr_pair32(c, dx, dy, dz, s.x, s.y, s.z, cx, cy, cz);
+#pragma unroll
+                for (int q = 0; q < CORR_U; ++q) {
+                    const int ax = cell[q][0], ay = cell[q][1], az = cell[q][2], m = c.m;
+                    corr_ld8(b1 + ((ax * m + ay) * m + az) * CORR_CELL32, g1[q]);
+                    corr_ld8(b2 + ((az * m + ay) * m + ax) * CORR_CELL32, g2[q]);
+                    corr_ld8(b3 + ((ax * m + az) * m + ay) * CORR_CELL32, g3[q]);
+                }
+#pragma unroll
+                for (int q = 0; q < CORR_U; ++q) {
+                    const float4 s = ss[k + q];
+                    const float tx = t[q][0], ty = t[q][1], tz = t[q][2];
+                    const float gz = corr_eval32(g1[q], tx, ty, tz), gx = corr_eval32(g2[q], tz, ty, tx),
+                                gy = corr_eval32(g3[q], tx, tz, ty);
+                    const float next = fmaf(gx, s.x, fmaf(gy, s.y, fmaf(gz, s.z, sum)));
+                    if (k + q < k1 && t0 + k + q != i) sum = next;
+                }
             }
-            Cx += (double)cx;
-            Cy += (double)cy;
-            Cz += (double)cz;
+            C += (double)sum;
         }
     }
-    if (active) {
-        double *P = partial + (size_t)blockIdx.y * 3 * plane;
-        P[i] = Cx;
-        P[plane + i] = Cy;
-        P[2 * plane + i] = Cz;
-    }
+    if (i < n && lane4 < 3) partial[((size_t)blockIdx.y * 3 + o) * plane + i] = C;
 }
 
 // v_i += sum over chunks (in order) + g_self F_i
@@ -118,20 +138,20 @@ __global__ void corr_reduce_kernel(int n, int splits, const double *__restrict__
 int launch_corr_direct_fp32(dem_ctx *ctx, const dem_corr *c, int n, const double *x, const double *y,
                             const double *z, const double *fx, const double *fy, const double *fz, double L,
                             int periodic, double *vx, double *vy, double *vz, cudaStream_t s) {
-    const int iblocks = ceil_div(n, CORR_T);
-    // enough CTAs for ~4 waves at 8 resident CTAs per SM, chunks of whole tiles
-    const int want = std::max(1, ceil_div(32LL * ctx->sm_count, iblocks));
-    const int j_chunk = ceil_div(ceil_div(n, std::min(want, ceil_div(n, CORR_TILE))), CORR_TILE) * CORR_TILE;
+    // Up to 64 CTAs per SM (an even finish: 16 per SM took 5 % longer at N = 8,192), chunks of at least two runs
+    // (whole tiles leave N = 500 with 32 CTAs: 64 us, against 21).
+    const int want = std::max(1, ceil_div(64LL * ctx->sm_count, ceil_div(n, CORR_OWN)));
+    const int j_chunk = ceil_div(ceil_div(n, want), 2 * CORR_SUB) * 2 * CORR_SUB;
     const int splits = ceil_div(n, j_chunk);
-    int rc = dem_ensure_partials(ctx, splits);
+    int rc = dem_ensure_partials(ctx, ceil_div((int64_t)splits * n, (int64_t)ctx->capacity));
     if (rc) return rc;
-    const size_t plane = (size_t)ctx->capacity;
+    const size_t plane = (size_t)n;
     const CorrF32 cf = corr_f32(c, 1.0);
     const float Lf = (float)L, invL = periodic ? (float)(1.0 / L) : 0.f;
     // FP32 separations err by <= ~2 ulp(L) ~ 2.4e-7 L: a margin of 1e-6 L catches every flip
     const float edge = (float)(0.5 * L), edge_tol = (float)(1e-6 * L);
     dem_prof_begin(ctx, "corr_direct_pass", s);
-    const dim3 grid(iblocks, splits);
+    const dim3 grid(ceil_div(n, CORR_OWN), splits);
     if (periodic)
         corr_direct_fp32_kernel<true><<<grid, CORR_T, 0, counted(s)>>>(n, j_chunk, x, y, z, fx, fy, fz, cf, c->common,
                                                                        Lf, invL, edge, edge_tol, L, ctx->partial,
@@ -147,24 +167,33 @@ int launch_corr_direct_fp32(dem_ctx *ctx, const dem_corr *c, int n, const double
 }
 
 // Roofline probe: every thread reads `per_thread` cells at pseudo-random
-// (xorshift) positions of the FP32 table, 96 bytes each (the three 256-bit
-// component loads of one lookup), and writes one sum.
+// (xorshift) positions of the FP32 table, 96 bytes each, the way the pass does
+// (four lanes read the cells of the four in turn, a component each), and writes
+// one sum.
 __global__ void corr_gather_probe_kernel(const float *__restrict__ c32, int cells, int per_thread,
                                          float *__restrict__ out) {
     const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane4 = threadIdx.x & 3, o = min(lane4, 2);
     uint32_t h = tid * 2654435761u + 12345u;
     float acc = 0.f;
     for (int k = 0; k < per_thread; ++k) {
         h ^= h << 13;
         h ^= h >> 17;
         h ^= h << 5;
-        const float *p = c32 + (size_t)(h % (uint32_t)cells) * CORR_CELL32;
-        float u[8], v[8], w[8];
-        corr_ld8(p, u);
-        corr_ld8(p + 8, v);
-        corr_ld8(p + 16, w);
+        const uint32_t cell = h % (uint32_t)cells;
+        float u[4][8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc += u[q] + v[q] + w[q];
+        for (int q = 0; q < 4; ++q)
+            corr_ld8(c32 + (size_t)__shfl_sync(0xffffffffu, cell, q, 4) * CORR_CELL32 + 8 * o, u[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float sum = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum += u[q][e];
+            const float s1 = __shfl_sync(0xffffffffu, sum, 1, 4), s2 = __shfl_sync(0xffffffffu, sum, 2, 4),
+                        s0 = __shfl_sync(0xffffffffu, sum, 0, 4);
+            if (lane4 == q) acc += s0 + s1 + s2;
+        }
     }
     out[tid] = acc;
 }

@@ -20,7 +20,8 @@
 //   c32: 32 floats   u[8] v[8] w[8] pad[8]   monomial coefficients of the same
 //        trilinear form (a0 a1 a2 a3 b0 b1 b2 b3, evaluated by corr_eval32),
 //        rounded once from FP64 differences; one 128-byte line per cell, one
-//        256-bit load per component
+//        256-bit load per component (which neighbouring lanes take side by side
+//        where they can)
 // The FP64 functions restate the reference's expressions in its order and must
 // be compiled without multiply-add contraction (-fmad=false).
 #pragma once
