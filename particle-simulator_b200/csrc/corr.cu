@@ -211,7 +211,7 @@ int launch_direct_convection_mixed(dem_ctx *, int, const double *, const double 
 static void build_cells(int n, const double *u, const double *v, const double *w, std::vector<double> &c64,
                         std::vector<float> &c32) {
     const size_t m = (size_t)n - 1;
-    c64.assign(m * m * m * 24, 0.0);
+    c64.assign(m * m * m * 2 * CORR_CELL64, 0.0);
     c32.assign(m * m * m * CORR_CELL32, 0.f);
     const double *g[3] = {u, v, w};
     for (size_t a = 0; a < m; ++a)
@@ -223,7 +223,7 @@ static void build_cells(int n, const double *u, const double *v, const double *w
                     for (int q = 0; q < 8; ++q) {
                         const size_t ia = a + (q >> 2), ib = b + ((q >> 1) & 1), id = d + (q & 1);
                         k[q] = g[comp][(ia * n + ib) * n + id];
-                        c64[cell * 24 + comp * 8 + q] = k[q];
+                        c64[cell * 2 * CORR_CELL64 + (q >> 2) * 16 + comp * 4 + (q & 3)] = k[q];
                     }
                     // f = a0 + t3 a1 + t2 (a2 + t3 a3) + t1 (b0 + t3 b1 + t2 (b2 + t3 b3))
                     const double a0 = k[0], a1 = k[1] - k[0], a2 = k[2] - k[0], a3 = (k[3] - k[2]) - (k[1] - k[0]);

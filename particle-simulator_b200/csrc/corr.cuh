@@ -16,7 +16,8 @@
 //
 // Device layout: cell-major.  Cell (a, b, c) of the (n-1)^3 cells holds what
 // one lookup needs, so a lookup reads one contiguous block:
-//   c64: 24 doubles  u[8] v[8] w[8]   corner values, corner k = (k>>2, (k>>1)&1, k&1)
+//   c64: two lines of 16 doubles  u[4] v[4] w[4] pad[4]  corner values, corner
+//        k = (k>>2, (k>>1)&1, k&1): k = 0..3 in the first line, 4..7 in the second
 //   c32: 32 floats   u[8] v[8] w[8] pad[8]   monomial coefficients of the same
 //        trilinear form (a0 a1 a2 a3 b0 b1 b2 b3, evaluated by corr_eval32),
 //        rounded once from FP64 differences; one 128-byte line per cell, one
@@ -28,10 +29,12 @@
 
 #include "common.cuh"
 
+constexpr int CORR_CELL64 = 16;  // double2 per cell in the FP64 table
+
 struct dem_corr {
     dem_ctx *ctx = nullptr;
     int n = 0;                  // grid points per axis
-    double2 *c64 = nullptr;     // (n-1)^3 cells x 12 double2
+    double2 *c64 = nullptr;     // (n-1)^3 cells x 16 double2 (128-byte aligned)
     float *c32 = nullptr;       // (n-1)^3 cells x 32 floats (128-byte aligned)
     double gmin = 0, ginv = 0;  // first node, 1 / spacing
     double Fz_inv = 0, cL = 0, eta_r = 0;
@@ -74,10 +77,11 @@ __device__ __forceinline__ double corr_interp64(const double (&c)[8], double t1,
 __device__ __forceinline__ void corr_cell64(const CorrDev &c, int a, int b, int d, double (&u)[8], double (&v)[8],
                                             double (&w)[8]) {
     const int m = c.n - 1;
-    const double2 *p = c.c64 + (((size_t)a * m + b) * m + d) * 12;
+    const double2 *p = c.c64 + (((size_t)a * m + b) * m + d) * CORR_CELL64;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const double2 qu = __ldg(p + k), qv = __ldg(p + 4 + k), qw = __ldg(p + 8 + k);
+        const double2 *h = p + 8 * (k >> 1) + (k & 1);
+        const double2 qu = __ldg(h), qv = __ldg(h + 2), qw = __ldg(h + 4);
         u[2 * k] = qu.x;
         u[2 * k + 1] = qu.y;
         v[2 * k] = qv.x;
@@ -85,6 +89,12 @@ __device__ __forceinline__ void corr_cell64(const CorrDev &c, int a, int b, int 
         w[2 * k] = qw.x;
         w[2 * k + 1] = qw.y;
     }
+}
+
+// One component's corner values (p: the component's first), a 256-bit load per line.
+__device__ __forceinline__ void corr_ld8(const double2 *p, double (&a)[8]) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a[0]), "=d"(a[1]), "=d"(a[2]), "=d"(a[3]) : "l"(p));
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a[4]), "=d"(a[5]), "=d"(a[6]), "=d"(a[7]) : "l"(p + 8));
 }
 
 // One pair (or accepted node): (x, y, z) = MIC(x_i - x_j), F = F_j; adds the

@@ -28,9 +28,13 @@
 //
 // With the periodic-image correction loaded, the convection kernel adds each
 // pair's correction term right after its Stokeslet term and the self term
-// after the loop (:413-464), bit-identical to the CPU restatement.  It is
-// bound by the correction table's gathers: n = 2,000 7,520 -> 550 us, 8,192
-// 30,800 -> 7,600.
+// after the loop (:413-464), bit-identical to the CPU restatement.  Bound: the
+// lines of the correction table that the L1 passes per pair, then the FP64
+// pipe (~500 operations per pair).  Four lanes take a component each of the
+// cells of one pair after another (corr_four), from a table whose half cells
+// are a line each: n = 2,000 7,520 -> 232 us, 8,192 30,800 -> 3,030, 16,384
+// 62,200 -> 11,700 (one lane per pair: 550, 7,600, 30,300; four lanes over
+// cells of 192 bytes side by side: 319, 4,330, 17,000).
 #include "common.cuh"
 #include "corr.cuh"
 #include "ieee64.cuh"
@@ -164,6 +168,35 @@ __device__ __forceinline__ bool oseen_term64(double X, double Y, double Z, doubl
     return ok;
 }
 
+// corr_pair64 from zero for the pairs of four neighbouring lanes, which have their j in common: lane o takes
+// component o of each lane's pair in turn (the last lane o = 2 again, unwritten), so that the four read
+// from one line.  Two pairs in flight: 4 unrolled are 15 % slower, one 7 %.  Written to out[q] (component 0 of lane q's pair), its planes `cs` apart.
+__device__ __forceinline__ void corr_four(const CorrDev &c, double X, double Y, double Z, double Fx, double Fy,
+                                          double Fz, double *out, int cs) {
+    const int lane4 = threadIdx.x & 3, o = min(lane4, 2);
+    int ax, ay, az;
+    double tx, ty, tz;
+    corr_axis64(X * c.cL, c.gmin, c.ginv, c.n, ax, tx);
+    corr_axis64(Y * c.cL, c.gmin, c.ginv, c.n, ay, ty);
+    corr_axis64(Z * c.cL, c.gmin, c.ginv, c.n, az, tz);
+    const int m = c.n - 1;
+    const int cell1 = (ax * m + ay) * m + az, cell2 = (az * m + ay) * m + ax, cell3 = (ax * m + az) * m + ay;
+    const double sx = Fx * c.common, sy = Fy * c.common, sz = Fz * c.common;
+    const double2 *const b1 = c.c64 + 2 * o, *const b2 = c.c64 + 2 * (2 - o), *const b3 = c.c64 + 2 * ((3 - o) % 3);
+#pragma unroll 2
+    for (int q = 0; q < 4; ++q) {
+        const double t1 = __shfl_sync(0xffffffffu, tx, q, 4), t2 = __shfl_sync(0xffffffffu, ty, q, 4),
+                     t3 = __shfl_sync(0xffffffffu, tz, q, 4);
+        double g1[8], g2[8], g3[8];
+        corr_ld8(b1 + CORR_CELL64 * (size_t)__shfl_sync(0xffffffffu, cell1, q, 4), g1);
+        corr_ld8(b2 + CORR_CELL64 * (size_t)__shfl_sync(0xffffffffu, cell2, q, 4), g2);
+        corr_ld8(b3 + CORR_CELL64 * (size_t)__shfl_sync(0xffffffffu, cell3, q, 4), g3);
+        const double gz = corr_interp64(g1, t1, t2, t3), gx = corr_interp64(g2, t3, t2, t1),
+                     gy = corr_interp64(g3, t1, t3, t2);
+        if (lane4 < 3) out[o * cs + q] = 0.0 + (gx * sx + gy * sy + gz * sz);
+    }
+}
+
 template <int R, bool PER, int KIND>
 __global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>::CTAS) ordered_pass_kernel(const Ord64Args a) {
     using S = OrdShape<R, KIND>;
@@ -234,18 +267,14 @@ __global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>:
                     w[0] = v.x;
                     w[S::CS] = v.y;
                     w[2 * S::CS] = v.z;
-                    if (KIND == OSEEN64_CORR) {
-                        D3 c{0.0, 0.0, 0.0};
-                        corr_pair64(a.corr, X, Y, Z, p1.y, p2.x, p2.y, c.x, c.y, c.z);
-                        w[3 * S::CS] = c.x;
-                        w[4 * S::CS] = c.y;
-                        w[5 * S::CS] = c.z;
-                    }
+                    if (KIND == OSEEN64_CORR && !decltype(plain)::value)
+                        corr_four(a.corr, X, Y, Z, p1.y, p2.x, p2.y, w - (tid & 3) + 3 * S::CS, S::CS);
                     return ok;
                 };
                 unsigned redo = row_ok && !odd ? 0u : (1u << S::U) - 1u;
 #pragma unroll
                 for (int u = 0; u < S::U; ++u) redo |= term(u, std::false_type{}) ? 0u : 1u << u;
+                if (KIND == OSEEN64_CORR) __syncwarp();  // the corrections are neighbours' writes
                 while (redo) {
                     const int u = __ffs(redo) - 1;
                     redo &= redo - 1;
