@@ -23,7 +23,7 @@
 #include "scan.cuh"
 
 constexpr int WALK_T = 128;  // threads per CTA of the walks
-constexpr size_t WALK_REC_BYTES = 64, WALK_DIP_BYTES = 80;
+constexpr size_t WALK_REC_BYTES = 64, WALK_DIP_BYTES = 96;
 
 struct dem_tree {
     dem_ctx *ctx = nullptr;  // must outlive the tree while kernels run; destroy does not touch it
@@ -402,7 +402,7 @@ __global__ void sweep_forces_kernel(TreeDev t, int a, int b) {
     }
 }
 // ---------------------------------------------------------------------------
-// Walk records.  A walk visits a node through one 64-byte record: the size
+// Walk records.  A walk visits a node through one 64-byte record (two loads): the size
 // squared and the centre (the same expressions the reference evaluates at every
 // visit, :466-520, evaluated once), what the accepted node needs, and two links
 // that leave out the nodes the walk passes over without a term (empty, R^3 sum
@@ -411,21 +411,33 @@ __global__ void sweep_forces_kernel(TreeDev t, int a, int b) {
 // (or what follows them), and the next node when it is done.  Links: -1 the end;
 // child <= -2 marks a leaf whose first slot is -2 - child.
 // ---------------------------------------------------------------------------
-struct __align__(16) ForceRec {
+struct __align__(32) ForceRec {
     double s2, cx, cy, cz, r3;
     int32_t child, next, count, pad[3];
 };
-struct __align__(16) VelRec {
+struct __align__(32) VelRec {
     double s2, cx, cy, cz;
     int32_t child, next;
     double fx, fy, fz;
 };
 // Dipole D_ab = P_ab - c_a F_b about the centre (:1215-1230) and its trace.
-struct __align__(16) DipRec {
-    double d[9], tr;
+struct __align__(32) DipRec {
+    double d[9], tr, pad[2];
 };
 static_assert(sizeof(ForceRec) == WALK_REC_BYTES && sizeof(VelRec) == WALK_REC_BYTES && sizeof(DipRec) == WALK_DIP_BYTES,
               "the tree's allocation");
+
+// Half a record or one droplet: 32 bytes (so aligned) in one 256-bit load.
+struct Half {
+    double a, b, c, d;
+};
+__device__ __forceinline__ Half half_at(const void *p, int k) {
+    Half h;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(h.a), "=d"(h.b), "=d"(h.c), "=d"(h.d)
+        : "l"((const char *)p + 32 * (size_t)k));
+    return h;
+}
 
 template <bool FORCE>
 __device__ __forceinline__ bool passed_over(const TreeDev &t, int k) {
@@ -500,7 +512,10 @@ __global__ void slot_forces_kernel(TreeDev t, int n, const double *__restrict__ 
 // Bound: latency (a visit's record, a chain of FP64 operations) and divergence (13 of 32 lanes active on
 // average): 21 warps per SM are all there is at N = 100,000.  N = 100,003, one droplet per leaf, open, force /
 // total-velocity walk: 2.00 / 3.54 ms with 11 to 23 scattered loads and a division per visit, half of the
-// visits on empty nodes; 1.24 / 2.13 ms now; 16 droplets per leaf, periodic: 11.5 / 15.0 -> 5.5 / 7.7.
+// visits on empty nodes; 1.24 / 2.13 ms with records, links past those nodes and terms taken together, 1.19 /
+// 1.96 with 256-bit loads (a diverged warp's loads pass the L1 a line at a time: two per visit instead of
+// four); 16 droplets per leaf, periodic: 11.5 / 15.0 -> 5.5 / 7.6.  CTAs of 32 threads: 2 % faster there with
+// one droplet per leaf, 5 to 10 % slower at N = 2,000.
 // (Loading the next node's record before a term is evaluated: 1.39 / 2.22, the loads wait all the same.)
 template <bool PER>
 __device__ __forceinline__ void image64x3(double &dx, double &dy, double &dz, double L, double halfL) {
@@ -518,7 +533,7 @@ __global__ void __launch_bounds__(WALK_T) force_walk_kernel(TreeDev t, double m_
                                                             double *__restrict__ fz) {
     const int N = t.cap, n = t.n;
     const double L = t.L, halfL = 0.5 * t.L;
-    const ForceRec *__restrict__ rec = reinterpret_cast<const ForceRec *>(t.rec_f);
+    const char *const rec = t.rec_f;
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= n) return;
     const int i = t.leaf_idx[slot];
@@ -535,13 +550,13 @@ __global__ void __launch_bounds__(WALK_T) force_walk_kernel(TreeDev t, double m_
             if (k < kend) {
                 const int s = k++;
                 if (s == slot) continue;
-                const double2 qa = t.slot_p[2 * (size_t)s], qb = t.slot_p[2 * (size_t)s + 1];
-                dx = qa.x - xi, dy = qa.y - yi, dz = qb.x - zi;
+                const Half q = half_at(t.slot_p, s);
+                dx = q.a - xi, dy = q.b - yi, dz = q.c - zi;
                 image64x3<PER>(dx, dy, dz, L, halfL);
                 d_sq = dx * dx + dy * dy + dz * dz;
-                const double r_sum = ri + qb.y;
+                const double r_sum = ri + q.d;
                 if (!(d_sq >= r_sum * r_sum)) continue;
-                w = ipow3(qb.y);
+                w = ipow3(q.d);
                 term = true;
                 break;
             }
@@ -550,20 +565,20 @@ __global__ void __launch_bounds__(WALK_T) force_walk_kernel(TreeDev t, double m_
                 node = -1;
                 break;
             }
-            const ForceRec &q = rec[node];
-            const int child = q.child;
+            const Half q = half_at(rec, 2 * node), l = half_at(rec, 2 * node + 1);  // size^2, centre | R^3, links, count
+            const int child = __double2loint(l.b), next = __double2hiint(l.b);
             if (child <= -2) {
                 k = -2 - child;
-                kend = k + q.count;
-                node = q.next;
+                kend = k + __double2loint(l.c);
+                node = next;
                 continue;
             }
-            dx = q.cx - xi, dy = q.cy - yi, dz = q.cz - zi;
+            dx = q.b - xi, dy = q.c - yi, dz = q.d - zi;
             image64x3<PER>(dx, dy, dz, L, halfL);
             d_sq = dx * dx + dy * dy + dz * dz;
-            if (q.s2 < theta_sq * d_sq && d_sq > 0.0) {
-                w = q.r3;
-                node = q.next;
+            if (q.a < theta_sq * d_sq && d_sq > 0.0) {
+                w = l.a;
+                node = next;
                 term = true;
                 break;
             }
@@ -600,8 +615,7 @@ __global__ void __launch_bounds__(WALK_T) velocity_walk_kernel(TreeDev t, const 
                                                                double *__restrict__ vz) {
     const int N = t.cap, n = t.n;
     const double L = t.L, halfL = 0.5 * t.L;
-    const VelRec *__restrict__ rec = reinterpret_cast<const VelRec *>(t.rec_v);
-    const DipRec *__restrict__ dip = reinterpret_cast<const DipRec *>(t.rec_d);
+    const char *const rec = t.rec_v;
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= n) return;
     const int i = t.leaf_idx[slot];
@@ -624,14 +638,14 @@ __global__ void __launch_bounds__(WALK_T) velocity_walk_kernel(TreeDev t, const 
             if (k < kend) {
                 const int s = k++;
                 if (s == slot) continue;
-                const double2 qa = t.slot_p[2 * (size_t)s], qb = t.slot_p[2 * (size_t)s + 1];
-                dx = xi - qa.x, dy = yi - qa.y, dz = zi - qb.x;
+                const Half q = half_at(t.slot_p, s);
+                dx = xi - q.a, dy = yi - q.b, dz = zi - q.c;
                 image64x3<PER>(dx, dy, dz, L, halfL);
                 d_sq = dx * dx + dy * dy + dz * dz;
-                const double r_sum = ri + qb.y;
+                const double r_sum = ri + q.d;
                 if (!(d_sq >= r_sum * r_sum)) continue;
-                const double2 fa = t.slot_f[2 * (size_t)s];
-                Fx = fa.x, Fy = fa.y, Fz = t.slot_f[2 * (size_t)s + 1].x;
+                const Half f = half_at(t.slot_f, s);
+                Fx = f.a, Fy = f.b, Fz = f.c;
                 term = true;
                 break;
             }
@@ -640,21 +654,21 @@ __global__ void __launch_bounds__(WALK_T) velocity_walk_kernel(TreeDev t, const 
                 node = -1;
                 break;
             }
-            const VelRec &q = rec[node];
-            const int child = q.child;
+            const Half q = half_at(rec, 2 * node), l = half_at(rec, 2 * node + 1);  // size^2, centre | links, force
+            const int child = __double2loint(l.a), next = __double2hiint(l.a);
             if (child <= -2) {
                 k = -2 - child;
                 kend = k + t.count[node];
-                node = q.next;
+                node = next;
                 continue;
             }
-            dx = xi - q.cx, dy = yi - q.cy, dz = zi - q.cz;
+            dx = xi - q.b, dy = yi - q.c, dz = zi - q.d;
             image64x3<PER>(dx, dy, dz, L, halfL);
             d_sq = dx * dx + dy * dy + dz * dz;
-            if (q.s2 < theta_sq * d_sq && d_sq > 0.0) {
-                Fx = q.fx, Fy = q.fy, Fz = q.fz;
+            if (q.a < theta_sq * d_sq && d_sq > 0.0) {
+                Fx = l.b, Fy = l.c, Fz = l.d;
                 accepted = node;
-                node = q.next;
+                node = next;
                 term = true;
                 break;
             }
@@ -671,15 +685,17 @@ __global__ void __launch_bounds__(WALK_T) velocity_walk_kernel(TreeDev t, const 
         uz += coeff * (Fz + dz * inv_r2 * dot);
         if (CORR) corr_pair64(corr, dx, dy, dz, Fx, Fy, Fz, ux, uy, uz);
         if (accepted >= 0) {  // dipole correction :1215-1265, R^3-weighted centre (same as get_center)
-            const DipRec D = dip[accepted];
+            const Half d0 = half_at(t.rec_d, 3 * accepted), d1 = half_at(t.rec_d, 3 * accepted + 1),
+                       d2 = half_at(t.rec_d, 3 * accepted + 2);
+            const double D[9] = {d0.a, d0.b, d0.c, d0.d, d1.a, d1.b, d1.c, d1.d, d2.a};
             const double rx = dx, ry = dy, rz = dz;
-            const double Ux = D.d[0] * rx + D.d[3] * ry + D.d[6] * rz;
-            const double Uy = D.d[1] * rx + D.d[4] * ry + D.d[7] * rz;
-            const double Uz = D.d[2] * rx + D.d[5] * ry + D.d[8] * rz;
-            const double wx = D.d[0] * rx + D.d[1] * ry + D.d[2] * rz;
-            const double wy = D.d[3] * rx + D.d[4] * ry + D.d[5] * rz;
-            const double wz = D.d[6] * rx + D.d[7] * ry + D.d[8] * rz;
-            const double s_tr = D.tr;
+            const double Ux = D[0] * rx + D[3] * ry + D[6] * rz;
+            const double Uy = D[1] * rx + D[4] * ry + D[7] * rz;
+            const double Uz = D[2] * rx + D[5] * ry + D[8] * rz;
+            const double wx = D[0] * rx + D[1] * ry + D[2] * rz;
+            const double wy = D[3] * rx + D[4] * ry + D[5] * rz;
+            const double wz = D[6] * rx + D[7] * ry + D[8] * rz;
+            const double s_tr = d2.b;
             const double q = rx * wx + ry * wy + rz * wz;
             const double inv_r3 = inv_r * inv_r2;
             const double inv_r5 = inv_r3 * inv_r2;
