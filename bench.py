@@ -767,9 +767,10 @@ def run_adjoint(args, device):
 
 
 # FP64 operations of vjp_pair_kernel per ordered pair (adds and multiplies 1, FMA 2), counted
-# from its source per unordered pair (each evaluated once): separation and |d|^-1 24, force-term
-# Hessian and radius terms 46, the two Oseen K terms 65, their sum into both sides 15
-FLOPS_VJP_PAIR = 150 / 2
+# from its source per unordered pair (each evaluated once): separation and its unit vector 23,
+# force-term Hessian and radius factors 33, the two Oseen K terms' factors 42, the gradient 39, its
+# sum into both sides 10
+FLOPS_VJP_PAIR = 147 / 2
 FP64_PEAK_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12  # SMs x FP64 lanes x 2 flop x max SM clock
 
 

@@ -84,13 +84,6 @@ __device__ __forceinline__ bool coord_ok(double v) { return v == 0.0 || hi_in(fa
 __device__ __forceinline__ bool factor_ok(double v) { return hi_in(v, hi_of_pow2(-125), hi_of_pow2(125)); }
 
 // ---- pair terms -------------------------------------------------------------
-// Minimum image, as mic64 (:234-240): the subtraction predicated, not selected.
-__device__ __forceinline__ void image1(double &d, double L, double halfL) {
-    asm("{\n\t.reg .pred p;\n\tsetp.gt.f64 p, %1, %2;\n\t@p sub.rn.f64 %0, %0, %3;\n\t}"
-        : "+d"(d)
-        : "d"(fabs(d)), "d"(halfL), "d"(copysign(L, d)));
-}
-
 template <bool PER>
 __device__ __forceinline__ void image3(double &x, double &y, double &z, double L, double halfL) {
     if (PER) {

@@ -29,7 +29,11 @@
 // enters x_i with + and x_j with -, its S = (mu_j - mu_i).f(d) enters r_i as r_j^3 S
 // and r_j as r_i^3 S.  With q = dz^2 / r^2, n = mu_j - mu_i, p = d.n / r^2:
 //   H n   = r^-5 [(15 q - 3) n + ((15 - 105 q) p + 30 dz nz / r^2) d + (30 dz p - 6 nz) z],
-//   n.f   = r^-5 [(5 q - 1) d.n - 2 dz nz].
+//   n.f   = r^-5 [(5 q - 1) d.n - 2 dz nz];
+// with the unit vector e = d / r the powers of r gather in two factors, and the z
+// terms join the coefficients of n and e:
+//   r^5 (H n)_xy = (15 q - 3) n + a e,  r^5 (H n)_z = (15 q - 9) nz + (a + 30 e.n) ez,
+//   a = (15 - 105 q) e.n + 30 ez nz,    r^4 n.f = (5 q - 1) e.n - 2 ez nz.
 #include "common.cuh"
 #include "ieee64.cuh"
 
@@ -46,10 +50,11 @@ namespace dem {
 // (deterministic).  A diagonal pair (I == J) meets every ordered pair and keeps
 // its i side.
 //
-// Bound: the FP64 pipe, ~106 operations per unordered pair, ~39 in the mu pass
-// (before: one thread per droplet and j chunk, every ordered pair).  Mu / pair
-// pass with their sums, periodic, us, before -> now: n = 2,000 40 / 85 -> 30 / 44;
-// 16,384 970 / 3,050 -> 480 / 1,080 (72 % of the pipe's issue rate by that count).
+// Bound: the FP64 pipe, ~102 operations per unordered pair, ~39 in the mu pass
+// (before: one thread per droplet and j chunk, every ordered pair); its three-
+// operand instructions issue at 75 % of its nominal rate, 67 % in the mu pass.
+// Mu / pair pass with their sums, periodic, us, before -> now: n = 2,000 40 / 85 ->
+// 30 / 44; 16,384 970 / 3,050 -> 444 / 1,034.
 // ---------------------------------------------------------------------------
 struct VjpBlocks {
     int nb;           // blocks
@@ -74,7 +79,8 @@ __device__ __forceinline__ void block_pair(const VjpBlocks &b, int &I, int &J) {
 
 template <bool PER>
 __device__ __forceinline__ double image64(double d, double L, double halfL) {
-    return PER ? mic64(d, L, halfL) : d;
+    if (PER) image1(d, L, halfL);
+    return d;
 }
 
 // 1 / sqrt(x) to ~1 ulp: seed y (2^-20), e = 1 - x y^2 and y (1 + e / 2 + 3/8 e^2).
@@ -224,29 +230,27 @@ __global__ void __launch_bounds__(32 * W) vjp_pair_kernel(const VjpArgs a, VjpBl
                              dz = image64<PER>(q[64] - v[k][2], a.L, a.halfL);
                 const double r2 = dx * dx + dy * dy + dz * dz;
                 const double ir = j < n && ii[k] >= 0 && ii[k] != j ? rsqrt64(r2) : 0.0;
-                const double ir2 = ir * ir, ir3 = ir2 * ir, ir5 = ir3 * ir2;
+                const double ex = dx * ir, ey = dy * ir, ez = dz * ir, ir2 = ir * ir;
                 // force terms, inside the contact cut of the forward pass (|d| = r2 / |d|) none
-                const double c5 = r2 * ir > v[k][3] + q[3 * 32] ? ir5 : 0.0;
+                const double c4 = r2 * ir > v[k][3] + q[3 * 32] ? ir2 * ir2 : 0.0;
                 const double nx = q[4 * 32] - v[k][4], ny = q[5 * 32] - v[k][5], nz = q[6 * 32] - v[k][6];
-                const double dn = dx * nx + dy * ny + dz * nz;
-                const double u = dz * ir2, qz = dz * u, p = dn * ir2;
-                const double a0 = fma(15.0, qz, -3.0);
-                const double a1 = fma(30.0 * u, nz, fma(-105.0, qz, 15.0) * p);
-                const double a2 = fma(30.0 * dz, p, -6.0 * nz);
-                const double S = c5 * fma(fma(5.0, qz, -1.0), dn, -2.0 * dz * nz);
-                const double wf = (m3 * wi[k]) * wj * c5;
+                const double en = ex * nx + ey * ny + ez * nz, qz = ez * ez, t = ez * nz;
+                const double a1 = fma(30.0, t, fma(-105.0, qz, 15.0) * en);
+                const double S = c4 * fma(-2.0, t, fma(5.0, qz, -1.0) * en);
+                const double wf = (m3 * wi[k]) * wj * (c4 * ir);
                 // Oseen terms
-                const double dl = dx * lix + dy * liy + dz * liz, ef = dx * fjx + dy * fjy + dz * fjz;
-                const double el = dx * ljx + dy * ljy + dz * ljz, df = dx * fix + dy * fiy + dz * fiz;
+                const double dl = ex * lix + ey * liy + ez * liz, ef = ex * fjx + ey * fjy + ez * fjz;
+                const double el = ex * ljx + ey * ljy + ez * ljz, df = ex * fix + ey * fiy + ez * fiz;
                 const double ab = lix * fjx + liy * fjy + liz * fjz + ljx * fix + ljy * fiy + ljz * fiz;
-                const double cd = fma(-3.0 * ir2, fma(dl, ef, el * df), -ab);
-                const double kf = -a.eta * ir3;
-                const double kx = fma(ef, lix, fma(dl, fjx, fma(df, ljx, fma(el, fix, cd * dx))));
-                const double ky = fma(ef, liy, fma(dl, fjy, fma(df, ljy, fma(el, fiy, cd * dy))));
-                const double kz = fma(ef, liz, fma(dl, fjz, fma(df, ljz, fma(el, fiz, cd * dz))));
-                const double tx = fma(wf, fma(a0, nx, a1 * dx), kf * kx);
-                const double ty = fma(wf, fma(a0, ny, a1 * dy), kf * ky);
-                const double tz = fma(wf, fma(a0, nz, fma(a1, dz, a2)), kf * kz);
+                const double kf = -a.eta * ir2;
+                const double kd = kf * fma(-3.0, fma(dl, ef, el * df), -ab);
+                const double kdl = kf * dl, kef = kf * ef, kel = kf * el, kdf = kf * df;
+                // along n, along e, and the z components of both
+                const double wn = wf * fma(15.0, qz, -3.0), we = fma(wf, a1, kd);
+                const double wnz = wf * fma(15.0, qz, -9.0), wez = fma(wf, fma(30.0, en, a1), kd);
+                const double tx = fma(wn, nx, fma(we, ex, fma(kef, lix, fma(kdl, fjx, fma(kdf, ljx, kel * fix)))));
+                const double ty = fma(wn, ny, fma(we, ey, fma(kef, liy, fma(kdl, fjy, fma(kdf, ljy, kel * fiy)))));
+                const double tz = fma(wnz, nz, fma(wez, ez, fma(kef, liz, fma(kdl, fjz, fma(kdf, ljz, kel * fiz)))));
                 gx[k] += tx;
                 gy[k] += ty;
                 gz[k] += tz;
@@ -293,13 +297,25 @@ __global__ void vjp_sum_kernel(int n, int B, int nb, int row0, int row1, const d
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)NC * n) return;
     const int c = (int)(t / n), i = (int)(t % n), b = i / B, k = i % B;
-    const long long base = pairs_before(nb, row0);
     double v = row0 ? sums[t] : 0.0;
-    for (int I = row0; I < min(b, row1); ++I)  // j side of (I, b)
-        v += records[((size_t)(pairs_before(nb, I) + (b - I) - base) * 2 * NC + NC + c) * B + k];
-    if (b >= row0 && b < row1)  // i side of (b, J)
-        for (int J = b; J < nb; ++J)
-            v += records[((size_t)(pairs_before(nb, b) + (J - b) - base) * 2 * NC + c) * B + k];
+    // 16 loads in flight, added in order
+    auto add = [&](long long item, int I, int end, int step, int less, int side) {
+        const size_t stride = (size_t)2 * NC * B;
+        const double *p = records + (size_t)item * stride + (size_t)(side * NC + c) * B + k;
+        for (; I < end; I += 16) {
+            double w[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                w[q] = I + q < end ? *p : 0.0;
+                if (I + q + 1 < end) p += (size_t)(step - less * (I + q)) * stride;
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (I + q < end) v += w[q];
+        }
+    };
+    add(b - row0, row0, min(b, row1), nb - 1, 1, 1);  // j side of (I, b): the next row's item is nb - I - 1 further
+    if (b >= row0 && b < row1) add(pairs_before(nb, b) - pairs_before(nb, row0), b, nb, 1, 0, 0);  // i side of (b, J)
     sums[t] = v;
 }
 
@@ -339,13 +355,15 @@ struct VjpShape {
 constexpr size_t VJP_RECORD_BYTES = size_t(2) << 30;
 
 // Blocks of 32 droplets fill the SMs with a small box's block pairs, blocks of 64 (two droplets per lane
-// share the loads and shuffles) are faster from n ~ 2,000 on, and one CTA of four warps on a block of 128
-// halves the records of a large n.  Both passes, periodic, us, with 32 / 64 / 128: n = 1,000: 45 / 64 / 70;
-// 2,000: 73 / 70 / 75; 3,000: 114 / 95 / 120; 8,000: 460 / 412 / 430; 16,384: 1,792 / 1,554 / 1,589.
+// share the loads and shuffles) are faster from n ~ 2,000 on, and two such warps on a block of 128, with
+// half the records and reads per pair, once its larger grains leave no last wave.  Both passes, periodic,
+// us, with 32 / 64 / 128: n = 1,000: 45 / 64 / -; 2,000: 73 / 68 / 102; 8,192: - / 407 / 449; 10,000: - / 603 /
+// 609; 11,000: - / 734 / 714; 16,384: 1,792 / 1,529 / 1,470; 40,000: - / 8,689 / 8,578; 65,536: - / 23,247 /
+// 22,738 (four warps of one droplet per lane 9,268 and 24,636, four of two 8,698 and 22,985).
 static VjpShape vjp_shape(int n) {
     VjpShape s;
-    s.warps = n > 32768 ? 4 : 1;
-    s.ipt = n >= 2000 && n <= 32768 ? 2 : 1;
+    s.warps = n > 10500 ? 2 : 1;
+    s.ipt = n >= 2000 ? 2 : 1;
     s.B = 32 * s.warps * s.ipt;
     s.nb = ceil_div(n, s.B);
     const size_t item = sizeof(double) * 8 * s.B;
@@ -380,8 +398,8 @@ static void vjp_pass(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, 
                      cudaStream_t s) {
     for (int row0 = 0; row0 < sh.nb; row0 += sh.rows) {
         const int row1 = min(sh.nb, row0 + sh.rows);
-        if (sh.warps == 4)
-            launch_rows<4, 1>(sh, a, per, pair, row0, row1, records, s);
+        if (sh.warps == 2)
+            launch_rows<2, 2>(sh, a, per, pair, row0, row1, records, s);
         else if (sh.ipt == 2)
             launch_rows<1, 2>(sh, a, per, pair, row0, row1, records, s);
         else

@@ -67,4 +67,11 @@ __device__ __forceinline__ bool hi_in(double v, unsigned lo, unsigned hi) {  // 
 }
 __device__ __forceinline__ bool low_word_ones(double v) { return __double2loint(v) == -1; }
 constexpr DEM_HD unsigned hi_of_pow2(int e) { return (unsigned)(e + 1023) << 20; }
+// Minimum image, as mic64 (direct_droplet_force_calculator.py:234-240): the subtraction predicated, not selected.
+__device__ __forceinline__ void image1(double &d, double L, double halfL) {
+    asm("{\n\t.reg .pred p;\n\tsetp.gt.f64 p, %1, %2;\n\t@p sub.rn.f64 %0, %0, %3;\n\t}"
+        : "+d"(d)
+        : "d"(fabs(d)), "d"(halfL), "d"(copysign(L, d)));
+}
+
 }  // namespace dem

@@ -13,7 +13,7 @@ TOL = 1e-10  # norm-wise; FP64 sums over up to 93,000 terms of both signs
 
 
 @pytest.mark.parametrize("periodic", [True, False])
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1999, 2000, 2001, 4097, 32768, 32769, 93057])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1999, 2000, 2001, 4097, 10500, 10501, 32769, 93057])
 def test_sampled_rows(n, periodic):
     import torch
 
