@@ -73,6 +73,17 @@ __device__ __forceinline__ void decode_item(int q, int nb, int &I, int &J) {
     J = I + (int)(q - rows_before(I, nb));
 }
 
+// A diagonal item is split into parts by its j's (whole runs of 64), each an item of its own: even alone it
+// outlasts the rest of a pass that fits the GPU's 592 resident CTAs.  Force / convection, periodic, us, with
+// 1 / 2 / 4 parts: N = 8,192 121 / 93 / 103 | 90 / 91 / 100; 16,384 322 / 236 / 252 | 277 / 271 / 285; 65,536
+// 2,355 / 2,345 / 2,378 | 2,928 / 2,924 / 2,993.
+constexpr int DIAG_PARTS = 2;
+static_assert(DIAG_PARTS - 1 <= SYM_T / 32, "a record of the j side has a place per warp");
+
+__host__ __device__ __forceinline__ int sorted_slots(const SymBoxes &t, int B) {
+    return t.items_total + (DIAG_PARTS - 1) * (t.npad_total / B);
+}
+
 // Processing order of the sorted pair kernel within a box: the nb diagonal
 // items (I, I) first, then the off-diagonal items (I < J) row by row.  A
 // diagonal item evaluates every ordered pair of a compact block, and most of
@@ -87,13 +98,15 @@ __device__ __forceinline__ void decode_item(int q, int nb, int &I, int &J) {
 // 65,536 2,390 / 2,911 -> 2,341 / 2,894.  In an ensemble the next box's items
 // fill a box's tail, and rows, whose items share block I, are level or 0.5 %
 // faster.
-__device__ __forceinline__ void decode_slot(int s, int nb, bool single, int &I, int &J) {
-    if (s < nb) {
-        I = J = s;
+__device__ __forceinline__ void decode_slot(int s, int nb, bool single, int &I, int &J, int &part) {
+    part = 0;
+    if (s < DIAG_PARTS * nb) {
+        I = J = s / DIAG_PARTS;
+        part = s % DIAG_PARTS;
         return;
     }
     int a, b;
-    decode_item(s - nb, nb - 1, a, b);  // upper triangle without the diagonal: rows a of nb - 1 - a items
+    decode_item(s - DIAG_PARTS * nb, nb - 1, a, b);  // upper triangle without the diagonal: rows a of nb - 1 - a items
     I = single ? b - a : a;             // or diagonals a + 1 of as many
     J = b + 1;
 }
@@ -101,16 +114,17 @@ __device__ __forceinline__ void decode_slot(int s, int nb, bool single, int &I, 
 // The box of work item q: droplet offset o0 and count n, padded offset p0,
 // blocks nbk, side L, scale slots sc; ql = item index within the box.
 struct BoxView {
-    int o0, n, p0, nbk;
+    int o0, n, p0, nbk, q0;
     double L;
     const unsigned long long *sc;
 };
 
+template <int PARTS>
 __device__ __forceinline__ BoxView item_box(const SymBoxes &t, int B, int q, int &ql) {
     BoxView v;
     if (t.nbox == 1) {
         ql = q;
-        v.o0 = 0;
+        v.o0 = v.q0 = 0;
         v.n = t.n1;
         v.p0 = 0;
         v.nbk = t.npad1 / B;
@@ -118,8 +132,17 @@ __device__ __forceinline__ BoxView item_box(const SymBoxes &t, int B, int q, int
         v.sc = t.scales1;
         return v;
     }
-    const int b = box_index(t.ioff, t.nbox, q);
-    ql = q - t.ioff[b];
+    auto first = [&](int b) { return t.ioff[b] + (PARTS > 1 ? (PARTS - 1) * (t.poff[b] / B) : 0); };
+    int b = 0, hi = t.nbox - 1;  // the last box whose first item is not past q
+    while (b < hi) {
+        const int mid = (b + hi + 1) >> 1;
+        if (first(mid) <= q)
+            b = mid;
+        else
+            hi = mid - 1;
+    }
+    ql = q - first(b);
+    v.q0 = t.ioff[b];
     v.o0 = t.off[b];
     v.n = t.off[b + 1] - v.o0;
     v.p0 = t.poff[b];
@@ -173,7 +196,7 @@ __global__ void __launch_bounds__(SYM_T, 4) mixed_sym_kernel(const SymArgs a) {
     // j tile t of item q starts at packed index tile_js(q, t)
     auto tile_js = [&](int q, int t) {
         int ql, I, J;
-        const BoxView v = item_box(a.t, B, q, ql);
+        const BoxView v = item_box<1>(a.t, B, q, ql);
         decode_item(ql, v.nbk, I, J);
         return v.p0 + J * B + t * TJ;
     };
@@ -197,7 +220,7 @@ __global__ void __launch_bounds__(SYM_T, 4) mixed_sym_kernel(const SymArgs a) {
     bool issued = true;   // tid 0: the copy of tile g is in flight
     for (int q = blockIdx.x; q < nitems; q += gridDim.x) {
         int ql, I, J;
-        const BoxView v = item_box(a.t, B, q, ql);
+        const BoxView v = item_box<1>(a.t, B, q, ql);
         decode_item(ql, v.nbk, I, J);
         const bool diag = (I == J);
         const double inv_ell = pow2_inv_of(v.sc[0]);
@@ -906,7 +929,7 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
     __shared__ unsigned s_live;                   // sub-tiles with a droplet (not of the last block's padding only)
     __shared__ int ctot[NCLS], cbase[NCLS];       // entries per class; first entry of a class in the masked run
 
-    const int nitems = a.s.t.items_total;
+    const int nitems = sorted_slots(a.s.t, B);
     if ((int)blockIdx.x >= nitems) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int c = tid; c < NW * 3 * 32; c += SYM_T) (&jnear[0][0][0])[c] = 0.0;
@@ -917,10 +940,10 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
     for (int slot = blockIdx.x; slot < nitems; slot += gridDim.x) {
         // slot: processing order (diagonal items first); q: the item's row-major index, which places its
         // partial sums, so the order changes nothing in the results
-        int sl, I, J;
-        const BoxView v = item_box(a.s.t, B, slot, sl);
-        decode_slot(sl, v.nbk, a.s.t.nbox == 1, I, J);
-        const int q = slot - sl + (int)(rows_before(I, v.nbk) + (J - I));
+        int sl, I, J, part;
+        const BoxView v = item_box<DIAG_PARTS>(a.s.t, B, slot, sl);
+        decode_slot(sl, v.nbk, a.s.t.nbox == 1, I, J, part);
+        const int q = v.q0 + (int)(rows_before(I, v.nbk) + (J - I));
         const bool diag = (I == J);
         const double inv_ell = pow2_inv_of(v.sc[0]);
         const double fscale_inv = FORCE ? 1.0 : pow2_inv_of(v.sc[1]);
@@ -1081,8 +1104,12 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
         const unsigned live_subs = s_live;
         // j-side partials of the item, interleaved per droplet: [j][warp][3] (the reduction adds the warps in order)
         double *PJ = a.s.pj + (size_t)q * NW * 3 * plane + warp * 3;
+        // a diagonal item's sub-tiles are shared out to its parts, whole runs of 64 j each
+        const int runs = (nsub + 1) / 2;
+        const int sub0 = diag ? 2 * (part * runs / DIAG_PARTS) : 0,
+                  sub1 = diag ? min(nsub, 2 * ((part + 1) * runs / DIAG_PARTS)) : nsub;
         {
-            for (int sub = 0; sub < nsub; ++sub) {
+            for (int sub = sub0; sub < sub1; ++sub) {
                 const bool live = (live_subs >> sub) & 1;
                 float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
                 bool had_exact = false;
@@ -1127,7 +1154,7 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
                         d[2] = vz;
                     }
                 }
-                if ((sub & 1) || sub == nsub - 1) {  // fold the FP32 i-side runs every 64 j and at the end
+                if ((sub & 1) || sub == sub1 - 1) {  // fold the FP32 i-side runs every 64 j and at the end
 #pragma unroll
                     for (int kp = 0; kp < KP; ++kp) {
                         two_sum_fold(hx[2 * kp], lx[2 * kp], ax[kp].x);
@@ -1146,14 +1173,18 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
             near_flush<IPT, PER, FORCE>(a, CI, CJ, IP, lane, warp, diag, v, inv_ell, fscale_inv, -1, nq, jnear, PJ,
                                         hx, hy, hz, lx, ly, lz);
         __syncthreads();  // every warp is done with the lists before the next item rebuilds them
-        double *PI = a.s.pi + (size_t)q * 3 * plane;  // interleaved per droplet: [i][3]
+        // interleaved per droplet: [i][3]; part p > 0 of a diagonal item, which has no j side, writes to its record's
+        // place for warp p - 1
+        double *const PI = part == 0 ? a.s.pi + (size_t)q * 3 * plane
+                                     : a.s.pj + (size_t)q * NW * 3 * plane + 3 * (part - 1);
+        const int step = part == 0 ? 3 : 3 * NW;
         const double sg = FORCE ? -1.0 : 1.0;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            const int li = k * SYM_T + tid;
-            PI[3 * li] = sg * ((double)hx[k] + (double)lx[k]);
-            PI[3 * li + 1] = sg * ((double)hy[k] + (double)ly[k]);
-            PI[3 * li + 2] = sg * ((double)hz[k] + (double)lz[k]);
+            double *const P = PI + step * (k * SYM_T + tid);
+            P[0] = sg * ((double)hx[k] + (double)lx[k]);
+            P[1] = sg * ((double)hy[k] + (double)ly[k]);
+            P[2] = sg * ((double)hz[k] + (double)lz[k]);
         }
     }
 }
@@ -1338,6 +1369,16 @@ __global__ void __launch_bounds__(256, DEM_RED_MIN_CTAS) reduce_sym_kernel(const
                     sx += a;
                     sy += b;
                     sz += c;
+                }
+            }
+            // the other parts of item (K, K), in the places of its j side
+            if (!PLANAR && q == 1) {
+                const double *P = pj + ((size_t)(ib + rows_before(K, nbk)) * JW * plane + (size_t)lb * JW) * 3;
+#pragma unroll
+                for (int w = 0; w < DIAG_PARTS - 1; ++w) {
+                    sx += P[3 * w];
+                    sy += P[3 * w + 1];
+                    sz += P[3 * w + 2];
                 }
             }
             // j side: items (q, K), (q + RED_SPLIT, K), ...; item (Ib, K) = rows_before(Ib) + K - Ib; an item
@@ -1626,7 +1667,7 @@ static int run_sym_sorted(dem_ctx *ctx, const SymBoxes &t, int ipt, int ctas, bo
     a.perm = perm;
     a.bounds = bounds;
     a.occ = occ;
-    const int grid = ctas > 0 ? min(ctas, t.items_total) : t.items_total;
+    const int slots = sorted_slots(t, B), grid = ctas > 0 ? min(ctas, slots) : slots;
     dem_prof_begin(ctx, FORCE ? "mixed_force_pass" : "mixed_convection_pass", s);
     if (ipt == 4)
         rc = per ? launch_sorted<4, true, FORCE>(ctx, a, grid, s) : launch_sorted<4, false, FORCE>(ctx, a, grid, s);

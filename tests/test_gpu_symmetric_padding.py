@@ -1,5 +1,5 @@
 """The symmetric mixed passes (csrc/direct_mixed_sym.cu) where a box's last block is nearly all padding, one
-sub-tile (32 entries) or run (64) from it, or whole: against the FP64
+sub-tile (32 entries) or run (64) from it, or whole, with the diagonal items split in two: against the FP64
 passes, with the mixed precision's own bounds, and the same bits in two calls."""
 
 from __future__ import annotations
