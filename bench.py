@@ -1313,7 +1313,7 @@ def report_correction(args, res):
         },
         "roofline": {
             "kernel": "corr_direct_pass",
-            "bound": "l2 (random 96-byte cell gathers from the L2-resident table)",
+            "bound": "l1 lines (random 96-byte cell gathers from the L2-resident table)",
             "achieved": gbs,
             "peak": res["probe_gbs"],
             "unit": "GB/s",

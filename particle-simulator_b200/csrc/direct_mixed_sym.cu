@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(SYM_T, DEM_SORTED_MIN_CTAS) mixed_sym_sorted_k
 
         const int nfs = A_pad >> 5, nms = B_used >> 5, nsub = nfs + nms + (C_pad >> 5);
         // a sub-tile of the last block's padding alone adds zeros: only its run's fold is kept (a step of
-        // 32 boxes of 1,000 to 16,384 droplets: 5.25 -> 5.11 ms)
+        // 32 boxes of 1,024 to 16,384 droplets: 5.25 -> 5.11 ms)
         const unsigned live_subs = s_live;
         // j-side partials of the item, interleaved per droplet: [j][warp][3] (the reduction adds the warps in order)
         double *PJ = a.s.pj + (size_t)q * NW * 3 * plane + warp * 3;
