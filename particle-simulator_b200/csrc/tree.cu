@@ -164,7 +164,10 @@ __global__ void zero_child_cnt_kernel(int32_t *child_cnt, int ls, int le) {
         child_cnt[(size_t)ls * 8 + k] = 0;
 }
 
-// _level_assign_octants :284-306 (octree_node.py:84-95)
+// _level_assign_octants :284-306 (octree_node.py:84-95).  In the first two levels many lanes of a warp fall into one
+// octant and count as one: atomics on 8 or 64 counters took 16 and 24 us at N = 100,003, 4 and 15 now (64 nodes:
+// 15 either way).
+constexpr int FEW_NODES = 8;
 __global__ void assign_octants_kernel(TreeDev t, int n, int ls, int le) {
     const int M = t.max_nodes, N = t.cap;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -178,7 +181,13 @@ __global__ void assign_octants_kernel(TreeDev t, int n, int ls, int le) {
             if (t.p[N + i] >= cy) o |= 2;
             if (t.p[2 * N + i] >= cz) o |= 4;
             t.part_oct[i] = o;
-            atomicAdd(&t.child_cnt[(size_t)node * 8 + o], 1);
+            if (le - ls <= FEW_NODES) {
+                const unsigned peers = __match_any_sync(__activemask(), node * 8 + o);
+                if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0)
+                    atomicAdd(&t.child_cnt[(size_t)node * 8 + o], __popc(peers));
+            } else {
+                atomicAdd(&t.child_cnt[(size_t)node * 8 + o], 1);
+            }
         }
     }
 }
@@ -190,35 +199,37 @@ __global__ void subdivide_flags_kernel(TreeDev t, int ls, int le, int mpl) {
     }
 }
 
-// _level_subdivide_and_alloc :309-354 for the first `sub` candidates
+// _level_subdivide_and_alloc :309-354 for the first `sub` candidates: a thread per child, so that neighbouring
+// lanes fill neighbouring entries of the node arrays (a thread per parent: 152 us over the levels of N = 100,003, one droplet
+// per leaf; 44 now)
 __global__ void subdivide_kernel(TreeDev t, int ls, int le, int sub, int node_count, int parent_count) {
     const int M = t.max_nodes;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < le - ls; k += gridDim.x * blockDim.x) {
+    const long long width = 8LL * (le - ls), stride = (long long)gridDim.x * blockDim.x;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < width; e += stride) {
+        const int k = (int)(e >> 3), o = (int)(e & 7);
         if (!t.flag[k]) continue;
         const int q = t.rank[k];
         if (q >= sub) continue;
         const int node = ls + k;
-        const int base = node_count + 8 * q;
-        t.first_child[node] = base;
-        t.parents[parent_count + q] = node;
-        t.parent_fc[parent_count + q] = base;
-        const double c[3] = {(t.mn[node] + t.mx[node]) * 0.5, (t.mn[M + node] + t.mx[M + node]) * 0.5,
-                             (t.mn[2 * M + node] + t.mx[2 * M + node]) * 0.5};
-        for (int o = 0; o < 8; ++o) {
-            const int child = base + o;
-            for (int a = 0; a < 3; ++a) {
-                const bool up = (o >> a) & 1;
-                t.mn[a * M + child] = up ? c[a] : t.mn[a * M + node];
-                t.mx[a * M + child] = up ? t.mx[a * M + node] : c[a];
-            }
-            t.first_child[child] = -1;  // init_node, octree_node.py:117-154
-            t.next[child] = -1;
-            t.leaf_start[child] = -1;
-            t.count[child] = t.child_cnt[(size_t)node * 8 + o];
-            for (int a = 0; a < 4; ++a) t.R3[a * M + child] = 0.0;
-            t.maxr[child] = 0.0;
-            for (int a = 0; a < 12; ++a) t.fs[a * M + child] = 0.0;
+        const int base = node_count + 8 * q, child = base + o;
+        if (o == 0) {
+            t.first_child[node] = base;
+            t.parents[parent_count + q] = node;
+            t.parent_fc[parent_count + q] = base;
         }
+        for (int a = 0; a < 3; ++a) {
+            const double lo = t.mn[a * M + node], hi = t.mx[a * M + node], c = (lo + hi) * 0.5;
+            const bool up = (o >> a) & 1;
+            t.mn[a * M + child] = up ? c : lo;
+            t.mx[a * M + child] = up ? hi : c;
+        }
+        t.first_child[child] = -1;  // init_node, octree_node.py:117-154
+        t.next[child] = -1;
+        t.leaf_start[child] = -1;
+        t.count[child] = t.child_cnt[(size_t)node * 8 + o];
+        for (int a = 0; a < 4; ++a) t.R3[a * M + child] = 0.0;
+        t.maxr[child] = 0.0;
+        for (int a = 0; a < 12; ++a) t.fs[a * M + child] = 0.0;
     }
 }
 
@@ -387,18 +398,18 @@ __global__ void leaf_forces_kernel(TreeDev t, int nc, const double *__restrict__
     }
 }
 
-// _sweep_forces_level :629-672
+// _sweep_forces_level :629-672: moment blockIdx.y of a parent per thread, children in order (N = 100,003: 103 us for
+// all levels with a thread's twelve sums per parent, 29 now)
 __global__ void sweep_forces_kernel(TreeDev t, int a, int b) {
-    const int M = t.max_nodes;
+    double *const fs = t.fs + (size_t)blockIdx.y * t.max_nodes;
     for (int i = a + blockIdx.x * blockDim.x + threadIdx.x; i < b; i += gridDim.x * blockDim.x) {
-        const int parent = t.parents[i], base = t.parent_fc[i];
-        double acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        const int base = t.parent_fc[i];
+        double acc = 0;
         for (int j = 0; j < 8; ++j) {
             const int c = base + j;
-            if (t.count[c] > 0)
-                for (int u = 0; u < 12; ++u) acc[u] += t.fs[u * M + c];
+            if (t.count[c] > 0) acc += fs[c];
         }
-        for (int u = 0; u < 12; ++u) t.fs[u * M + parent] = acc[u];
+        fs[t.parents[i]] = acc;
     }
 }
 // ---------------------------------------------------------------------------
@@ -913,7 +924,7 @@ int dem_tree_build(dem_tree *t, int n, const double *x, const double *y, const d
         const int sub = total < room ? total : (room > 0 ? room : 0);
         if (sub < total) t->pool_exhausted = 1;
         if (sub > 0) {
-            subdivide_kernel<<<grid_for(ctx, width), 256, 0, counted(s)>>>(view(t), ls, le, sub, t->node_count, t->parent_count);
+            subdivide_kernel<<<grid_for(ctx, 8LL * width), 256, 0, counted(s)>>>(view(t), ls, le, sub, t->node_count, t->parent_count);
             t->node_count += 8 * sub;
             t->parent_count += sub;
         }
@@ -987,7 +998,7 @@ int dem_tree_propagate_forces(dem_tree *t, const double *fx, const double *fy, c
     const int nl = (int)t->level_off.size();
     for (int l = nl - 1; l >= 0; --l) {
         const int a = t->level_off[l], b = l + 1 < nl ? t->level_off[l + 1] : t->parent_count;
-        sweep_forces_kernel<<<grid_for(ctx, b - a), 256, 0, counted(s)>>>(view(t), a, b);
+        sweep_forces_kernel<<<dim3(grid_for(ctx, b - a), 12), 256, 0, counted(s)>>>(view(t), a, b);
     }
     velocity_records(t, s);
     return dem_check_launch(ctx, "tree propagate forces");
