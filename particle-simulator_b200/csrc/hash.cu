@@ -310,8 +310,8 @@ __global__ void write_pairs_kernel(int n, const double *__restrict__ x, const do
 struct SearchParams {
     HashParams hash;   // the reference's cells
     double inv_h;      // search cells per unit length
-    int32_t m;         // search cells per axis of a periodic box; 0: open
-    float r_max;       // rounded up
+    double r_max;
+    int32_t m;         // search cells per axis, cyclic (a periodic box); 0: unbounded; 1: one cell holds everything
 };
 
 // Words of the workspace that a detection zeroes: these, the bucket counts, the row counts.
@@ -329,6 +329,9 @@ static_assert(sizeof(SearchMisc) == 4 * SEARCH_MISC_WORDS, "ctx.cu sizes the wor
 // a cell holds ~0.4 droplets at 2 % volume fraction and ~6 at 30 %; not below half the largest radius (whose
 // droplet then searches at most 10^3 cells) nor above 4.5 of it.  Periodic boxes: whole cells, at most
 // 1,024 per axis (cell_id tells the cells of one search apart).
+// One cell for everything where distance does not decide: cells without a finite size (an infinite radius, whose
+// droplet touches droplets at any distance; L = 0, negative or not finite) and radii below 2^-500 (the contact
+// test's squares underflow: droplets many radii apart pass it).
 __global__ void radius_kernel(int n, const double *__restrict__ r, double L, int periodic, int even_cells,
                               SearchMisc *__restrict__ misc, SearchParams *__restrict__ out) {
     __shared__ bool last;
@@ -363,13 +366,17 @@ __global__ void radius_kernel(int n, const double *__restrict__ r, double L, int
     const double mean = (double)*(volatile float *)&misc->r_sum / n;
     double h = fmax(4.5 * mean, 0.5 * r_max);
     h = h <= 4.5 * r_max ? h : 4.5 * r_max;
-    p.r_max = __double2float_ru(r_max);
+    p.r_max = r_max;
     p.m = 0;
     p.inv_h = 1.0 / h;
     if (periodic) {
         const double cells = floor(L / h);
         p.m = cells >= 1024.0 ? 1024 : cells >= 1.0 ? (int32_t)cells : 1;
         p.inv_h = p.m / L;
+    }
+    if (!(p.inv_h > 0.0 && p.inv_h < INFINITY && r_max >= 0x1p-500)) {
+        p.m = 1;
+        p.inv_h = 0.0;
     }
     *out = p;
 }
@@ -534,11 +541,14 @@ __device__ __forceinline__ bool far_apart(const float4 &q, const float4 &c, bool
 }
 
 // The search cells within `reach` of a coordinate, per axis: first cell and how many (periodic: wrapped, each
-// cell once).  `slack` covers the rounding of v and of the cell coordinates.
+// cell once).  `slack` covers the rounding of v and of the cell coordinates.  A coordinate that is not finite
+// touches nothing (unless a radius is infinite: one cell).
 struct Span {
     int32_t first, len;
 };
 __device__ __forceinline__ Span span_of(double v, double reach, double slack, const SearchParams &p) {
+    if (p.m == 1) return {0, 1};
+    if (!(fabs(v) < INFINITY)) return {0, 0};
     const double wide = reach * (1.0 + 0x1p-18) + slack;
     const int32_t lo = search_floor((v - wide) * p.inv_h), hi = search_floor((v + wide) * p.inv_h);
     const long long len = (long long)hi - lo + 1;
