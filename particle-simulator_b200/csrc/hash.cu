@@ -320,7 +320,7 @@ struct SearchMisc {
     float r_sum;                  // of the positive radii
     unsigned int done;            // CTAs of radius_kernel that have finished
     unsigned int next_slot;       // slots given out to buckets
-    unsigned int found;           // pairs in the list
+    unsigned int found;           // pairs in the list, modulo 2^32 (the scan of the row counts has the pairs' number)
     unsigned int pad[2];
 };
 static_assert(sizeof(SearchMisc) == 4 * SEARCH_MISC_WORDS, "ctx.cu sizes the workspace by this");
@@ -689,8 +689,8 @@ __global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __gri
 
 // The listed pairs into their rows (any order within a row).
 __global__ void place_pairs_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset) {
-    if (!a.sp->hash.valid || a.misc->found > a.list_cap) return;
-    const unsigned k = a.misc->found;
+    if (!a.sp->hash.valid || offset[a.n] > (int64_t)a.list_cap) return;
+    const unsigned k = (unsigned)offset[a.n];
     for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
         const int2 e = a.list[q];
         a.tmp[offset[e.x] + atomicSub(&a.row_count[e.x], 1) - 1] = e;
@@ -710,8 +710,8 @@ __global__ void write_rows_kernel(const __grid_constant__ SearchArgs a, const in
         if (p.hash.valid && offset[a.n] > cap) raise_device_error(err, DEM_DEVERR_PAIR_OVERFLOW);
     }
     if (!p.hash.valid) return;
-    if (a.misc->found <= a.list_cap) {
-        for (int64_t q = tid; q < (int64_t)a.misc->found; q += threads) {
+    if (offset[a.n] <= (int64_t)a.list_cap) {
+        for (int64_t q = tid; q < offset[a.n]; q += threads) {
             const int2 e = a.tmp[q];
             const int64_t o0 = offset[e.x], o1 = offset[e.x + 1];
             int64_t to = o0;

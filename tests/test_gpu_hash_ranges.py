@@ -1,6 +1,6 @@
 """Collision search with radii and positions at the ends of FP64's range: infinite radii, radii above FP32's
 largest and below its smallest number, radii whose squares underflow, positions at infinity among droplets
-that touch.  The oracle's pair sets."""
+that touch (the oracle's pair sets); and more pairs than 32 bits count."""
 
 from __future__ import annotations
 
@@ -61,3 +61,22 @@ def test_pair_set(case, periodic):
     hit, pairs = det.detect(pos, r)
     assert hit == hit_ref
     np.testing.assert_array_equal(pairs, ref)
+
+
+def test_more_than_2_32_pairs():
+    """92,683 coincident droplets have 2^32 + 55,607 pairs: a count modulo 2^32 would fit the list."""
+    import torch
+
+    from dem import _native as N
+
+    n, cap = 92683, 16
+    total = n * (n - 1) // 2
+    ctx = N.Context(n)
+    assert 0 < total - 2**32 < 2 * n + 65536
+    soa = torch.full((3, n), 0.5, dtype=torch.float64, device=ctx.device)
+    r = torch.full((n,), 0.01, dtype=torch.float64, device=ctx.device)
+    pairs = torch.full((cap, 2), -1, dtype=torch.int32, device=ctx.device)
+    counts = torch.zeros(2, dtype=torch.int64, device=ctx.device)
+    ctx.hash_detect(n, soa, r, 1.0, True, 1 << 18, pairs, cap, counts)
+    assert int(counts[0]) == total and ctx.device_errors() & N.DEVERR_PAIR_OVERFLOW
+    np.testing.assert_array_equal(pairs.cpu().numpy(), [[0, j] for j in range(1, cap + 1)])
