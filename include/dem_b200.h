@@ -61,7 +61,9 @@ typedef struct dem_corr dem_corr; /* periodic-image correction grid (dem_corr_cr
  * dem/collision_detector/spatial_hash_collision_detector.py:45-69. */
 DEM_API int dem_ctx_create(int device, int capacity, dem_ctx **out);
 DEM_API void dem_ctx_destroy(dem_ctx *ctx);
-/* Grows the workspace to `capacity` particles (no-op when already large enough). */
+/* Grows the workspace to `capacity` particles (no-op when already large enough).
+ * When an allocation fails the capacity is 0: calls with particles are refused
+ * until a later reserve succeeds. */
 DEM_API int dem_ctx_reserve(dem_ctx *ctx, int capacity);
 DEM_API int dem_ctx_capacity(const dem_ctx *ctx);
 DEM_API const char *dem_last_error(const dem_ctx *ctx);

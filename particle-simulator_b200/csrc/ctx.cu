@@ -38,6 +38,7 @@ int dem_set_error(dem_ctx *ctx, int code, const std::string &msg) {
 
 int dem_check_cuda(dem_ctx *ctx, cudaError_t e, const char *where) {
     if (e == cudaSuccess) return DEM_OK;
+    cudaGetLastError();  // reported here: not again by the next launch's check
     return dem_set_error(ctx, DEM_E_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
@@ -52,6 +53,7 @@ static int grow(dem_ctx *ctx, T **p, size_t count, const char *what) {
 
 int dem_ensure_partials(dem_ctx *ctx, int splits) {
     if (splits <= ctx->partial_splits) return DEM_OK;
+    ctx->partial_splits = 0;  // nothing is held if the allocation fails
     int rc = grow(ctx, &ctx->partial, (size_t)splits * 3 * (size_t)ctx->capacity, "partial sums");
     if (rc) return rc;
     ctx->partial_splits = splits;
@@ -203,6 +205,7 @@ int dem_ctx_reserve(dem_ctx *ctx, int capacity) {
     int rc = dem_check_cuda(ctx, cudaSetDevice(ctx->device), "cudaSetDevice");
     if (rc) return rc;
     const size_t n = (size_t)capacity;
+    ctx->capacity = 0;  // a failure leaves no arrays: every call is refused until a reserve succeeds
     if ((rc = grow(ctx, &ctx->pack_a, n, "workspace"))) return rc;
     if ((rc = grow(ctx, &ctx->pack_b, n, "workspace"))) return rc;
     // the collision search's arrays in one allocation (an allocation costs more than its bytes)
