@@ -351,6 +351,17 @@ struct VjpShape {
     size_t bytes;  // records of one launch and the sums
 };
 
+static size_t record_bytes(const VjpShape &s) {
+    return (size_t)pairs_before(s.nb, s.rows) * sizeof(double) * 8 * s.B;
+}
+
+// Block rows per launch whose records stay below `budget` (at least one).
+static void fit_rows(VjpShape &s, int n, size_t budget) {
+    s.rows = s.nb;
+    while (s.rows > 1 && record_bytes(s) > budget) s.rows = (s.rows + 1) / 2;
+    s.bytes = record_bytes(s) + sizeof(double) * 4 * n;
+}
+
 // Records of a launch stay below this; a larger n goes through its block rows in several launches.
 constexpr size_t VJP_RECORD_BYTES = size_t(2) << 30;
 
@@ -366,10 +377,7 @@ static VjpShape vjp_shape(int n) {
     s.ipt = n >= 2000 ? 2 : 1;
     s.B = 32 * s.warps * s.ipt;
     s.nb = ceil_div(n, s.B);
-    const size_t item = sizeof(double) * 8 * s.B;
-    s.rows = s.nb;
-    while (s.rows > 1 && (size_t)pairs_before(s.nb, s.rows) * item > VJP_RECORD_BYTES) s.rows = (s.rows + 1) / 2;
-    s.bytes = (size_t)pairs_before(s.nb, s.rows) * item + sizeof(double) * 4 * n;
+    fit_rows(s, n, VJP_RECORD_BYTES);
     return s;
 }
 
@@ -419,9 +427,17 @@ int launch_direct_vjp(dem_ctx *ctx, int n, const double *x, const double *y, con
                       double *mx, double *my, double *mz, double *gx, double *gy, double *gz, double *gr,
                       cudaStream_t s) {
     if (n == 0) return DEM_OK;
-    const VjpShape sh = vjp_shape(n);
-    // the context's partial sums, [splits][3][capacity]: the sums, then the records
-    int rc = dem_ensure_partials(ctx, ceil_div((int64_t)(sh.bytes / sizeof(double)), 3LL * ctx->capacity));
+    VjpShape sh = vjp_shape(n);
+    // the context's partial sums, [splits][3][capacity]: the sums, then the records; where the device has no room
+    // for them, fewer block rows per launch (the same sums in the same order)
+    auto ensure = [&] {
+        return dem_ensure_partials(ctx, ceil_div((int64_t)(sh.bytes / sizeof(double)), 3LL * ctx->capacity));
+    };
+    int rc = ensure();
+    while (rc && sh.rows > 1) {
+        fit_rows(sh, n, record_bytes(sh) / 2);
+        rc = ensure();
+    }
     if (rc) return rc;
     double *sums = ctx->partial, *records = sums + 4 * (size_t)n;
     const int egrid = min(ceil_div(n, 256), 8 * ctx->sm_count);

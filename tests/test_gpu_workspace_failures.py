@@ -69,3 +69,33 @@ def test_partial_sums(nearly_full):
     calc.set_tuning(schedule=N.SCHED_SPLIT, j_splits=8)
     for a, b in zip(calc.calculate_forces_and_convection(pos, r), first):
         assert torch.equal(a, b)
+
+
+def test_vjp_records():
+    """Records of 1.1 GB: with room for half of them the same bits, from more and smaller launches."""
+    import torch
+
+    from dem import _native as N
+
+    n, L = 65536, 2e-3
+    g = torch.Generator("cuda").manual_seed(2)
+    kw = dict(dtype=torch.float64, device="cuda", generator=g)
+    pos, F, lam = L * torch.rand((3, n), **kw), torch.randn((3, n), **kw), torch.randn((3, n), **kw)
+    r = 5e-6 * (0.5 + torch.rand(n, **kw))
+
+    def vjp():
+        out = [torch.zeros((3, n), dtype=torch.float64, device="cuda") for _ in range(2)] + [torch.zeros_like(r)]
+        before = N.launch_count()
+        N.Context(n).direct_vjp(n, pos, r, F, lam, 1e-9, 0.7, 1.3, L, True, *out)
+        return out, N.launch_count() - before
+
+    roomy, launches = vjp()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    ballast = torch.empty(free - (700 << 20), dtype=torch.uint8, device="cuda")
+    tight, more = vjp()
+    del ballast
+    torch.cuda.empty_cache()
+    assert more > launches
+    for a, b in zip(tight, roomy):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
