@@ -75,7 +75,7 @@ struct dem_ctx {
     double *dscratch = nullptr;     // 8 doubles: reductions (max radius, ...)
     // collision detection (hash.cu): zeroed words (SEARCH_MISC_WORDS, row counts, bucket counts), per particle
     // (bucket, rank in it, cell id), (first slot, particles) per bucket, FP32 records with (particle, cell id) in
-    // bucket order (2 each), the pair list and its rows (search_list_cap each)
+    // bucket order (2 each), twice search_list_cap pairs: the list's place and, from search_key on, its rows'
     char *search_mem = nullptr;  // the allocation that holds them
     int32_t *search_zero = nullptr;
     int4 *search_key = nullptr;

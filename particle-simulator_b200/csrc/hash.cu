@@ -11,7 +11,7 @@
 // something.  Its pair set is {touching pairs} intersected with {pairs whose
 // bucket the 27 cells reach}; the second condition is a property of two droplets
 // alone, so it is checked for touching pairs only and these are found on a search
-// grid of their own (hashed cells of 4.5 MEAN radii):
+// grid of their own (hashed cells of 4.5 MEAN radii, smaller in dense boxes):
 //   1. maximum and mean radius; the last CTA derives both grids
 //   2. search cell of every droplet, rank in its bucket (atomics)
 //   3. bucket starts (any order: one CTA-wide scan and one atomic per CTA)
@@ -21,15 +21,24 @@
 //      far test, then the reference's contact test in FP64, then the reachability
 //      test: list of pairs, pairs per row, raw hits
 //   6. exclusive scan of the row counts, pairs into their rows, rows sorted by rank
+//      (more pairs than the list holds: found again, straight into the output's rows)
 // A droplet reads ~6 cells and ~2 candidates at 2 % volume fraction.
 // Memory roofline: the chain is bounded by HBM and latency, not arithmetic.  Its
 // algorithmic bytes per detection are 32 N + 8 K (N droplets, K pairs): position and
 // radius read once, 8 B per pair written.  Kernels, periodic, before (27 buckets per
-// droplet) -> now: N = 2^20 765 -> 240 us (the search 580 -> 138, bound by L2
-// latency), N = 2,000 118 -> 55, of which most are gaps between short kernels.
+// droplet) -> now: N = 2^20 769 -> 235 us (the search 580 -> 125, bound by L2
+// latency), N = 2,000 123 -> 54, of which most are gaps between short kernels.
+// Dense boxes are bounded by the tests' instructions.  A whole detection, equal
+// radii, periodic, us, before -> now, N = 100,000: volume fraction 0.3 (1.2 pairs
+// per droplet) 328 -> 222, 0.6 386 -> 239, 2 545 -> 347, 7 1,205 -> 689; N = 400,000:
+// 0.3 730 -> 464, 0.6 864 -> 540, 2 1,225 -> 824, 5 2,098 -> 1,605, and at 27 pairs
+// per droplet, which the list no longer holds, 2,877 -> 3,995.
 // The contact test is the same IEEE expression as the reference's (this file is
 // compiled with -fmad=false) and does not depend on the order of the two droplets,
 // so the pair set is bit-identical to the reference's np.unique output.
+#include <algorithm>
+#include <climits>
+
 #include "common.cuh"
 #include "scan.cuh"
 
@@ -93,6 +102,7 @@ __device__ __forceinline__ int32_t hash_cell(int32_t ix, int32_t iy, int32_t iz,
 }
 
 __device__ __forceinline__ int32_t floor_mod(int32_t a, int32_t m) {
+    if ((uint32_t)a < (uint32_t)m) return a;
     const int32_t q = a % m;
     return q < 0 ? q + m : q;
 }
@@ -325,10 +335,13 @@ struct SearchMisc {
 };
 static_assert(sizeof(SearchMisc) == 4 * SEARCH_MISC_WORDS, "ctx.cu sizes the workspace by this");
 
-// Search cells: 4.5 mean radii, so that a mean droplet's reach (2 r) covers (4 / 4.5 + 1)^3 ~ 6.7 cells, that
-// a cell holds ~0.4 droplets at 2 % volume fraction and ~6 at 30 %; not below half the largest radius (whose
-// droplet then searches at most 10^3 cells) nor above 4.5 of it.  Periodic boxes: whole cells, at most
-// 1,024 per axis (cell_id tells the cells of one search apart).
+// Search cells: 4.5 mean radii, so that a mean droplet's reach (2 r) covers (4 / 4.5 + 1)^3 ~ 6.7 cells and a cell
+// holds ~0.4 droplets at 2 % volume fraction; in dense boxes 1.3 mean distances (2 droplets per cell) down to one
+// mean radius, which leaves fewer candidates outside the reach.  Detection, equal radii, periodic, us, with 4.5
+// mean radii / this: N = 400,000, volume fraction 0.3: 503 / 483, 0.6: 1,241 / 1,033, 2: 3,344 / 2,127; N = 2^20 at
+// 0.02: 369 / 374 (1 or 1.7 mean distances: within 3 %; all before the list could lie in the output).  Not below
+// half the largest radius (whose droplet then searches at most 10^3 cells) nor above 4.5 of it.  Periodic boxes:
+// whole cells, at most 1,024 per axis (cell_id tells the cells of one search apart).
 // One cell for everything where distance does not decide: cells without a finite size (an infinite radius, whose
 // droplet touches droplets at any distance; L = 0, negative or not finite) and radii below 2^-500 (the contact
 // test's squares underflow: droplets many radii apart pass it).
@@ -364,7 +377,7 @@ __global__ void radius_kernel(int n, const double *__restrict__ r, double L, int
     p.hash = hash_params(from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits), L, even_cells);
     const double r_max = from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits);
     const double mean = (double)*(volatile float *)&misc->r_sum / n;
-    double h = fmax(4.5 * mean, 0.5 * r_max);
+    double h = fmax(fmax(fmin(1.3 * L / cbrt((double)n), 4.5 * mean), 1.0 * mean), 0.5 * r_max);
     h = h <= 4.5 * r_max ? h : 4.5 * r_max;
     p.r_max = r_max;
     p.m = 0;
@@ -479,8 +492,11 @@ struct SearchArgs {
     const float4 *rec;   // per slot: (x, y, z, r), (droplet, cell id, -, -)
     SearchMisc *misc;
     int32_t *row_count;
-    int2 *list, *tmp;
+    int32_t *list;       // pairs (i, j) in any order, list_cap of them
     uint32_t list_cap;
+    int2 *tmp;           // the list's pairs in rows: tmp_cap pairs, or (rows' j only) 2 tmp_cap int32
+    uint32_t tmp_cap;
+    int2 *cut;           // the row that the capacity cuts, when the list does not hold all pairs: n pairs
     unsigned long long *raw;
 };
 
@@ -492,18 +508,20 @@ __device__ __noinline__ int reference_hits(const SearchArgs &a, const HashParams
                   cz = cell_coord(a.z[i], p.cell, p.grid, per);
     const int32_t hj = hash_cell(cell_coord(a.x[j], p.cell, p.grid, per), cell_coord(a.y[j], p.cell, p.grid, per),
                                  cell_coord(a.z[j], p.cell, p.grid, per), a.hash_mask);
-    int hits = 0;
-    for (int c = 0; c < 27; ++c) {
-        int32_t nx = cx + c / 9 - 1, ny = cy + (c / 3) % 3 - 1, nz = cz + c % 3 - 1;
-        if (per) {
-            nx = wrap1(nx, p.grid);
-            ny = wrap1(ny, p.grid);
-            nz = wrap1(nz, p.grid);
-        } else if (nx < 0 || ny < 0 || nz < 0 || nx >= p.grid || ny >= p.grid || nz >= p.grid) {
-            continue;
-        }
-        hits += hash_cell(nx, ny, nz, a.hash_mask) == hj;
+    uint32_t hx[3], hy[3], hz[3];  // hash_cell's products of the three neighbours per axis
+    bool in[3][3];                 // inside the grid (a periodic one: always)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        int32_t nx = cx + d - 1, ny = cy + d - 1, nz = cz + d - 1;
+        if (per) nx = wrap1(nx, p.grid), ny = wrap1(ny, p.grid), nz = wrap1(nz, p.grid);
+        hx[d] = (uint32_t)nx * 73856093u, hy[d] = (uint32_t)ny * 19349663u, hz[d] = (uint32_t)nz * 83492791u;
+        in[d][0] = (uint32_t)nx < (uint32_t)p.grid, in[d][1] = (uint32_t)ny < (uint32_t)p.grid, in[d][2] = (uint32_t)nz < (uint32_t)p.grid;
     }
+    int hits = 0;
+#pragma unroll
+    for (int c = 0; c < 27; ++c)
+        hits += in[c / 9][0] && in[c / 3 % 3][1] && in[c % 3][2] &&
+                (int32_t)((hx[c / 9] ^ hy[c / 3 % 3] ^ hz[c % 3]) & (uint32_t)a.hash_mask) == hj;
     return hits;
 }
 
@@ -569,41 +587,45 @@ __device__ __forceinline__ int32_t span_cell(const Span &s, int k, const SearchP
     return p.m && c >= p.m ? c - p.m : c;
 }
 
-// `group` <= 32 droplets (bucket order) per warp.  Their search cells form one list, 32 of which the warp looks up
-// at a time, and the droplets found in them another, of which it tests 32 at a time: a droplet has 1 to 27 cells,
-// rarely thousands, and 0 to a few candidates in each, so loops per lane would mostly wait for the longest
-// lane's loads (436 us at N = 2^20; this form 139).
-constexpr int SP_WARPS = 4;
-__global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __grid_constant__ SearchArgs a, int group) {
-    __shared__ float4 s_q[SP_WARPS][32];                // widened record
-    __shared__ float s_r[SP_WARPS][32];                 // radius
-    __shared__ int s_i[SP_WARPS][32];                   // droplet
-    __shared__ Span s_span[SP_WARPS][3][32];
-    __shared__ int s_first[SP_WARPS][32];               // the droplet's first entry in the list of cells
-    __shared__ int2 s_queue[SP_WARPS][64];              // candidates: slot, (cell id)
-    __shared__ unsigned char s_owner[SP_WARPS][64];     // and whose
-    const SearchParams p = *a.sp;
-    if (!p.hash.valid) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int t = (blockIdx.x * SP_WARPS + w) * group + lane;
+// `group` <= 32 droplets (bucket order, from slot t0 on) per warp.  Their search cells form one list, 32 of which
+// the warp looks up at a time, and the droplets found in them another, of which it tests 32 at a time: a droplet
+// has 1 to 27 cells, rarely thousands, and 0 to a few candidates in each, so loops per lane would mostly wait for
+// the longest lane's loads (436 us at N = 2^20; this form 125).  Pairs that pass the far test queue up in turn, and
+// settle(touching, i, j), i < j, takes 32 of them: the contact test and its caller's reachability test, ~1,500
+// instructions, run with full warps.
+struct SearchWarp {
+    float4 q[32];              // widened record
+    float r[32];               // radius
+    int i[32];                 // droplet
+    Span span[3][32];
+    int first[32];             // the droplet's first entry in the list of cells
+    int2 queue[64];            // candidates: slot, (cell id)
+    unsigned char owner[64];   // and whose
+    int2 near[64];             // pairs to settle
+};
+
+template <typename Settle>
+__device__ __forceinline__ void search_warp(const SearchArgs &a, const SearchParams &p, SearchWarp &sh, int t0, int group,
+                                            Settle &&settle) {
+    const int lane = threadIdx.x & 31, t = t0 + lane;
+    const unsigned lt = (1u << lane) - 1u;
     const float Lf = (float)a.L;
-    unsigned long long raw = 0;
     int cells = 0;
     if (lane < group && t < a.n) {
         const float4 q = a.rec[2 * (size_t)t];
         const int i = __float_as_int(a.rec[2 * (size_t)t + 1].x);
-        s_q[w][lane] = widened(q, a.L);
-        s_r[w][lane] = q.w;
-        s_i[w][lane] = i;
+        sh.q[lane] = widened(q, a.L);
+        sh.r[lane] = q.w;
+        sh.i[lane] = i;
         // The partner's radius is at most this droplet's (by the FP32 order), so 2 r covers the contact
         // distance; where FP32 radii are not normal numbers their order says nothing and r_max bounds it.
         const double reach = q.w > 0x1p-100f && q.w < 0x1p100f ? 2.0 * q.w : a.r[i] + p.r_max;
         if (reach >= 0.0) {  // (a pair of negative radii never touches)
             const Span sx = span_of32(q.x, a.x, i, reach, a.L, p), sy = span_of32(q.y, a.y, i, reach, a.L, p),
                        sz = span_of32(q.z, a.z, i, reach, a.L, p);
-            s_span[w][0][lane] = sx;
-            s_span[w][1][lane] = sy;
-            s_span[w][2][lane] = sz;
+            sh.span[0][lane] = sx;
+            sh.span[1][lane] = sy;
+            sh.span[2][lane] = sz;
             cells = sx.len * sy.len * sz.len;
         }
     }
@@ -614,7 +636,7 @@ __global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __gri
         if (lane >= o) end += v;
     }
     const int total = __shfl_sync(0xffffffffu, end, 31);
-    s_first[w][lane] = end - cells;
+    sh.first[lane] = end - cells;
     __syncwarp();
 
     // Entry e of the list of cells: its owner, its cell's id and bucket.
@@ -623,34 +645,44 @@ __global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __gri
         int lo = 0;
 #pragma unroll
         for (int step = 16; step; step >>= 1)  // the last lane whose first entry is <= e (an empty lane shares the next one's)
-            if (lo + step < 32 && s_first[w][lo + step] <= e) lo += step;
+            if (lo + step < 32 && sh.first[lo + step] <= e) lo += step;
         owner = lo;
-        const Span sx = s_span[w][0][lo], sy = s_span[w][1][lo], sz = s_span[w][2][lo];
-        const int k = e - s_first[w][lo], kxy = k / sz.len;
+        const Span sx = sh.span[0][lo], sy = sh.span[1][lo], sz = sh.span[2][lo];
+        const int k = e - sh.first[lo], kxy = k / sz.len;
         const int32_t cz = span_cell(sz, k - kxy * sz.len, p), kx = kxy / sy.len;
         const int32_t cy = span_cell(sy, kxy - kx * sy.len, p), cx = span_cell(sx, kx, p);
         id = cell_id(cx, cy, cz);
         return a.bucket[search_bucket(cx, cy, cz, a.mask)];
     };
+    int near = 0;
+    auto settle_near = [&](int k) {
+        const int2 e = lane < k ? sh.near[lane] : make_int2(0, 0);
+        settle(lane < k && in_contact(a, e.x, e.y), e.x, e.y);
+    };
     // The first `k` <= 32 queued candidates: the smaller droplets (ties: the smaller index) of their cells.
     auto test = [&](int k) {
+        bool hit = false;
+        int i = 0, j = 0;
         if (lane < k) {
-            const int2 c = s_queue[w][lane];
-            const int o = s_owner[w][lane];
+            const int2 c = sh.queue[lane];
+            const int o = sh.owner[lane];
             const float4 q = a.rec[2 * (size_t)c.x], r = a.rec[2 * (size_t)c.x + 1];
-            const int i = s_i[w][o], j = __float_as_int(r.x);
-            const bool smaller = q.w < s_r[w][o] || (q.w == s_r[w][o] && j < i);
-            if (smaller && __float_as_int(r.y) == c.y && !far_apart(s_q[w][o], q, a.periodic, Lf) &&
-                in_contact(a, i, j)) {
-                const int hits = reference_hits(a, p.hash, min(i, j), max(i, j));
-                if (hits) {
-                    raw += hits;
-                    atomicAdd(&a.row_count[min(i, j)], 1);
-                    const unsigned at = atomicAdd(&a.misc->found, 1u);
-                    if (at < a.list_cap) a.list[at] = make_int2(min(i, j), max(i, j));
-                }
-            }
+            i = sh.i[o];
+            j = __float_as_int(r.x);
+            const bool smaller = q.w < sh.r[o] || (q.w == sh.r[o] && j < i);
+            hit = smaller && __float_as_int(r.y) == c.y && !far_apart(sh.q[o], q, a.periodic, Lf);
         }
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (!hits) return;
+        if (hit) sh.near[near + __popc(hits & lt)] = make_int2(min(i, j), max(i, j));
+        near += __popc(hits);
+        __syncwarp();
+        if (near < 32) return;
+        settle_near(32);
+        near -= 32;
+        const int2 rest = sh.near[32 + lane];
+        __syncwarp();
+        if (lane < near) sh.near[lane] = rest;
         __syncwarp();
     };
     int queued = 0;
@@ -662,20 +694,20 @@ __global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __gri
         for (int k = 0; __any_sync(0xffffffffu, k < b.y); ++k) {
             const unsigned live = __ballot_sync(0xffffffffu, k < b.y);
             if (k < b.y) {
-                const int at = queued + __popc(live & ((1u << lane) - 1u));
-                s_queue[w][at] = make_int2(b.x + k, id);
-                s_owner[w][at] = (unsigned char)owner;
+                const int at = queued + __popc(live & lt);
+                sh.queue[at] = make_int2(b.x + k, id);
+                sh.owner[at] = (unsigned char)owner;
             }
             queued += __popc(live);
             __syncwarp();
             if (queued >= 32) {
                 test(32);
                 queued -= 32;
-                const int2 c = s_queue[w][32 + lane];
-                const unsigned char o = s_owner[w][32 + lane];
+                const int2 c = sh.queue[32 + lane];
+                const unsigned char o = sh.owner[32 + lane];
                 __syncwarp();
-                s_queue[w][lane] = c;
-                s_owner[w][lane] = o;
+                sh.queue[lane] = c;
+                sh.owner[lane] = o;
                 __syncwarp();
             }
         }
@@ -684,84 +716,218 @@ __global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __gri
         id = next_id;
     }
     test(queued);
+    if (near) settle_near(near);
+    __syncwarp();  // the warp's next droplets may take its place
+}
+
+// The pairs into the list (as many as it holds), pairs per row, raw hits.
+constexpr int SP_WARPS = 4;
+__global__ void __launch_bounds__(32 * SP_WARPS) search_pairs_kernel(const __grid_constant__ SearchArgs a, int group) {
+    __shared__ SearchWarp sh[SP_WARPS];
+    const SearchParams p = *a.sp;
+    if (!p.hash.valid) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long raw = 0;
+    search_warp(a, p, sh[w], (blockIdx.x * SP_WARPS + w) * group, group, [&](bool touching, int i, int j) {
+        const int hits = touching ? reference_hits(a, p.hash, i, j) : 0;
+        raw += hits;
+        if (hits) atomicAdd(&a.row_count[i], 1);
+        const unsigned found = __ballot_sync(0xffffffffu, hits > 0);
+        unsigned at = 0;
+        if (lane == 0 && found) at = atomicAdd(&a.misc->found, (unsigned)__popc(found));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(found & ((1u << lane) - 1u));
+        if (hits && at < a.list_cap) {
+            a.list[2 * (size_t)at] = i;
+            a.list[2 * (size_t)at + 1] = j;
+        }
+    });
     if (raw) atomicAdd(a.raw, raw);
 }
 
-// The listed pairs into their rows (any order within a row).
-__global__ void place_pairs_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset) {
-    if (!a.sp->hash.valid || offset[a.n] > (int64_t)a.list_cap) return;
-    const unsigned k = (unsigned)offset[a.n];
-    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
-        const int2 e = a.list[q];
-        a.tmp[offset[e.x] + atomicSub(&a.row_count[e.x], 1) - 1] = e;
+// The row that the capacity cuts (n when it cuts none): some of its pairs lie below `cap`, some above.
+__device__ __forceinline__ int cut_row(const int64_t *__restrict__ offset, int n, int64_t cap) {
+    if (offset[n] <= cap) return n;
+    int lo = 0, hi = n;  // offset[lo] <= cap < offset[hi]
+    while (hi - lo > 1) {
+        const int mid = lo + (hi - lo) / 2;
+        if (offset[mid] <= cap)
+            lo = mid;
+        else
+            hi = mid;
     }
+    return offset[lo] < cap ? lo : n;
 }
 
-// The rows sorted by j: a pair goes to its rank in its row; entries at or past `cap` are dropped, so the
-// buffer holds the lexicographically first cap pairs.  More pairs than the list holds: every droplet i
-// searches its reach r_i + r_max for its row and inserts each j > i into the row's sorted run, the largest
-// dropping out of a row that the capacity cuts.
-__global__ void write_rows_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset, int32_t *__restrict__ pairs,
-                                  int64_t cap, int64_t *__restrict__ counts, uint32_t *err) {
+// The pairs into their rows (any order within a row): those of the list into `tmp`, their j only where `tmp` has no
+// room for pairs.  More pairs than the list holds: they are searched again, straight into the output (j only), and
+// the row that the capacity cuts into `cut`.
+constexpr int PL_WARPS = 8;
+__global__ void __launch_bounds__(32 * PL_WARPS) place_pairs_kernel(const __grid_constant__ SearchArgs a, int group,
+                                                                    const int64_t *__restrict__ offset, int32_t *pairs,
+                                                                    int64_t cap) {
+    __shared__ SearchWarp sh[PL_WARPS];
     const SearchParams p = *a.sp;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
-    if (tid == 0) {
-        counts[0] = p.hash.valid ? offset[a.n] : 0;
-        if (p.hash.valid && offset[a.n] > cap) raise_device_error(err, DEM_DEVERR_PAIR_OVERFLOW);
-    }
     if (!p.hash.valid) return;
-    if (offset[a.n] <= (int64_t)a.list_cap) {
-        for (int64_t q = tid; q < offset[a.n]; q += threads) {
-            const int2 e = a.tmp[q];
-            const int64_t o0 = offset[e.x], o1 = offset[e.x + 1];
-            int64_t to = o0;
-            for (int64_t w = o0; w < o1; ++w) to += a.tmp[w].y < e.y;
-            if (to < cap) {
-                pairs[2 * to] = e.x;
-                pairs[2 * to + 1] = e.y;
-            }
+    const int64_t total = offset[a.n];
+    if (total <= (int64_t)a.list_cap) {
+        int32_t *const tmp_j = reinterpret_cast<int32_t *>(a.tmp);
+        for (int64_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+            const int i = a.list[2 * q], j = a.list[2 * q + 1];
+            const int64_t at = offset[i] + atomicSub(&a.row_count[i], 1) - 1;
+            if (total <= (int64_t)a.tmp_cap)
+                a.tmp[at] = make_int2(i, j);
+            else
+                tmp_j[at] = j;
         }
         return;
     }
-    const float Lf = (float)a.L;
-    for (int t = tid; t < a.n; t += threads) {
-        const float4 q = a.rec[2 * (size_t)t];
-        const int i = __float_as_int(a.rec[2 * (size_t)t + 1].x);
-        const int64_t o0 = offset[i], o1 = offset[i + 1];
-        const int64_t m = (o1 < cap ? o1 : cap) - o0;
-        const double reach = a.r[i] + p.r_max;
-        if (m <= 0 || !(reach >= 0.0)) continue;
-        const float4 qw = widened(q, a.L);
-        const Span sx = span_of32(q.x, a.x, i, reach, a.L, p), sy = span_of32(q.y, a.y, i, reach, a.L, p),
-                   sz = span_of32(q.z, a.z, i, reach, a.L, p);
-        int64_t len = 0;
-        for (int c = 0; c < sx.len * sy.len * sz.len; ++c) {
-            const int cxy = c / sz.len;
-            const int32_t cx = span_cell(sx, cxy / sy.len, p), cy = span_cell(sy, cxy % sy.len, p),
-                          cz = span_cell(sz, c % sz.len, p);
-            const int2 b = a.bucket[search_bucket(cx, cy, cz, a.mask)];
-            const int32_t id = cell_id(cx, cy, cz);
-            for (int s = b.x; s < b.x + b.y; ++s) {
-                const float4 r = a.rec[2 * (size_t)s + 1];
-                const int j = __float_as_int(r.x);
-                if (j <= i || __float_as_int(r.y) != id || far_apart(qw, a.rec[2 * (size_t)s], a.periodic, Lf) ||
-                    !in_contact(a, i, j) || !reference_hits(a, p.hash, i, j))
-                    continue;
-                int64_t at;
-                if (len < m) {
-                    pairs[2 * (o0 + len)] = i;
-                    at = len++;
-                } else {
-                    if (j >= pairs[2 * (o0 + m - 1) + 1]) continue;
-                    at = m - 1;
-                }
-                while (at > 0 && pairs[2 * (o0 + at - 1) + 1] > j) {
-                    pairs[2 * (o0 + at) + 1] = pairs[2 * (o0 + at - 1) + 1];
-                    --at;
-                }
-                pairs[2 * (o0 + at) + 1] = j;
+    const int w = threadIdx.x >> 5, warps = gridDim.x * PL_WARPS;
+    for (int64_t t0 = (int64_t)(blockIdx.x * PL_WARPS + w) * group; t0 < a.n; t0 += (int64_t)warps * group)
+        search_warp(a, p, sh[w], (int)t0, group, [&](bool touching, int i, int j) {
+            if (!touching || offset[i] >= cap || !reference_hits(a, p.hash, i, j)) return;
+            const int64_t o0 = offset[i], at = o0 + atomicSub(&a.row_count[i], 1) - 1;
+            if (offset[i + 1] <= cap)
+                pairs[2 * at + 1] = j;
+            else
+                a.cut[at - o0] = make_int2(i, j);
+        });
+}
+
+// Row i: its j's (STRIDE apart) in ascending order, as pairs, to `to`; STRIDE 2: they are the second entries there.
+// By one thread: up to 8; by a warp: up to 128 from registers, more as a bitonic sort in place whose comparators all
+// put the smaller value first (entries past the end would be the largest: left out).
+constexpr int ROW_THREAD = 8, ROW_REGS = 4;
+template <int STRIDE>
+__device__ __forceinline__ void sort_row_thread(const int32_t *from, int len, int i, int32_t *to) {
+    int v[ROW_THREAD];
+#pragma unroll
+    for (int k = 0; k < ROW_THREAD; ++k) v[k] = k < len ? from[STRIDE * k] : INT_MAX;
+#pragma unroll
+    for (int k = 0; k < ROW_THREAD; ++k) {
+        int rank = 0;
+#pragma unroll
+        for (int q = 0; q < ROW_THREAD; ++q) rank += v[q] < v[k];
+        if (k < len) {
+            to[2 * rank] = i;
+            to[2 * rank + 1] = v[k];
+        }
+    }
+}
+template <int STRIDE>
+__device__ __forceinline__ void sort_row_warp(int32_t *from, int64_t len, int i, int32_t *to, int lane) {
+    if (len <= 32 * ROW_REGS) {
+        int v[ROW_REGS], rank[ROW_REGS];
+#pragma unroll
+        for (int k = 0; k < ROW_REGS; ++k) {
+            v[k] = 32 * k + lane < len ? from[STRIDE * (32 * k + lane)] : INT_MAX;
+            rank[k] = 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < ROW_REGS; ++q) {
+            if (32 * q >= len) break;
+            for (int l = 0; l < 32; ++l) {
+                const int other = __shfl_sync(0xffffffffu, v[q], l);
+#pragma unroll
+                for (int k = 0; k < ROW_REGS; ++k) rank[k] += other < v[k];
             }
         }
+#pragma unroll
+        for (int k = 0; k < ROW_REGS; ++k)
+            if (32 * k + lane < len) {
+                to[2 * rank[k]] = i;
+                to[2 * rank[k] + 1] = v[k];
+            }
+        __syncwarp();
+        return;
+    }
+    auto order = [&](int64_t x, int64_t y) {
+        if (y >= len) return;
+        const int32_t u = from[STRIDE * x], v = from[STRIDE * y];
+        if (u > v) {
+            from[STRIDE * x] = v;
+            from[STRIDE * y] = u;
+        }
+    };
+    for (int64_t size = 2; size < 2 * len; size <<= 1) {
+        const int64_t whole = (len + size - 1) / size * size;
+        for (int64_t t = lane; 2 * t < whole; t += 32) {  // blocks of `size`: ends inwards
+            const int64_t first = 2 * t / size * size, k = t % (size / 2);
+            order(first + k, first + size - 1 - k);
+        }
+        __syncwarp();
+        for (int64_t step = size / 4; step > 0; step >>= 1) {
+            for (int64_t t = lane; 2 * t < whole; t += 32) {
+                const int64_t x = 2 * t - (t & (step - 1));
+                order(x, x + step);
+            }
+            __syncwarp();
+        }
+    }
+    for (int64_t t = lane; t < len; t += 32) {
+        to[2 * t] = i;
+        if (STRIDE == 1) to[2 * t + 1] = from[t];
+    }
+    __syncwarp();
+}
+
+// The rows that end at or before `cap`, from `tmp` (STRIDE 1) or in the output itself.
+template <int STRIDE>
+__device__ __forceinline__ void sort_rows(int n, const int64_t *__restrict__ offset, int32_t *from, int32_t *pairs, int64_t cap) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warps = gridDim.x * blockDim.x >> 5;
+    const int per = min(32, max(1, (n + warps - 1) / warps));  // rows per warp and round
+    for (int64_t i0 = (int64_t)(tid >> 5) * per; i0 < n; i0 += (int64_t)warps * per) {
+        const int64_t i = i0 + lane;
+        int64_t o0 = 0, o1 = 0;
+        if (lane < per && i < n) o0 = offset[i], o1 = offset[i + 1];
+        const int64_t len = o1 <= cap ? o1 - o0 : 0;
+        if (len > 0 && len <= ROW_THREAD) sort_row_thread<STRIDE>(from + STRIDE * o0, (int)len, (int)i, pairs + 2 * o0);
+        for (unsigned m = __ballot_sync(0xffffffffu, len > ROW_THREAD); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const int64_t at = __shfl_sync(0xffffffffu, o0, l);
+            sort_row_warp<STRIDE>(from + STRIDE * at, __shfl_sync(0xffffffffu, len, l), (int)(i0 + l), pairs + 2 * at, lane);
+        }
+    }
+}
+
+// The rows sorted by j; entries at or past `cap` are dropped, so the buffer holds the lexicographically first
+// cap pairs.  Pairs in `tmp` go to their rank in their row, a thread each; else the rows are sorted, and the row
+// that the capacity cuts comes from `cut`.
+__global__ void __launch_bounds__(256) write_rows_kernel(const __grid_constant__ SearchArgs a, const int64_t *__restrict__ offset,
+                                                         int32_t *pairs, int64_t cap, int64_t *__restrict__ counts,
+                                                         uint32_t *err) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    const bool valid = a.sp->hash.valid;
+    const int64_t total = valid ? offset[a.n] : 0;
+    if (tid == 0) {
+        counts[0] = total;
+        if (total > cap) raise_device_error(err, DEM_DEVERR_PAIR_OVERFLOW);
+    }
+    if (!valid) return;
+    // Entry e of a row of `len` entries to its place from `to` on.
+    auto place = [&](const int2 &e, const int2 *row, int64_t len, int64_t to) {
+        for (int64_t w = 0; w < len; ++w) to += row[w].y < e.y;
+        if (to < cap) {
+            pairs[2 * to] = e.x;
+            pairs[2 * to + 1] = e.y;
+        }
+    };
+    const bool listed = total <= (int64_t)a.list_cap;
+    if (listed && total <= (int64_t)a.tmp_cap) {
+        for (int64_t q = tid; q < total; q += threads) {
+            const int2 e = a.tmp[q];
+            const int64_t o0 = offset[e.x];
+            place(e, a.tmp + o0, offset[e.x + 1] - o0, o0);
+        }
+    } else if (listed) {
+        sort_rows<1>(a.n, offset, reinterpret_cast<int32_t *>(a.tmp), pairs, cap);
+    } else {
+        const int cut = cut_row(offset, a.n, cap);
+        if (cut < a.n) {
+            const int64_t len = offset[cut + 1] - offset[cut];
+            for (int64_t q = tid; q < len; q += threads) place(a.cut[q], a.cut, len, offset[cut]);
+        }
+        sort_rows<2>(a.n, offset, pairs + 1, pairs, cap);
     }
 }
 
@@ -820,9 +986,17 @@ int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, co
     a.rec = ctx->search_rec;
     a.misc = misc;
     a.row_count = row_count;
-    a.list = ctx->search_list;
-    a.tmp = ctx->search_list + ctx->search_list_cap;
-    a.list_cap = ctx->search_list_cap;
+    // The list lies in the output where that is the larger place (every listed pair's final place is there, too), else
+    // at the workspace's end.  Its rows take the workspace before it, from the search's own arrays on (no longer
+    // needed when the list holds all pairs).
+    const int64_t list_cap = ctx->search_list_cap;
+    const bool out = cap > list_cap;
+    const int64_t room = (char *)(ctx->search_list + (out ? 2 : 1) * list_cap) - (char *)ctx->search_key;
+    a.list = out ? pairs : reinterpret_cast<int32_t *>(ctx->search_list + list_cap);
+    a.list_cap = (uint32_t)std::min<int64_t>({out ? cap : list_cap, room / 4, INT_MAX});
+    a.tmp = reinterpret_cast<int2 *>(ctx->search_key);
+    a.tmp_cap = (uint32_t)std::min<int64_t>(room / 8, INT_MAX);
+    a.cut = ctx->search_list;
     a.raw = reinterpret_cast<unsigned long long *>(counts + 1);
     // few droplets: fewer per warp, so that ~8 warps per SM share the search (N = 2,000: 14.7 -> 7.6 us with 4)
     int group = 32;
@@ -831,8 +1005,8 @@ int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, co
     if ((rc = dem_check_launch(ctx, "hash search"))) return rc;
     rc = exclusive_scan<int32_t, int64_t>(ctx, row_count, ctx->pair_offset, n, s);
     if (rc) return rc;
-    const int pgrid = max(1, min(ceil_div(n, 256), 2 * ctx->sm_count));
-    place_pairs_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset);
+    const int pgrid = max(1, min(ceil_div(n, group * PL_WARPS), 2 * ctx->sm_count));
+    place_pairs_kernel<<<pgrid, 32 * PL_WARPS, 0, counted(s)>>>(a, group, ctx->pair_offset, pairs, cap);
     write_rows_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset, pairs, cap, counts, ctx->d_err);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "hash write");
