@@ -83,6 +83,21 @@ struct D3 {
 __device__ __forceinline__ bool coord_ok(double v) { return v == 0.0 || hi_in(fabs(v), hi_of_pow2(-300), hi_of_pow2(90)); }
 __device__ __forceinline__ bool factor_ok(double v) { return hi_in(v, hi_of_pow2(-125), hi_of_pow2(125)); }
 
+// Barrier of the CTA's THREADS threads; whether any of them passed a true value.  The producers and the adders
+// reach it from different places, which PTX's barrier allows whole warps, and __syncthreads_or, which wants the
+// whole CTA at one call, does not.
+template <int THREADS>
+__device__ __forceinline__ int cta_any(int v) {
+    int any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.aligned.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"(v), "n"(THREADS)
+        : "memory");
+    return any;
+}
+
 // ---- pair terms -------------------------------------------------------------
 template <bool PER>
 __device__ __forceinline__ void image3(double &x, double &y, double &z, double L, double halfL) {
@@ -280,7 +295,7 @@ __global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>:
                     }
                 }
             }
-            odd = __syncthreads_or(0);
+            odd = cta_any<S::THREADS>(0);
         }
     } else {
         const int q = tid - ORD_P;
@@ -316,7 +331,7 @@ __global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>:
                     if (k < S::TJ) odd |= !put(s + NV * k, v[l], j0 + k < n) && j0 + k < n;
                 }
             }
-            __syncthreads_or(odd);
+            cta_any<S::THREADS>(odd);
         }
         const int i = row0 + row;
         if (chain && i < n) {
