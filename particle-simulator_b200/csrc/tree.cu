@@ -981,7 +981,7 @@ int dem_tree_forces(dem_tree *t, double m_const, double theta_sq, double *fx, do
 // The velocity walk's records from the node force sums.
 static void velocity_records(dem_tree *t, cudaStream_t s) {
     walk_records_kernel<false><<<grid_for(t->ctx, t->node_count), 256, 0, counted(s)>>>(view(t), t->node_count, t->roots + 1);
-    t->vel_records = t->built;
+    t->vel_records = true;
 }
 
 int dem_tree_propagate_forces(dem_tree *t, const double *fx, const double *fy, const double *fz, void *stream) {
@@ -1000,7 +1000,7 @@ int dem_tree_propagate_forces(dem_tree *t, const double *fx, const double *fy, c
         const int a = t->level_off[l], b = l + 1 < nl ? t->level_off[l + 1] : t->parent_count;
         sweep_forces_kernel<<<dim3(grid_for(ctx, b - a), 12), 256, 0, counted(s)>>>(view(t), a, b);
     }
-    velocity_records(t, s);
+    if (t->built) velocity_records(t, s);  // the links of a tree without a build lead anywhere
     return dem_check_launch(ctx, "tree propagate forces");
 }
 
