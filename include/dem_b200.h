@@ -324,6 +324,12 @@ DEM_API int dem_corr_info(const dem_corr *corr, int *n, double *common, double *
  * `stream` to get the table's random-gather bandwidth. */
 DEM_API int dem_corr_gather_probe(const dem_corr *corr, int ctas, int per_thread, float *out, void *stream);
 
+/* The branch-free square root, reciprocals and quotients of the FP64 direct
+ * passes by themselves (no counterpart in the reference; a build is checked with
+ * it): out (device, [4][n]) takes sqrt(a), the passes' reciprocal of that root,
+ * 1 / b and a / b.  Their ranges are csrc/ieee64.cuh's. */
+DEM_API int dem_ieee64_probe(dem_ctx *ctx, int n, const double *a, const double *b, double *out, void *stream);
+
 /* Oseen convection with the periodic-image correction: as
  * dem_direct_convection, plus for every pair j != i the correction of
  * d = MIC(x_i - x_j) (three permuted trilinear lookups contracted with F_j)

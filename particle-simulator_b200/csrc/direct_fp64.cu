@@ -420,4 +420,26 @@ int launch_direct_convection_fp64_corr(dem_ctx *ctx, const dem_corr *c, int n, c
     return dem_check_launch(ctx, "direct_convection_fp64_corr");
 }
 
+// The operations of ieee64.cuh by themselves, as the terms use them.
+__global__ void ieee64_probe_kernel(int n, const double *__restrict__ a, const double *__restrict__ b,
+                                    double *__restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double h;
+        const double g = sqrt_rn(a[i], h), y = rcp_rn(b[i]);
+        out[i] = g;
+        out[(size_t)n + i] = rcp_last(g, rcp_last(g, times_pow2(h, 1)));
+        out[2 * (size_t)n + i] = y;
+        out[3 * (size_t)n + i] = quotient_rn(a[i], b[i], y);
+    }
+}
+
 }  // namespace dem
+
+extern "C" int dem_ieee64_probe(dem_ctx *ctx, int n, const double *a, const double *b, double *out, void *stream) {
+    if (!ctx) return DEM_E_INVALID;
+    if (n < 0 || (n > 0 && (!a || !b || !out))) return dem_set_error(ctx, DEM_E_INVALID, "ieee64 probe arguments");
+    if (n == 0) return DEM_OK;
+    const int grid = min(ceil_div(n, 256), 8 * ctx->sm_count);
+    dem::ieee64_probe_kernel<<<grid, 256, 0, counted((cudaStream_t)stream)>>>(n, a, b, out);
+    return dem_check_launch(ctx, "ieee64 probe");
+}

@@ -10,11 +10,22 @@ namespace dem {
 // operators).  The operators test for such operands each time; without their branches several
 // pairs are in flight per thread, and quotients by one divisor share its reciprocal.
 //
-// Checked against the operators' results on 2e10 operands (random, and with mantissas near 0 and
-// near 1), the quotient also exhaustively in precisions of 5 to 8 bits.  The square root's error before
-// its last rounding is below 2^-102.8 of the result's unit, so only an x whose root lies within
-// 37 x 2^-108 of a midpoint of two doubles could round wrongly; those x = m^2 + k 2^-106 (m odd in units
-// of 2^-53, k = 7 mod 8) were enumerated for |k| <= 513 and agree for every even power of two in range.
+// tests/test_gpu_ieee64.py compares them with the operators on random operands, on mantissas near 1
+// and near 2, and on the square roots and quotients nearest to the midpoints of two doubles.  The square root's error
+// before its last rounding is below 2^-102.8 of the result's unit, so only an x whose root lies within
+// 37 x 2^-108 of a midpoint could round wrongly; those x = m^2 + k 2^-106 (m odd in units of 2^-53, k = 7 mod 8) are
+// enumerated there for |k| <= 513.
+//
+// The quotient (ulp: of a / b; mantissas in [1, 2)).  q = RN(a RN(1 / b)) is up to 1.5 ulp off, where Markstein's
+// theorem asks for 1.  With E = |q - a / b|, the last step's argument is off by at most E m_b / 2 2^-53 for RN(1 / b)
+// and, if E > 2 / m_b, when the residual takes 54 bits, 2^-52 / m_b for its rounding: below 2.5 x 2^-53 in all, so
+// that only an a / b within that of a midpoint could round wrongly.  There E is 1/2 or 3/2 (to 2.5 x 2^-53).
+//   E = 1/2: the residual is exact and the argument off by less than m_b / 4 2^-53 (1 + 2^-50), while a / b is at
+//     least 2^-53 / m_b from any midpoint: too near only if m_b >= 2.
+//   E = 3/2: a RN(1 / b) is 1 ulp - 2.5 x 2^-53 or more from a / b, so that m_a > 2 - 3 x 2^-52 and 1 / b lies
+//     within 0.75 x 2^-53 of its unit of a midpoint.  Such a b has an integer mantissa B < 2^53 that divides
+//     2^106 - 1 or 2^106 + 1: 2^53 - 1 (all ones, left to the operators) and 2^53 - 2^27 + 1, which the test takes
+//     with the mantissas of a in question.
 // Seeds: 2^-20 relative.
 __device__ __forceinline__ double rsqrt_seed(double x) {
     double y;
@@ -56,7 +67,7 @@ __device__ __forceinline__ double rcp_rn(double b) {
     return rcp_last(b, __fma_rn(__fma_rn(e, e, e), y, y));
 }
 
-// RN(a / b) from y = RN(1 / b): a y corrected by its residual (Markstein 1990).
+// RN(a / b) from y = RN(1 / b): a y corrected by its residual (Markstein 1990; above).
 __device__ __forceinline__ double quotient_rn(double a, double b, double y) {
     const double q = a * y;
     return __fma_rn(__fma_rn(-b, q, a), y, q);

@@ -80,6 +80,7 @@ SIGNATURES = {
     "dem_corr_destroy": (None, [_vp]),
     "dem_corr_info": (_i, [_vp, C.POINTER(_i), C.POINTER(_d), C.POINTER(_d)]),
     "dem_corr_gather_probe": (_i, [_vp, _i, _i, _vp, _vp]),
+    "dem_ieee64_probe": (_i, [_vp, _i, _vp, _vp, _vp, _vp]),
     "dem_direct_convection_corr": (_i, [_vp, _vp, _i] + [_vp] * 7 + [_d, _d, _i, _i, _vp, _vp, _vp, _vp]),
     "dem_batch_create": (_i, [_vp, _i, C.POINTER(_i64), C.POINTER(_d), _i, C.POINTER(_vp)]),
     "dem_batch_destroy": (None, [_vp]),
@@ -318,6 +319,11 @@ class Context:
         `done` (torch events that have been recorded before) are recorded after the two."""
         self._check(lib().dem_frame_copy(self.handle, n, *xyz(soa), ptr(aos_dev), ptr(aos_host), self.stream(),
                                          copy_stream.cuda_stream, ready.cuda_event, done.cuda_event), "frame_copy")
+
+    def ieee64_probe(self, a, b, out):
+        """The FP64 passes' square root, its reciprocal, 1 / b and a / b (see dem_ieee64_probe)."""
+        self._check(lib().dem_ieee64_probe(self.handle, a.numel(), ptr(a), ptr(b), ptr(out), self.stream()),
+                    "ieee64_probe")
 
     def direct_forces(self, n, pos, r, m_const, L, periodic, precision, out):
         self._check(
