@@ -34,6 +34,8 @@
 // terms join the coefficients of n and e:
 //   r^5 (H n)_xy = (15 q - 3) n + a e,  r^5 (H n)_z = (15 q - 9) nz + (a + 30 e.n) ez,
 //   a = (15 - 105 q) e.n + 30 ez nz,    r^4 n.f = (5 q - 1) e.n - 2 ez nz.
+#include <cmath>
+
 #include "common.cuh"
 #include "ieee64.cuh"
 
@@ -46,7 +48,7 @@ namespace dem {
 // s, and the j-side sums travel with their droplet (one shuffle per step), so
 // both sides of a pair are added without atomics.  The warps' j-side sums meet
 // in shared memory in warp order; every block pair leaves one record per side,
-// and the finish kernels add a droplet's records in block order
+// and the sum kernel adds a droplet's records in block order
 // (deterministic).  A diagonal pair (I == J) meets every ordered pair and keeps
 // its i side.
 //
@@ -83,7 +85,7 @@ __device__ __forceinline__ double image64(double d, double L, double halfL) {
     return d;
 }
 
-// 1 / sqrt(x) to ~1 ulp: seed y (2^-20), e = 1 - x y^2 and y (1 + e / 2 + 3/8 e^2).
+// 1 / sqrt(x) to ~1 ulp: seed y (2^-20), e = 1 - x y^2 and y (1 + e / 2 + 3/8 e^2).  x below infinity.
 __device__ __forceinline__ double rsqrt64(double x) {
     const double y = rsqrt_seed(x);
     const double e = fma(-(x * y), y, 1.0);
@@ -177,7 +179,7 @@ struct VjpArgs {
     const double *x, *y, *z, *r;
     const double *fx, *fy, *fz;  // forces at this state
     const double *lx, *ly, *lz;  // lambda: cotangent on u
-    const double *mx, *my, *mz;  // mu: cotangent on F
+    double *mx, *my, *mz;        // mu: cotangent on F
     double m_const, eta, stokes, L, halfL;
     double *gx, *gy, *gz, *gr;
 };
@@ -290,10 +292,29 @@ __global__ void __launch_bounds__(32 * W) vjp_pair_kernel(const VjpArgs a, VjpBl
     }
 }
 
-// sums[c][i] (+)= droplet i's records of block rows [row0, row1), in block order.
+// What the block pairs read for the droplets' own arrays: finite coordinates no farther out than that a squared
+// distance stays finite (the terms of a pair so far apart are below 2^-500 of any other's), and radii whose cube does:
+// the zero factor of a cut pair must not meet an infinity.
+__global__ void vjp_admit_kernel(const VjpArgs a, double *__restrict__ adm) {
+    const int n = a.n;
+    const double *const src[3] = {a.x, a.y, a.z};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double v = src[c][i];
+            adm[c * (size_t)n + i] = fabs(v) < INFINITY ? fmin(fmax(v, -0x1p510), 0x1p510) : v;
+        }
+        adm[3 * (size_t)n + i] = fmin(a.r[i], 0x1p341);
+    }
+}
+
+// sums[c][i] (+)= droplet i's records of block rows [row0, row1), in block order; the last rows' launch writes the
+// results: mu_i = eta sum_i + lambda_i / (gamma r_i), for the pair pass in mu_pairs (zeros where r_i, not a number, cuts
+// every pair), or the gradients.
 template <int NC>
-__global__ void vjp_sum_kernel(int n, int B, int nb, int row0, int row1, const double *__restrict__ records,
-                               double *__restrict__ sums) {
+__global__ void vjp_sum_kernel(const VjpArgs a, int B, int nb, int row0, int row1, const double *__restrict__ records,
+                               double *__restrict__ sums, double *__restrict__ mu_pairs) {
+    const int n = a.n;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)NC * n) return;
     const int c = (int)(t / n), i = (int)(t % n), b = i / B, k = i % B;
@@ -316,39 +337,30 @@ __global__ void vjp_sum_kernel(int n, int B, int nb, int row0, int row1, const d
     };
     add(b - row0, row0, min(b, row1), nb - 1, 1, 1);  // j side of (I, b): the next row's item is nb - I - 1 further
     if (b >= row0 && b < row1) add(pairs_before(nb, b) - pairs_before(nb, row0), b, nb, 1, 0, 0);  // i side of (b, J)
-    sums[t] = v;
-}
-
-// mu_i = eta sum_i + lambda_i / (gamma r_i)
-__global__ void vjp_mu_kernel(int n, const double *__restrict__ sums, const double *__restrict__ r,
-                              const double *__restrict__ lx, const double *__restrict__ ly,
-                              const double *__restrict__ lz, double eta, double stokes, double *__restrict__ mx,
-                              double *__restrict__ my, double *__restrict__ mz) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double a = 1.0 / (stokes * r[i]);
-        mx[i] = eta * sums[i] + a * lx[i];
-        my[i] = eta * sums[n + i] + a * ly[i];
-        mz[i] = eta * sums[2 * (size_t)n + i] + a * lz[i];
+    if (row1 < nb) {
+        sums[t] = v;
+        return;
     }
-}
-
-// The gradients from the sums.
-__global__ void vjp_finish_kernel(const VjpArgs a, const double *__restrict__ sums) {
-    const int n = a.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double ri = a.r[i];
-        a.gx[i] = sums[i];
-        a.gy[i] = sums[n + i];
-        a.gz[i] = sums[2 * (size_t)n + i];
+    const double ri = a.r[i];
+    if (NC == 3) {
+        const double w = 1.0 / (a.stokes * ri);
+        const double mu = a.eta * v + w * (c == 0 ? a.lx : c == 1 ? a.ly : a.lz)[i];
+        (c == 0 ? a.mx : c == 1 ? a.my : a.mz)[i] = mu;
+        mu_pairs[t] = ri == ri ? mu : 0.0;
+    } else if (c < 3) {
+        (c == 0 ? a.gx : c == 1 ? a.gy : a.gz)[i] = v;
+    } else {
         const double lf = a.lx[i] * a.fx[i] + a.ly[i] * a.fy[i] + a.lz[i] * a.fz[i];
-        a.gr[i] = -3.0 * a.m_const * ri * ri * sums[3 * (size_t)n + i] - lf / (a.stokes * ri * ri);
+        a.gr[i] = -3.0 * a.m_const * ri * ri * v - lf / (a.stokes * ri * ri);
     }
 }
+
+constexpr int VJP_OWN = 11;  // workspace doubles per droplet: sums (4), admitted x, y, z, r, and mu
 
 struct VjpShape {
     int warps, ipt, B, nb;
     int rows;      // block rows per launch
-    size_t bytes;  // records of one launch and the sums
+    size_t bytes;  // records of one launch, the sums and what the pairs read
 };
 
 static size_t record_bytes(const VjpShape &s) {
@@ -359,7 +371,7 @@ static size_t record_bytes(const VjpShape &s) {
 static void fit_rows(VjpShape &s, int n, size_t budget) {
     s.rows = s.nb;
     while (s.rows > 1 && record_bytes(s) > budget) s.rows = (s.rows + 1) / 2;
-    s.bytes = record_bytes(s) + sizeof(double) * 4 * n;
+    s.bytes = record_bytes(s) + sizeof(double) * VJP_OWN * n;
 }
 
 // Records of a launch stay below this; a larger n goes through its block rows in several launches.
@@ -382,10 +394,10 @@ static VjpShape vjp_shape(int n) {
 }
 
 template <int W, int IPT>
-static void launch_rows(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, int row0, int row1, double *records,
+static void launch_rows(int nb, const VjpArgs &a, bool per, bool pair, int row0, int row1, double *records,
                         cudaStream_t s) {
-    const VjpBlocks b{sh.nb, row0, pairs_before(sh.nb, row0)};
-    const unsigned grid = (unsigned)(pairs_before(sh.nb, row1) - b.item0);
+    const VjpBlocks b{nb, row0, pairs_before(nb, row0)};
+    const unsigned grid = (unsigned)(pairs_before(nb, row1) - b.item0);
     if (pair) {
         if (per)
             vjp_pair_kernel<W, IPT, true><<<grid, 32 * W, 0, counted(s)>>>(a, b, records);
@@ -401,23 +413,28 @@ static void launch_rows(const VjpShape &sh, const VjpArgs &a, bool per, bool pai
     }
 }
 
-// One O(N^2) pass (mu or pair terms) into sums[3 or 4][n].
-static void vjp_pass(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, double *records, double *sums,
+// One O(N^2) pass: mu (into a.mx, ... and own + 8 n) or the pair terms (into the gradients).  a: the caller's arrays.
+static void vjp_pass(const VjpShape &sh, const VjpArgs &a, bool per, bool pair, double *records, double *own,
                      cudaStream_t s) {
+    const size_t n = (size_t)a.n;
+    double *const sums = own, *const adm = own + 4 * n, *const mu = own + 8 * n;
+    VjpArgs p = a;  // as the pairs read them
+    p.x = adm, p.y = adm + n, p.z = adm + 2 * n, p.r = adm + 3 * n;
+    p.mx = mu, p.my = mu + n, p.mz = mu + 2 * n;
     for (int row0 = 0; row0 < sh.nb; row0 += sh.rows) {
         const int row1 = min(sh.nb, row0 + sh.rows);
         if (sh.warps == 2)
-            launch_rows<2, 2>(sh, a, per, pair, row0, row1, records, s);
+            launch_rows<2, 2>(sh.nb, p, per, pair, row0, row1, records, s);
         else if (sh.ipt == 2)
-            launch_rows<1, 2>(sh, a, per, pair, row0, row1, records, s);
+            launch_rows<1, 2>(sh.nb, p, per, pair, row0, row1, records, s);
         else
-            launch_rows<1, 1>(sh, a, per, pair, row0, row1, records, s);
+            launch_rows<1, 1>(sh.nb, p, per, pair, row0, row1, records, s);
         if (pair)
-            vjp_sum_kernel<4><<<ceil_div(4LL * a.n, 128), 128, 0, counted(s)>>>(a.n, sh.B, sh.nb, row0, row1, records,
-                                                                               sums);
+            vjp_sum_kernel<4><<<ceil_div(4LL * a.n, 128), 128, 0, counted(s)>>>(a, sh.B, sh.nb, row0, row1, records, sums,
+                                                                               nullptr);
         else
-            vjp_sum_kernel<3><<<ceil_div(3LL * a.n, 128), 128, 0, counted(s)>>>(a.n, sh.B, sh.nb, row0, row1, records,
-                                                                               sums);
+            vjp_sum_kernel<3><<<ceil_div(3LL * a.n, 128), 128, 0, counted(s)>>>(a, sh.B, sh.nb, row0, row1, records, sums,
+                                                                               mu);
     }
 }
 
@@ -428,8 +445,8 @@ int launch_direct_vjp(dem_ctx *ctx, int n, const double *x, const double *y, con
                       cudaStream_t s) {
     if (n == 0) return DEM_OK;
     VjpShape sh = vjp_shape(n);
-    // the context's partial sums, [splits][3][capacity]: the sums, then the records; where the device has no room
-    // for them, fewer block rows per launch (the same sums in the same order)
+    // the context's partial sums, [splits][3][capacity]: the droplets' own, then the records; where the device has no
+    // room for them, fewer block rows per launch (the same sums in the same order)
     auto ensure = [&] {
         return dem_ensure_partials(ctx, ceil_div((int64_t)(sh.bytes / sizeof(double)), 3LL * ctx->capacity));
     };
@@ -439,17 +456,15 @@ int launch_direct_vjp(dem_ctx *ctx, int n, const double *x, const double *y, con
         rc = ensure();
     }
     if (rc) return rc;
-    double *sums = ctx->partial, *records = sums + 4 * (size_t)n;
-    const int egrid = min(ceil_div(n, 256), 8 * ctx->sm_count);
+    double *own = ctx->partial, *records = own + VJP_OWN * (size_t)n;
     const VjpArgs a{n, x, y, z, r, fx, fy, fz, lx, ly, lz, mx, my, mz, m_const, eta, stokes, L, 0.5 * L, gx, gy, gz, gr};
     dem_prof_begin(ctx, "vjp_mu_pass", s);
-    vjp_pass(sh, a, periodic != 0, false, records, sums, s);
-    vjp_mu_kernel<<<egrid, 256, 0, counted(s)>>>(n, sums, r, lx, ly, lz, eta, stokes, mx, my, mz);
+    vjp_admit_kernel<<<min(ceil_div(n, 256), 8 * ctx->sm_count), 256, 0, counted(s)>>>(a, own + 4 * (size_t)n);
+    vjp_pass(sh, a, periodic != 0, false, records, own, s);
     dem_prof_end(ctx, s);
     if ((rc = dem_check_launch(ctx, "vjp mu"))) return rc;
     dem_prof_begin(ctx, "vjp_pass", s);
-    vjp_pass(sh, a, periodic != 0, true, records, sums, s);
-    vjp_finish_kernel<<<egrid, 256, 0, counted(s)>>>(a, sums);
+    vjp_pass(sh, a, periodic != 0, true, records, own, s);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "vjp pair pass");
 }
