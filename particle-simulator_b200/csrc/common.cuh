@@ -72,6 +72,7 @@ struct dem_ctx {
         int threads = 0;
         int ctas[2][2][4] = {};
     } split_occ;
+    unsigned ord_smem_set = 0;      // FP64 passes: kernels whose shared-memory limit this context has raised
     double *dscratch = nullptr;     // 8 doubles: reductions (max radius, ...)
     // collision detection (hash.cu): zeroed words (SEARCH_MISC_WORDS, row counts, bucket counts), per particle
     // (bucket, rank in it, cell id), (first slot, particles) per bucket, FP32 records with (particle, cell id) in

@@ -26,7 +26,6 @@ extern "C" void dem_count_replayed_launches(unsigned long long k) { dem_count_la
 
 namespace dem {
 int sym_sorted_prepare(dem_ctx *ctx);
-int direct_fp64_prepare(dem_ctx *ctx);
 int direct_plan(dem_ctx *ctx, int n, int periodic, int *schedule, int *i_per_thread, int *threads,
                 long long *ctas, int *j_splits);
 }
@@ -249,14 +248,13 @@ int dem_ctx_create(int device, int capacity, dem_ctx **out) {
     if (!rc) rc = dem_check_cuda(ctx, cudaMalloc((void **)&ctx->merged_cnt, 4 * sizeof(int32_t)), "scratch");
     if (!rc) rc = dem_ctx_reserve(ctx, capacity);
     // scan block sums (fixed size) and the sorted pair kernels' shared-memory limit, set up front so
-    // that no later call allocates or changes a kernel attribute (calls may run under stream capture)
+    // that no later call needs them (calls may run under stream capture)
     if (!rc) {
         const size_t need = sizeof(int64_t) * (dem::SCAN_MAX_BLOCKS + 1);
         rc = dem_check_cuda(ctx, cudaMalloc(&ctx->scan_tmp, need), "scan workspace");
         if (!rc) ctx->scan_tmp_bytes = need;
     }
     if (!rc) rc = dem::sym_sorted_prepare(ctx);
-    if (!rc) rc = dem::direct_fp64_prepare(ctx);
     if (rc) {
         fprintf(stderr, "dem_ctx_create: %s\n", ctx->last_error.c_str());
         dem_ctx_destroy(ctx);

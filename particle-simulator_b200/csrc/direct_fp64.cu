@@ -42,9 +42,6 @@
 
 namespace dem {
 
-#ifndef ORD_UNROLL
-#define ORD_UNROLL 4
-#endif
 enum : int { FORCE64 = 0, OSEEN64 = 1, OSEEN64_CORR = 2 };
 
 constexpr int ORD_P = 256;  // producer threads
@@ -57,7 +54,7 @@ struct OrdShape {
     static constexpr int TJ = SUBS * U;                          // j's per tile
     static constexpr int ADD_T = (3 * R + 31) / 32 * 32;         // adder threads: one per (row, component)
     static constexpr int THREADS = ORD_P + ADD_T;
-    static constexpr int CTAS = KIND == OSEEN64_CORR ? 2 : 3;    // per SM: 64 - 72 registers (the correction: 112)
+    static constexpr int CTAS = KIND == OSEEN64_CORR ? 2 : 3;    // per SM: 64 - 72 registers (the correction: 96)
     static constexpr int PLANES = KIND == OSEEN64_CORR ? 6 : 3;  // terms per pair
     static constexpr int CS = TJ * R + (R < 16 ? R : 0);         // plane stride (narrow rows: offset banks)
     static constexpr int LOADS = (TJ + ADD_T - 1) / ADD_T;       // staged j's per adder thread
@@ -341,35 +338,22 @@ __global__ void __launch_bounds__(OrdShape<R, KIND>::THREADS, OrdShape<R, KIND>:
     }
 }
 
+// Launches the pass; a shape that wants more than 48 KB of shared memory (8 rows and more, or the correction) has
+// its kernel's limit raised by the context's first call that takes it.  (Raised for all of them when a context was
+// created, the driver loaded 18 kernels: 1.6 ms of a process's first context.)
 template <int R, bool PER, int KIND>
-static void launch_ordered(const Ord64Args &a, cudaStream_t s) {
+static int launch_ordered(dem_ctx *ctx, const Ord64Args &a, cudaStream_t s) {
     using S = OrdShape<R, KIND>;
+    constexpr unsigned bit = 1u << ((R == 4 ? 0 : R == 8 ? 1 : 2) + 3 * (KIND + 3 * PER));
+    if (S::SMEM > 48 * 1024 && !(ctx->ord_smem_set & bit)) {
+        const int rc = dem_check_cuda(ctx, cudaFuncSetAttribute(ordered_pass_kernel<R, PER, KIND>,
+                                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM),
+                                      "direct_fp64 attributes");
+        if (rc) return rc;
+        ctx->ord_smem_set |= bit;
+    }
     ordered_pass_kernel<R, PER, KIND><<<ceil_div(a.n, R), S::THREADS, S::SMEM, counted(s)>>>(a);
-}
-
-template <int R, int KIND>
-static cudaError_t allow_smem() {
-    cudaError_t e = cudaFuncSetAttribute(ordered_pass_kernel<R, true, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)OrdShape<R, KIND>::SMEM);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(ordered_pass_kernel<R, false, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)OrdShape<R, KIND>::SMEM);
-}
-
-template <int KIND>
-static cudaError_t allow_smem_all() {
-    cudaError_t e = allow_smem<4, KIND>();
-    if (e == cudaSuccess) e = allow_smem<8, KIND>();
-    if (e == cudaSuccess) e = allow_smem<16, KIND>();
-    return e;
-}
-
-// Shared-memory limits of the ordered passes, set at context creation (a pass may run under capture).
-int direct_fp64_prepare(dem_ctx *ctx) {
-    cudaError_t e = allow_smem_all<FORCE64>();
-    if (e == cudaSuccess) e = allow_smem_all<OSEEN64>();
-    if (e == cudaSuccess) e = allow_smem_all<OSEEN64_CORR>();
-    return dem_check_cuda(ctx, e, "direct_fp64 attributes");
+    return DEM_OK;
 }
 
 // Rows per CTA.  Few rows per CTA spread a small box over the SMs (one wave: 3 CTAs of 4 rows per SM hold
@@ -378,35 +362,35 @@ int direct_fp64_prepare(dem_ctx *ctx) {
 // 1,215 / 1,240; 13,000: 2,526 / 1,891 / 1,921; 16,000: 3,871 / 2,910 / 2,716; 30,000: 12,998 / 9,951 / 9,246
 // (32 rows are slower throughout).  With the correction, bound by its gathers, 4 and 8 rows are as fast
 // as 16 or faster from n = 4,097 to 16,384.
-template <int KIND>
-static void run_ordered(const dem_ctx *ctx, const Ord64Args &a, int periodic, cudaStream_t s) {
+template <bool PER, int KIND>
+static int run_rows(dem_ctx *ctx, const Ord64Args &a, cudaStream_t s) {
     const int sm = ctx->sm_count;
-    if (a.n <= 12 * sm)
-        periodic ? launch_ordered<4, true, KIND>(a, s) : launch_ordered<4, false, KIND>(a, s);
-    else if (KIND == OSEEN64_CORR || a.n <= 95 * sm)
-        periodic ? launch_ordered<8, true, KIND>(a, s) : launch_ordered<8, false, KIND>(a, s);
-    else
-        periodic ? launch_ordered<16, true, KIND>(a, s) : launch_ordered<16, false, KIND>(a, s);
+    if (a.n <= 12 * sm) return launch_ordered<4, PER, KIND>(ctx, a, s);
+    if constexpr (KIND != OSEEN64_CORR)
+        if (a.n > 95 * sm) return launch_ordered<16, PER, KIND>(ctx, a, s);
+    return launch_ordered<8, PER, KIND>(ctx, a, s);
+}
+
+template <int KIND>
+static int run_ordered(dem_ctx *ctx, const char *name, const Ord64Args &a, int periodic, cudaStream_t s) {
+    dem_prof_begin(ctx, name, s);
+    const int rc = periodic ? run_rows<true, KIND>(ctx, a, s) : run_rows<false, KIND>(ctx, a, s);
+    dem_prof_end(ctx, s);
+    return rc ? rc : dem_check_launch(ctx, name);
 }
 
 int launch_direct_forces_fp64(dem_ctx *ctx, int n, const double *x, const double *y, const double *z,
                               const double *r, double m_const, double L, int periodic, double *fx, double *fy,
                               double *fz, cudaStream_t s) {
     const Ord64Args a{n, x, y, z, r, nullptr, nullptr, nullptr, m_const, L, L * 0.5, CorrDev{}, fx, fy, fz};
-    dem_prof_begin(ctx, "fp64_force_pass", s);
-    run_ordered<FORCE64>(ctx, a, periodic, s);
-    dem_prof_end(ctx, s);
-    return dem_check_launch(ctx, "direct_force_fp64");
+    return run_ordered<FORCE64>(ctx, "fp64_force_pass", a, periodic, s);
 }
 
 int launch_direct_convection_fp64(dem_ctx *ctx, int n, const double *x, const double *y, const double *z,
                                   const double *fx, const double *fy, const double *fz, double eta, double L,
                                   int periodic, double *vx, double *vy, double *vz, cudaStream_t s) {
     const Ord64Args a{n, x, y, z, nullptr, fx, fy, fz, eta, L, L * 0.5, CorrDev{}, vx, vy, vz};
-    dem_prof_begin(ctx, "fp64_convection_pass", s);
-    run_ordered<OSEEN64>(ctx, a, periodic, s);
-    dem_prof_end(ctx, s);
-    return dem_check_launch(ctx, "direct_convection_fp64");
+    return run_ordered<OSEEN64>(ctx, "fp64_convection_pass", a, periodic, s);
 }
 
 int launch_direct_convection_fp64_corr(dem_ctx *ctx, const dem_corr *c, int n, const double *x, const double *y,
@@ -414,10 +398,7 @@ int launch_direct_convection_fp64_corr(dem_ctx *ctx, const dem_corr *c, int n, c
                                        double eta, double L, int periodic, double *vx, double *vy, double *vz,
                                        cudaStream_t s) {
     const Ord64Args a{n, x, y, z, nullptr, fx, fy, fz, eta, L, L * 0.5, corr_view(c), vx, vy, vz};
-    dem_prof_begin(ctx, "fp64_convection_corr_pass", s);
-    run_ordered<OSEEN64_CORR>(ctx, a, periodic, s);
-    dem_prof_end(ctx, s);
-    return dem_check_launch(ctx, "direct_convection_fp64_corr");
+    return run_ordered<OSEEN64_CORR>(ctx, "fp64_convection_corr_pass", a, periodic, s);
 }
 
 // The operations of ieee64.cuh by themselves, as the terms use them.
