@@ -412,6 +412,7 @@ __global__ void sweep_forces_kernel(TreeDev t, int a, int b) {
         fs[t.parents[i]] = acc;
     }
 }
+
 // ---------------------------------------------------------------------------
 // Walk records.  A walk visits a node through one 64-byte record (two loads): the size
 // squared and the centre (the same expressions the reference evaluates at every
@@ -873,7 +874,7 @@ int dem_tree_create(dem_ctx *ctx, int capacity, int max_nodes, dem_tree **out) {
     if (e != cudaSuccess) {
         tree_free(t);
         delete t;
-        return dem_set_error(ctx, DEM_E_CUDA, std::string("tree allocation: ") + cudaGetErrorString(e));
+        return dem_check_cuda(ctx, e, "tree allocation");
     }
     *out = t;
     return DEM_OK;
