@@ -1648,7 +1648,6 @@ static BhWalk walk_args(dem_bh *b, float theta) {
 }
 
 static int walk_grid(dem_bh *b) { return std::max(1, (b->n + BH_T - 1) / BH_T); }
-// bh_walk2_kernel: 64 targets per warp
 
 int dem_bh_forces(dem_bh *b, double m_const, double theta, double *fx, double *fy, double *fz, void *stream) {
     if (!b || !(theta >= 0)) return DEM_E_INVALID;

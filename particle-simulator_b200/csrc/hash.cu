@@ -377,7 +377,7 @@ __global__ void radius_kernel(int n, const double *__restrict__ r, double L, int
     p.hash = hash_params(from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits), L, even_cells);
     const double r_max = from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits);
     const double mean = (double)*(volatile float *)&misc->r_sum / n;
-    double h = fmax(fmax(fmin(1.3 * L / cbrt((double)n), 4.5 * mean), 1.0 * mean), 0.5 * r_max);
+    double h = fmax(fmax(fmin(1.3 * L / cbrt((double)n), 4.5 * mean), mean), 0.5 * r_max);
     h = h <= 4.5 * r_max ? h : 4.5 * r_max;
     p.r_max = r_max;
     p.m = 0;
@@ -947,6 +947,7 @@ __global__ void pair_bin_kernel(const int32_t *__restrict__ pairs, const int64_t
 int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, const double *z, const double *r,
                        double L, int periodic, int table_size, int32_t *pairs, int64_t cap, int64_t *counts,
                        cudaStream_t s, int even_cells) {
+    // the limit from when the table was scanned (now a mask only, and the row counts are): 2^25 buckets, 2^24 droplets
     if (table_size > (int64_t)SCAN_MAX_BLOCKS * SCAN_TILE)
         return dem_set_error(ctx, DEM_E_CAPACITY, "scan: too many elements");
     int rc = dem_check_cuda(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(int64_t), s), "memset");
