@@ -38,6 +38,7 @@
 // so the pair set is bit-identical to the reference's np.unique output.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "common.cuh"
 #include "scan.cuh"
@@ -345,7 +346,7 @@ static_assert(sizeof(SearchMisc) == 4 * SEARCH_MISC_WORDS, "ctx.cu sizes the wor
 // One cell for everything where distance does not decide: cells without a finite size (an infinite radius, whose
 // droplet touches droplets at any distance; L = 0, negative or not finite) and radii below 2^-500 (the contact
 // test's squares underflow: droplets many radii apart pass it).
-__global__ void radius_kernel(int n, const double *__restrict__ r, double L, int periodic, int even_cells,
+__global__ void radius_kernel(int n, const double *__restrict__ r, double L, double spaced, int periodic, int even_cells,
                               SearchMisc *__restrict__ misc, SearchParams *__restrict__ out) {
     __shared__ bool last;
     unsigned long long m = 0ull;  // below every ordered value
@@ -377,7 +378,7 @@ __global__ void radius_kernel(int n, const double *__restrict__ r, double L, int
     p.hash = hash_params(from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits), L, even_cells);
     const double r_max = from_ordered_bits(*(volatile unsigned long long *)&misc->max_bits);
     const double mean = (double)*(volatile float *)&misc->r_sum / n;
-    double h = fmax(fmax(fmin(1.3 * L / cbrt((double)n), 4.5 * mean), mean), 0.5 * r_max);
+    double h = fmax(fmax(fmin(spaced, 4.5 * mean), mean), 0.5 * r_max);
     h = h <= 4.5 * r_max ? h : 4.5 * r_max;
     p.r_max = r_max;
     p.m = 0;
@@ -963,8 +964,8 @@ int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, co
     if (rc) return rc;
     const int grid = max(1, min(ceil_div(n, 256), 8 * ctx->sm_count));
     dem_prof_begin(ctx, "hash_detect", s);
-    radius_kernel<<<max(1, min(ceil_div(n, 1024), 4 * ctx->sm_count)), 256, 0, counted(s)>>>(n, r, L, periodic, even_cells,
-                                                                                         misc, sp);
+    radius_kernel<<<max(1, min(ceil_div(n, 1024), 4 * ctx->sm_count)), 256, 0, counted(s)>>>(
+        n, r, L, 1.3 * L / std::cbrt((double)n), periodic, even_cells, misc, sp);
     search_assign_kernel<<<grid, 256, 0, counted(s)>>>(n, x, y, z, sp, buckets - 1, bucket_count, ctx->search_key);
     search_starts_kernel<<<ceil_div(buckets, SB_T * SB_ITEMS), SB_T, 0, counted(s)>>>(buckets, bucket_count, misc, sp,
                                                                                      ctx->search_bucket);
@@ -1007,7 +1008,12 @@ int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, co
     rc = exclusive_scan<int32_t, int64_t>(ctx, row_count, ctx->pair_offset, n, s);
     if (rc) return rc;
     const int pgrid = max(1, min(ceil_div(n, group * PL_WARPS), 2 * ctx->sm_count));
-    place_pairs_kernel<<<pgrid, 32 * PL_WARPS, 0, counted(s)>>>(a, group, ctx->pair_offset, pairs, cap);
+    // At most 32 droplets' pairs per warp, whatever `group` is: its CTAs hold as much of an SM as a pass's do, and a pass
+    // that starts beside it (the solver's speculative step) is spread over the SMs that they leave.  N = 2,000, FP64: with
+    // 63 CTAs every eighth convection pass took 54 us, with 8 all take 38.6; found again, 40 pairs per droplet, 178 -> 521
+    // (768 with the reference's buckets).
+    place_pairs_kernel<<<max(1, min(ceil_div(n, 32 * PL_WARPS), 2 * ctx->sm_count)), 32 * PL_WARPS, 0, counted(s)>>>(
+        a, group, ctx->pair_offset, pairs, cap);
     write_rows_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset, pairs, cap, counts, ctx->d_err);
     dem_prof_end(ctx, s);
     return dem_check_launch(ctx, "hash write");
