@@ -31,8 +31,9 @@
 // Dense boxes are bounded by the tests' instructions.  A whole detection, equal
 // radii, periodic, us, before -> now, N = 100,000: volume fraction 0.3 (1.2 pairs
 // per droplet) 328 -> 222, 0.6 386 -> 239, 2 545 -> 347, 7 1,205 -> 689; N = 400,000:
-// 0.3 730 -> 464, 0.6 864 -> 540, 2 1,225 -> 824, 5 2,098 -> 1,605, and at 27 pairs
-// per droplet, which the list no longer holds, 2,877 -> 3,995.
+// 0.3 730 -> 464, 0.6 864 -> 540, 2 1,225 -> 824, 5 2,098 -> 1,605.  Past about 25
+// pairs per droplet the list no longer holds them: the kernels alone, at 28, N =
+// 100,000 1,098 -> 1,011, 400,000 2,816 -> 3,423.
 // The contact test is the same IEEE expression as the reference's (this file is
 // compiled with -fmad=false) and does not depend on the order of the two droplets,
 // so the pair set is bit-identical to the reference's np.unique output.
@@ -1011,8 +1012,9 @@ int launch_hash_detect(dem_ctx *ctx, int n, const double *x, const double *y, co
     // At most 32 droplets' pairs per warp, whatever `group` is: its CTAs hold as much of an SM as a pass's do, and a pass
     // that starts beside it (the solver's speculative step) is spread over the SMs that they leave.  N = 2,000, FP64: with
     // 63 CTAs every eighth convection pass took 54 us, with 8 all take 38.6; found again, 40 pairs per droplet, 178 -> 521
-    // (768 with the reference's buckets).
-    place_pairs_kernel<<<max(1, min(ceil_div(n, 32 * PL_WARPS), 2 * ctx->sm_count)), 32 * PL_WARPS, 0, counted(s)>>>(
+    // (768 with the reference's buckets).  Three CTAs per SM, all that are resident: with two, N = 100,000 and 400,000 at
+    // 28 pairs per droplet took 1,266 and 3,915 us, not 1,011 and 3,423.
+    place_pairs_kernel<<<max(1, min(ceil_div(n, 32 * PL_WARPS), 3 * ctx->sm_count)), 32 * PL_WARPS, 0, counted(s)>>>(
         a, group, ctx->pair_offset, pairs, cap);
     write_rows_kernel<<<pgrid, 256, 0, counted(s)>>>(a, ctx->pair_offset, pairs, cap, counts, ctx->d_err);
     dem_prof_end(ctx, s);
