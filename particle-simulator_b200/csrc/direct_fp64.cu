@@ -21,10 +21,11 @@
 //
 // Bound: the FP64 pipe (59 / 86 operations per pair) at large n, the adders'
 // chains and the terms' latency at small n.  Force / convection pass, periodic,
-// us, before -> now: n = 500 137 / 310 -> 13 / 13; 2,000 527 / 1,220 -> 34 / 43;
-// 8,000 2,090 / 4,860 -> 328 / 446; 20,011 5,650 / 12,800 -> 1,800 / 2,520 (FP64
-// pipe 68 / 74 % of peak; more resident warps, larger tiles or 512 producers
-// change that by a few per cent either way).
+// us, before -> now, events around the pass: n = 500 137 / 310 -> 13 / 13; 2,000 527
+// / 1,220 -> 34 / 43; 8,000 2,090 / 4,860 -> 328 / 446; 20,011 5,650 / 12,800 -> 1,800
+// / 2,520 (FP64 pipe 68 / 74 % of peak; more resident warps, larger tiles or 512
+// producers change that by a few per cent either way).  In a graph, without the
+// events' ~6 us: 6.8 / 7.3, 29 / 37, 322 / 439, 1,786 / 2,513.
 //
 // With the periodic-image correction loaded, the convection kernel adds each
 // pair's correction term right after its Stokeslet term and the self term
