@@ -309,8 +309,8 @@ __global__ void vjp_admit_kernel(const VjpArgs a, double *__restrict__ adm) {
 }
 
 // sums[c][i] (+)= droplet i's records of block rows [row0, row1), in block order; the last rows' launch writes the
-// results: mu_i = eta sum_i + lambda_i / (gamma r_i), for the pair pass in mu_pairs (zeros where r_i, not a number, cuts
-// every pair), or the gradients.
+// results: mu_i = eta sum_i + lambda_i / (gamma r_i), for the pair pass in mu_pairs (zeros where r_i is zero, whose
+// weight r_i^3 outdoes the quotient, or not a number, which cuts every pair), or the gradients.
 template <int NC>
 __global__ void vjp_sum_kernel(const VjpArgs a, int B, int nb, int row0, int row1, const double *__restrict__ records,
                                double *__restrict__ sums, double *__restrict__ mu_pairs) {
@@ -346,7 +346,7 @@ __global__ void vjp_sum_kernel(const VjpArgs a, int B, int nb, int row0, int row
         const double w = 1.0 / (a.stokes * ri);
         const double mu = a.eta * v + w * (c == 0 ? a.lx : c == 1 ? a.ly : a.lz)[i];
         (c == 0 ? a.mx : c == 1 ? a.my : a.mz)[i] = mu;
-        mu_pairs[t] = ri == ri ? mu : 0.0;
+        mu_pairs[t] = fabs(w) < INFINITY ? mu : 0.0;
     } else if (c < 3) {
         (c == 0 ? a.gx : c == 1 ? a.gy : a.gz)[i] = v;
     } else {

@@ -1,6 +1,6 @@
 """The adjoint's passes (csrc/direct_vjp.cu) with one droplet whose radius or position leaves the range: it takes its
 own terms with it (every pair of an infinite radius is cut, a pair too far apart for its squared distance has no
-term), and the others' are the plain FP64 sums over the pairs that remain."""
+term, a radius of zero has no weight), and the others' are the plain FP64 sums over the pairs that remain."""
 
 from __future__ import annotations
 
@@ -46,7 +46,8 @@ def _sums(x, r, F, lam, mu, m, eta, gamma):
 
 
 @pytest.mark.parametrize("n", [70, 2081])
-@pytest.mark.parametrize("case", ["infinite radius", "radius not a number", "radius 1e110", "position 1e200", "none"])
+@pytest.mark.parametrize("case", ["infinite radius", "radius not a number", "radius 1e110", "zero radius", "position 1e200",
+                                  "none"])
 def test_one_droplet_out_of_range(n, case):
     import torch
 
@@ -60,7 +61,9 @@ def test_one_droplet_out_of_range(n, case):
     if case == "position 1e200":
         x[k, 1] = 1e200
     elif case != "none":
-        r[k] = {"infinite radius": np.inf, "radius not a number": np.nan, "radius 1e110": 1e110}[case]
+        r[k] = {"infinite radius": np.inf, "radius not a number": np.nan, "radius 1e110": 1e110, "zero radius": 0.0}[case]
+    if case == "zero radius":
+        x[k - 1] = x[k] + 0.3 * r[k - 1]  # in contact with it
     ctx = N.Context(n)
 
     def dev(a):
@@ -69,7 +72,7 @@ def test_one_droplet_out_of_range(n, case):
     mu, g, gr = (torch.empty_like(dev(v)) for v in (x, x, r))
     ctx.direct_vjp(n, dev(x), dev(r), dev(F), dev(lam), m, eta, gamma, 1.0, False, mu, g, gr)
     mu, g, gr = mu.cpu().numpy().T, g.cpu().numpy().T, gr.cpu().numpy()
-    mu_ref, g_ref, gr_ref = _sums(x, r, F, lam, mu, m, eta, gamma)
+    mu_ref, g_ref, gr_ref = _sums(x, r, F, lam, np.where(r[:, None] == 0, 0.0, mu), m, eta, gamma)
     rest = np.arange(n) != k if "radius" in case else np.ones(n, bool)
     for a, b in ((mu, mu_ref), (g, g_ref), (gr, gr_ref)):
         assert np.linalg.norm(a[rest] - b[rest]) <= TOL * np.linalg.norm(b[rest])
